@@ -572,6 +572,7 @@ int dl_autotune(dl_context* ctx, const dl_request* reqs, int32_t n, int32_t tria
         for (auto& it : items) it.opts.max_paths_in_flight = 0;  // the pool size is what is tuned
         const bool timing = ctx->kernel_timing;
         ctx->kernel_timing = false;
+        ctx->tuning = true;
         int count = 0;
         auto time_of = [&](const dl::TuneParams& tp) {
             ctx->tune = tp;
@@ -610,10 +611,12 @@ int dl_autotune(dl_context* ctx, const dl_request* reqs, int32_t n, int32_t tria
         } catch (...) {
             ctx->tune = best;
             ctx->kernel_timing = timing;
+            ctx->tuning = false;
             throw;
         }
         ctx->tune = best;
         ctx->kernel_timing = timing;
+        ctx->tuning = false;
         if (trials) *trials = count;
         if (out) {
             std::memset(out, 0, sizeof(*out));

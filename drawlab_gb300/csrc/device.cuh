@@ -21,15 +21,30 @@
 #include "../../include/drawlab.h"
 #include "layout.h"
 
+// Helpers with many call sites.  A kernel that holds every material's code
+// (resident.cu) compiles them as functions: inlined, its code outgrows the
+// instruction cache.
+#ifndef DL_SHARED_FN
+#define DL_SHARED_FN __forceinline__
+#endif
+
 namespace dl {
 
 // ------------------------------------------------------------ float3 math
+// (sin, cos) of x, and each alone: the full-range functions
+__device__ DL_SHARED_FN float2 sin_cos(float x) {
+    float2 r;
+    sincosf(x, &r.x, &r.y);
+    return r;
+}
+__device__ DL_SHARED_FN float sin_of(float x) { return sinf(x); }
+__device__ DL_SHARED_FN float cos_of(float x) { return cosf(x); }
 __device__ __forceinline__ float3 f3(float x, float y, float z) { return make_float3(x, y, z); }
 __device__ __forceinline__ float3 add(float3 a, float3 b) { return f3(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z)); }
 __device__ __forceinline__ float3 sub(float3 a, float3 b) { return f3(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y), __fsub_rn(a.z, b.z)); }
 __device__ __forceinline__ float3 neg(float3 a) { return f3(-a.x, -a.y, -a.z); }
 __device__ __forceinline__ float3 scale(float3 a, float s) { return f3(__fmul_rn(a.x, s), __fmul_rn(a.y, s), __fmul_rn(a.z, s)); }
-__device__ __forceinline__ float3 divs(float3 a, float s) { return f3(__fdiv_rn(a.x, s), __fdiv_rn(a.y, s), __fdiv_rn(a.z, s)); }
+__device__ DL_SHARED_FN float3 divs(float3 a, float s) { return f3(__fdiv_rn(a.x, s), __fdiv_rn(a.y, s), __fdiv_rn(a.z, s)); }
 __device__ __forceinline__ float3 mul(float3 a, float3 b) { return f3(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y), __fmul_rn(a.z, b.z)); }
 __device__ __forceinline__ float dot(float3 a, float3 b) {
     return __fadd_rn(__fadd_rn(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)), __fmul_rn(a.z, b.z));
@@ -40,7 +55,7 @@ __device__ __forceinline__ float3 cross(float3 a, float3 b) {
               __fsub_rn(__fmul_rn(a.x, b.y), __fmul_rn(a.y, b.x)));
 }
 __device__ __forceinline__ float length(float3 a) { return __fsqrt_rn(dot(a, a)); }
-__device__ __forceinline__ float3 normalize(float3 a) {
+__device__ DL_SHARED_FN float3 normalize(float3 a) {
     float l = length(a);
     return f3(__fdiv_rn(a.x, l), __fdiv_rn(a.y, l), __fdiv_rn(a.z, l));
 }
@@ -328,12 +343,11 @@ __device__ __forceinline__ float3 to_world(const Frame& f, float3 v) {
 }
 
 // ------------------------------------------------------------------ warps
-__device__ __forceinline__ float2 square_to_uniform_disk(float2 s) {
+__device__ DL_SHARED_FN float2 square_to_uniform_disk(float2 s) {
     float r = __fsqrt_rn(s.x);
     float theta = __fmul_rn(__fmul_rn(2.0f, kPiF), s.y);
-    float sn, cs;
-    sincosf(theta, &sn, &cs);
-    return make_float2(__fmul_rn(r, cs), __fmul_rn(r, sn));
+    const float2 sc = sin_cos(theta);
+    return make_float2(__fmul_rn(r, sc.y), __fmul_rn(r, sc.x));
 }
 __device__ __forceinline__ float3 square_to_cosine_hemisphere(float2 s) {
     float2 p = square_to_uniform_disk(s);
@@ -341,15 +355,13 @@ __device__ __forceinline__ float3 square_to_cosine_hemisphere(float2 s) {
     return f3(p.x, p.y, __fsqrt_rn(__fsub_rn(1.0f, sum)));
 }
 __device__ __forceinline__ float cosine_hemisphere_pdf(float3 v) { return v.z <= 0.f ? 0.f : __fmul_rn(v.z, kInvPiF); }
-__device__ __forceinline__ float3 square_to_beckmann(float2 s, float alpha) {
+__device__ DL_SHARED_FN float3 square_to_beckmann(float2 s, float alpha) {
     float theta = atanf(__fsqrt_rn(__fmul_rn(__fmul_rn(-alpha, alpha), logf(__fsub_rn(1.0f, s.x)))));
     float phi = __fmul_rn(__fmul_rn(2.0f, kPiF), s.y);
-    float st, ct, sp, cp;
-    sincosf(theta, &st, &ct);
-    sincosf(phi, &sp, &cp);
-    return f3(__fmul_rn(st, cp), __fmul_rn(st, sp), ct);
+    const float2 t = sin_cos(theta), p = sin_cos(phi);
+    return f3(__fmul_rn(t.x, p.y), __fmul_rn(t.x, p.x), t.y);
 }
-__device__ __forceinline__ float beckmann_pdf(float3 m, float alpha) {
+__device__ DL_SHARED_FN float beckmann_pdf(float3 m, float alpha) {
     if (m.z <= 0.f) return 0.f;
     float c = m.z;
     float cc = __fmul_rn(c, c);
@@ -364,7 +376,7 @@ __device__ __forceinline__ float3 square_to_uniform_triangle(float2 s) {
     return f3(__fsub_rn(1.f, t), ty, __fsub_rn(t, ty));
 }
 
-__device__ __forceinline__ float fresnel(float cosI, float extIOR, float intIOR) {
+__device__ DL_SHARED_FN float fresnel(float cosI, float extIOR, float intIOR) {
     float etaI = extIOR, etaT = intIOR;
     if (extIOR == intIOR) return 0.0f;
     if (cosI < 0.0f) {
@@ -413,7 +425,7 @@ __device__ __forceinline__ float tan_theta(float3 v) {
     return __fdiv_rn(__fsqrt_rn(temp), v.z);
 }
 // microfacet.cpp:35-44 (rational Smith G1), evaluated in float
-__device__ __forceinline__ float beckmann_g1(float3 wv, float3 wh, float alpha) {
+__device__ DL_SHARED_FN float beckmann_g1(float3 wv, float3 wh, float alpha) {
     float c = __fdiv_rn(dot(wv, wh), wv.z);
     if (c <= 0.f) return 0.f;
     float b = __fdiv_rn(1.0f, __fmul_rn(alpha, tan_theta(wv)));
@@ -424,23 +436,22 @@ __device__ __forceinline__ float beckmann_g1(float3 wv, float3 wh, float alpha) 
     return __fdiv_rn(num, den);
 }
 // aniso_ggx.cu:9-15 and include/optix/math/wrap.h:54-77
-__device__ __forceinline__ float ggx_g1(float3 v, float ax, float ay) {
+__device__ DL_SHARED_FN float ggx_g1(float3 v, float ax, float ay) {
     if (v.z <= 0.f) return 0.f;
     float3 vv = f3(__fmul_rn(v.x, ax), __fmul_rn(v.y, ay), v.z);
     return __fdiv_rn(__fmul_rn(2.0f, v.z), __fadd_rn(v.z, length(vv)));
 }
-__device__ __forceinline__ float ggx_pdf(float3 m, float ax, float ay) {
+__device__ DL_SHARED_FN float ggx_pdf(float3 m, float ax, float ay) {
     if (m.z <= 0.f) return 0.f;
     float3 h = f3(__fdiv_rn(m.x, ax), __fdiv_rn(m.y, ay), m.z);
     float len2 = dot(h, h);
     return __fdiv_rn(1.f, __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(kPiF, ax), ay), len2), len2));
 }
-__device__ __forceinline__ float3 square_to_ggx(float2 s, float ax, float ay) {
+__device__ DL_SHARED_FN float3 square_to_ggx(float2 s, float ax, float ay) {
     float sq = __fdiv_rn(__fsqrt_rn(s.x), __fsqrt_rn(__fsub_rn(1.f, s.x)));
-    float sp, cp;
-    sincosf(__fmul_rn(__fmul_rn(2.f, kPiF), s.y), &sp, &cp);
-    float x = __fmul_rn(__fmul_rn(ax, sq), cp);
-    float y = __fmul_rn(__fmul_rn(ay, sq), sp);
+    const float2 p = sin_cos(__fmul_rn(__fmul_rn(2.f, kPiF), s.y));
+    float x = __fmul_rn(__fmul_rn(ax, sq), p.y);
+    float y = __fmul_rn(__fmul_rn(ay, sq), p.x);
     return normalize(f3(-x, -y, 1.f));
 }
 
@@ -587,7 +598,7 @@ constexpr float kHalfInvPiF = (float)(0.5 / (double)kPiF);  // (float)(0.5 / M_P
 // Bilinear, wrap-addressed lookup at normalised coordinates (u, v) of a
 // W x H texel array (the filtering of a CUDA texture with linear filtering
 // and wrap addressing, restated with fp32 weights).
-__device__ __forceinline__ float3 tex_bilinear(const float4* tex, int W, int H, float u, float v) {
+__device__ DL_SHARED_FN float3 tex_bilinear(const float4* tex, int W, int H, float u, float v) {
     if (!isfinite(u) || !isfinite(v)) return f3(0.f, 0.f, 0.f);
     u = __fsub_rn(u, floorf(u));
     v = __fsub_rn(v, floorf(v));
@@ -631,7 +642,7 @@ __device__ __forceinline__ float3 env_lookup(const DevScene& sc, float u, float 
 }
 
 // Envmap::environment_coords (envmap.h:26-30)
-__device__ __forceinline__ float2 env_coords(float3 d) {
+__device__ DL_SHARED_FN float2 env_coords(float3 d) {
     float u = __fadd_rn(__fmul_rn(atan2f(d.z, d.x), kHalfInvPiF), 0.5f);
     float v = __fmul_rn(acosf(fmaxf(fminf(d.y, 1.0f), -1.0f)), kInvPiF);
     return make_float2(u, v);
@@ -673,11 +684,11 @@ __device__ __forceinline__ float3 env_sample(const DevScene& sc, float3 sh_n, fl
     float phi = (float)__dsub_rn(__dmul_rn(__dmul_rn((double)u, 2.0), (double)kPiF), (double)kPiF);
     float step_theta = __fdiv_rn(kPiF, (float)H);
     float theta0 = __fmul_rn((float)py, step_theta);
-    float cos_theta = __fadd_rn(__fmul_rn(cosf(theta0), __fsub_rn(1.0f, xi.z)),
-                                __fmul_rn(cosf(__fadd_rn(theta0, step_theta)), xi.z));
+    float cos_theta = __fadd_rn(__fmul_rn(cos_of(theta0), __fsub_rn(1.0f, xi.z)),
+                                __fmul_rn(cos_of(__fadd_rn(theta0, step_theta)), xi.z));
     float theta = acosf(cos_theta);
-    float sin_theta = sinf(theta);
-    d = f3(__fmul_rn(cosf(phi), sin_theta), cos_theta, __fmul_rn(sinf(phi), sin_theta));
+    float sin_theta = sin_of(theta);
+    d = f3(__fmul_rn(cos_of(phi), sin_theta), cos_theta, __fmul_rn(sin_of(phi), sin_theta));
     if (!(pdf > 0.f)) return f3(0.f, 0.f, 0.f);
     float3 val = env_lookup(sc, u, __fmul_rn(theta, kInvPiF));
     float c = fmaxf(dot(sh_n, d), 0.f);

@@ -172,6 +172,7 @@ struct dl_context {
     int num_sms = 0;
     dl::TuneParams tune;
     bool kernel_timing = false;
+    bool tuning = false;   // dl_autotune is timing the wavefront's launch shapes
     std::vector<cudaEvent_t> timing_events;  // created on first timed render
     // CUDA graph of one batch of wavefront iterations, reused while the
     // kernel parameters stay byte-identical.

@@ -40,455 +40,10 @@
 #include "guide.cuh"
 #include "guide_tc.cuh"
 #include "internal.h"
+#include "path.cuh"
 #include "scene.h"
 
 namespace dl {
-
-enum PathFlags { PF_CAMERA = 1, PF_PREV_DIFFUSE = 2 };
-
-struct __align__(32) RayRec {
-    float4 o;   // origin, tmin
-    float4 d;   // direction, tmax
-};
-struct __align__(32) PathRec {
-    float4 tp;  // throughput.rgb, eta
-    float4 L;   // radiance.rgb, pdf of the last BSDF sample
-};
-struct __align__(32) MetaRec {
-    int4 m;     // depth, flags, path index lo, path index hi
-    uint4 rng;  // pcg32 state lo/hi, inc lo/hi
-};
-struct __align__(32) HitRec {
-    float4 h;   // t, u, v, leaf-order triangle (int bits; -1 = miss)
-    float4 pad;
-};
-static_assert(sizeof(RayRec) == 32 && sizeof(PathRec) == 32 && sizeof(MetaRec) == 32 && sizeof(HitRec) == 32,
-              "path records are one 32-byte sector each");
-// A slot's four records share one 128-byte line: the ray and its hit in one
-// half, the path state in the other.  Slots are visited in queue order, i.e.
-// at random; a random 32-byte read costs a whole DRAM burst, so records read
-// together are kept inside one.
-struct __align__(128) SlotRec {
-    RayRec ray;
-    HitRec hit;
-    PathRec path;
-    MetaRec meta;
-};
-static_assert(sizeof(SlotRec) == 128, "one 128-byte line per slot");
-constexpr size_t kSlotBytes = 4 * 32 + 8 + 3 * 16 + 4 * (2 + kNumMaterialTypes + 1);  // records, pos, shadow, queues
-
-constexpr int kMissQueue = kNumMaterialTypes;  // queue index of rays that hit nothing
-
-// One render request: a scene and its render options.  A single render has
-// one request, carried in the kernel parameters; a batch has a table of them
-// in device memory and every path carries its request's index (in the path
-// flags, in the ray records' w slot).
-struct DevRequest {
-    DevScene sc;
-    unsigned long long pid_first;  // the request's first path index in the current pass
-    int spp_offset;                // sample index of its first sample in the pass
-    int max_depth;
-    int rr_depth;
-    unsigned int flags;
-    unsigned long long seed_mix;
-};
-constexpr int kReqShift = 8;  // path flags: request index << kReqShift | PathFlags
-
-// Guided renders: per slot, the training records of the path's two most
-// recent guided vertices with the throughput after each (a: older, b: newer;
-// record index in w, -1 for none).  Radiance the path gathers later is
-// credited to them divided by that throughput: the estimate of the radiance
-// arriving along the direction sampled there.
-struct __align__(32) GuideRec {
-    float4 a;
-    float4 b;
-};
-
-struct RenderParams {
-    DevRequest r0;                 // the request of a single render
-    int capacity;                  // path slots (queue and record arrays hold this many entries)
-    const DevRequest* reqs;        // batch: request table (pid_first ascending)
-    int num_reqs;
-    SlotRec* rec;    // per slot: ray, hit, path state
-    float2* pos;     // film position of the camera sample (Li mode only)
-    int* ext_q[2];
-    int* mat_q[kNumMaterialTypes + 1];  // per material type, then the miss queue
-    float4* sh_o;
-    float4* sh_d;
-    float4* sh_c;    // contribution.rgb, target: slot >= 0 (live path) or -1 - path index (ended path)
-    RenderCounters* cnt;
-    float4* samples; // radiance.rgb + presence flag per path index of this chunk
-    int mode;        // 0: film, 1: Li of explicit paths
-    const int* xys;
-    float* li_L;
-    float* li_pos;
-    // guided renders
-    int guided;
-    GuideNet gnet;
-    GuideRec* grec;
-    GuideRecord* grecords;
-    int grecord_cap;
-};
-
-template <bool kMulti>
-__device__ __forceinline__ const DevRequest& request(const RenderParams& P, int rid) {
-    if (kMulti) return P.reqs[rid];
-    return P.r0;
-}
-
-// Bounds-checked build (compiled with -DDL_CHECKS): before each access whose
-// index comes from a queue, a counter or a record -- path slots, queue
-// positions, path indices, BVH nodes and triangles -- the index is checked
-// against its array; a violation sets kErrBounds in the render's error word
-// and the access is skipped.  Without DL_CHECKS the checks compile to
-// nothing.
-constexpr unsigned kErrBounds = 4u;
-#ifdef DL_CHECKS
-__device__ __forceinline__ bool in_bounds(bool ok, unsigned int* err) {
-    if (!ok) atomicOr(err, kErrBounds);
-    return ok;
-}
-#define DL_IN_BOUNDS(cond, err) in_bounds((cond), (err))
-#else
-#define DL_IN_BOUNDS(cond, err) true
-#endif
-constexpr const char* kBoundsMessage = "bounds check failed: a queue, slot, path, node or triangle index "
-                                        "outside its array (bounds-checked build)";
-// 32 bytes (32-byte aligned) of read-only global data in one load.
-__device__ __forceinline__ void ld_nc_256(const float4* p, float4& a, float4& b) {
-    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-        : "l"(p));
-}
-__device__ __forceinline__ bool slot_ok(const RenderParams& P, int slot) {
-    return DL_IN_BOUNDS(slot >= 0 && slot < P.capacity, &P.cnt->err);
-}
-
-// Request of batch path `pid`: the last request whose first path is <= pid.
-__device__ __forceinline__ int find_request(const RenderParams& P, unsigned long long pid) {
-    int lo = 0, hi = P.num_reqs;
-    while (hi - lo > 1) {
-        int mid = (lo + hi) >> 1;
-        if (P.reqs[mid].pid_first <= pid) lo = mid; else hi = mid;
-    }
-    return lo;
-}
-
-// ------------------------------------------------------------ warp helpers
-__device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
-
-// All 32 lanes call this with their predicate; returns the lane's slot in the
-// queue (or -1).  One atomic per warp.
-__device__ __forceinline__ int warp_push(int* counter, bool pred) {
-    unsigned mask = __ballot_sync(0xffffffffu, pred);
-    if (mask == 0) return -1;
-    int leader = __ffs(mask) - 1;
-    int base = 0;
-    if (lane_id() == leader) base = atomicAdd(counter, __popc(mask));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    return pred ? base + __popc(mask & ((1u << lane_id()) - 1u)) : -1;
-}
-__device__ __forceinline__ unsigned long long warp_claim(unsigned long long* counter, bool pred) {
-    unsigned mask = __ballot_sync(0xffffffffu, pred);
-    if (mask == 0) return ~0ull;
-    int leader = __ffs(mask) - 1;
-    unsigned long long base = 0;
-    if (lane_id() == leader) base = atomicAdd(counter, (unsigned long long)__popc(mask));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    return pred ? base + (unsigned long long)__popc(mask & ((1u << lane_id()) - 1u)) : ~0ull;
-}
-
-__device__ __forceinline__ unsigned long long warp_claim_u32(unsigned int* counter, bool pred) {
-    unsigned mask = __ballot_sync(0xffffffffu, pred);
-    if (mask == 0) return ~0ull;
-    int leader = __ffs(mask) - 1;
-    unsigned base = 0;
-    if (lane_id() == leader) base = atomicAdd(counter, (unsigned)__popc(mask));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    return pred ? (unsigned long long)base + __popc(mask & ((1u << lane_id()) - 1u)) : ~0ull;
-}
-
-__device__ __forceinline__ Pcg32 load_rng(const uint4& r) {
-    Pcg32 g;
-    g.state = ((uint64_t)r.y << 32) | r.x;
-    g.inc = ((uint64_t)r.w << 32) | r.z;
-    return g;
-}
-__device__ __forceinline__ uint4 store_rng(const Pcg32& g) {
-    return make_uint4((uint32_t)g.state, (uint32_t)(g.state >> 32), (uint32_t)g.inc, (uint32_t)(g.inc >> 32));
-}
-__device__ __forceinline__ unsigned long long path_index(const int4& m) {
-    return (unsigned long long)(unsigned)m.z | ((unsigned long long)(unsigned)m.w << 32);
-}
-
-// Start path `pid` in `slot`: camera sample and ray (cpu_renderer.cpp:36-44).
-// Ray records carry the request index in o.w (every render ray starts at
-// tmin = kRayEps).
-template <bool kMulti>
-__device__ void start_path(const RenderParams& P, int slot, unsigned long long pid) {
-    if (!slot_ok(P, slot) || !DL_IN_BOUNDS(pid < P.cnt->pass_total, &P.cnt->err)) return;
-    const int rid = kMulti ? find_request(P, pid) : 0;
-    const DevRequest& R = request<kMulti>(P, rid);
-    const DevCamera& cam = R.sc.cam;
-    int x, y, s;
-    if (P.mode == 1) {
-        x = P.xys[3 * pid];
-        y = P.xys[3 * pid + 1];
-        s = P.xys[3 * pid + 2];
-    } else {
-        unsigned long long local = pid - R.pid_first;
-        unsigned long long npix = (unsigned long long)cam.w * cam.h;
-        if ((local | npix) < 0x100000000ull) {  // 32-bit division where it fits
-            const unsigned l32 = (unsigned)local, n32 = (unsigned)npix, pix = l32 % n32;
-            s = (int)(l32 / n32);
-            x = (int)(pix % (unsigned)cam.w);
-            y = (int)(pix / (unsigned)cam.w);
-        } else {
-            unsigned long long pix = local % npix;
-            s = (int)(local / npix);
-            x = (int)(pix % cam.w);
-            y = (int)(pix / cam.w);
-        }
-        s += kMulti ? R.spp_offset : P.cnt->pass_spp_offset;
-    }
-    Pcg32 g;
-    seed_path(g, R.seed_mix, cam.w, cam.h, x, y, s);
-    float2 ps = g.next2d();
-    ps.x = __fadd_rn((float)x, ps.x);
-    ps.y = __fadd_rn((float)y, ps.y);
-    (void)g.next2d();  // aperture sample: drawn, unused by the "virtual" camera
-    float3 o, d;
-    float tmax;
-    camera_ray(cam, ps, o, d, tmax);
-    RayRec r;
-    r.o = make_float4(o.x, o.y, o.z, __int_as_float(rid));
-    r.d = make_float4(d.x, d.y, d.z, tmax);
-    P.rec[slot].ray = r;
-    PathRec pr;
-    pr.tp = make_float4(1.f, 1.f, 1.f, 1.f);
-    pr.L = make_float4(0.f, 0.f, 0.f, 0.f);
-    P.rec[slot].path = pr;
-    MetaRec mr;
-    mr.m = make_int4(0, PF_CAMERA | (rid << kReqShift), (int)(pid & 0xffffffffu), (int)(pid >> 32));
-    mr.rng = store_rng(g);
-    P.rec[slot].meta = mr;
-    if (P.mode == 1) P.pos[slot] = ps;
-    if (P.guided) {
-        GuideRec gr;
-        gr.a = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
-        gr.b = gr.a;
-        P.grec[slot] = gr;
-    }
-}
-
-// Radiance of ended path `pid` (slot `slot`): into the sample buffer at its
-// path index (the film kernel gathers it), or as its Li.
-__device__ __forceinline__ void store_sample(const RenderParams& P, unsigned long long pid, float3 L, int slot) {
-    if (!slot_ok(P, slot) || !DL_IN_BOUNDS(pid < P.cnt->pass_total, &P.cnt->err)) return;
-    if (P.mode == 1) {
-        P.li_L[3 * pid] = L.x;
-        P.li_L[3 * pid + 1] = L.y;
-        P.li_L[3 * pid + 2] = L.z;
-        float2 ps = P.pos[slot];
-        P.li_pos[2 * pid] = ps.x;
-        P.li_pos[2 * pid + 1] = ps.y;
-    } else {
-        P.samples[pid] = make_float4(L.x, L.y, L.z, 1.f);
-    }
-}
-
-// A shadow ray of an ended path was unoccluded: add its contribution to the
-// stored sample.  One shadow ray per path at a time, so no atomics.
-__device__ __forceinline__ void add_to_sample(const RenderParams& P, unsigned long long pid, float4 c) {
-    if (!DL_IN_BOUNDS(pid < P.cnt->pass_total, &P.cnt->err)) return;
-    if (P.mode == 1) {
-        P.li_L[3 * pid] = __fadd_rn(P.li_L[3 * pid], c.x);
-        P.li_L[3 * pid + 1] = __fadd_rn(P.li_L[3 * pid + 1], c.y);
-        P.li_L[3 * pid + 2] = __fadd_rn(P.li_L[3 * pid + 2], c.z);
-    } else {
-        float4 s = P.samples[pid];
-        P.samples[pid] = make_float4(__fadd_rn(s.x, c.x), __fadd_rn(s.y, c.y), __fadd_rn(s.z, c.z), s.w);
-    }
-}
-
-// Radiance `c` reached the path: credit it to the training records of its
-// guided vertices (the newer one too if `both`), divided by the throughput
-// after each vertex (mean over the channels it is non-zero in).
-__device__ __forceinline__ void credit_one(const RenderParams& P, float4 t, float3 c) {
-    int idx = __float_as_int(t.w);
-    if (idx < 0) return;
-    float s = 0.f;
-    int k = 0;
-    if (t.x > 0.f) { s += c.x / t.x; k++; }
-    if (t.y > 0.f) { s += c.y / t.y; k++; }
-    if (t.z > 0.f) { s += c.z / t.z; k++; }
-    if (k > 0 && isfinite(s)) static_cast<GuideRecord*>(P.cnt->pass_recs)[idx].L += s / (float)k;
-}
-__device__ __forceinline__ void credit(const RenderParams& P, const GuideRec& gr, float3 c, bool both) {
-    credit_one(P, gr.a, c);
-    if (both) credit_one(P, gr.b, c);
-}
-
-// Claim new path indices for the lanes in `want`, start them; returns true
-// for lanes that now hold a fresh camera ray.
-template <bool kMulti>
-__device__ __forceinline__ bool regenerate(const RenderParams& P, int slot, bool want) {
-    unsigned long long pid = warp_claim(&P.cnt->next_path, want);
-    bool ok = want && pid < P.cnt->pass_total;
-    if (ok) start_path<kMulti>(P, slot, pid);
-    return ok;
-}
-
-struct HitInfo {
-    float3 p;
-    Frame sh;
-    int mesh;
-};
-
-__device__ __forceinline__ HitInfo hit_info(const DevScene& sc, int tri, float u, float v) {
-    HitInfo h;
-    const float4* tp = sc.tris + 3 * tri;
-    float3 p0 = xyz(__ldg(tp)), p1 = xyz(__ldg(tp + 1)), p2 = xyz(__ldg(tp + 2));
-    float b0 = __fsub_rn(__fsub_rn(1.f, u), v);
-    h.p = add(add(scale(p0, b0), scale(p1, u)), scale(p2, v));
-    int4 vi = __ldg(sc.tri_vidx + tri);
-    h.mesh = vi.w;
-    if (sc.meshes[vi.w].has_normals) {
-        float3 n0 = xyz(__ldg(sc.normals + vi.x)), n1 = xyz(__ldg(sc.normals + vi.y));
-        float3 n2 = normalize(xyz(__ldg(sc.normals + vi.z)));
-        // only the third term normalised (src/tracer/accel/octree.cpp:202-206)
-        h.sh = make_frame(add(add(scale(n0, b0), scale(n1, u)), scale(n2, v)));
-    } else {
-        h.sh = make_frame(normalize(cross(sub(p1, p0), sub(p2, p0))));
-    }
-    return h;
-}
-
-// Mesh::samplePosition over an area light's triangles (mesh.cpp:222-244,
-// DiscretePDF::sampleReuse dpdf.h:131-136).
-__device__ __forceinline__ void sample_area(const DevScene& sc, const DevLight& L, float2 s, float3& p,
-                                            float3& n) {
-    const float* cdf = sc.emit_cdf + L.cdf_begin;
-    int cnt = L.tri_count;
-    // lower_bound over cdf[0..cnt]
-    int lo = 0, hi = cnt + 1;
-    while (lo < hi) {
-        int mid = (lo + hi) >> 1;
-        if (__ldg(cdf + mid) < s.x) lo = mid + 1; else hi = mid;
-    }
-    int f = max(lo - 1, 0);
-    f = min(f, cnt - 1);
-    float c0 = __ldg(cdf + f), c1 = __ldg(cdf + f + 1);
-    s.x = __fdiv_rn(__fsub_rn(s.x, c0), __fsub_rn(c1, c0));
-    const float4* et = sc.emit_tris + 6 * (L.tri_begin + f);
-    float3 p0 = xyz(__ldg(et)), p1 = xyz(__ldg(et + 1)), p2 = xyz(__ldg(et + 2));
-    float3 b = square_to_uniform_triangle(s);
-    p = add(add(scale(p0, b.x), scale(p1, b.y)), scale(p2, b.z));
-    if (L.has_normals) {
-        float3 n0 = xyz(__ldg(et + 3)), n1 = xyz(__ldg(et + 4)), n2 = xyz(__ldg(et + 5));
-        n = add(add(scale(n0, b.x), scale(n1, b.y)), scale(n2, b.z));
-    } else {
-        n = cross(sub(p1, p0), sub(p2, p1));
-    }
-    n = normalize(n);
-}
-
-// The emitter that the NEE sample's first number picks, that number rescaled
-// to [0, 1) for reuse: uniformly (scene.cpp:148-163), or, with
-// DL_RENDER_POWER_LIGHT_PICK, through the power alias table (slot from the
-// number, alias coin from its fraction).
-__device__ __forceinline__ int pick_light(const DevRequest& R, float& sx) {
-    const DevScene& sc = R.sc;
-    const int N = sc.num_lights;
-    if (!(R.flags & DL_RENDER_POWER_LIGHT_PICK)) {
-        if (N <= 1) return 0;
-        int idx = min((int)__fmul_rn(sx, (float)N), N - 1);
-        sx = __fsub_rn(__fmul_rn(sx, (float)N), (float)idx);
-        return idx;
-    }
-    float u = __fmul_rn(sx, (float)N);
-    int i = min((int)u, N - 1);
-    float coin = fminf(__fsub_rn(u, (float)i), 0.99999994f);
-    float4 a = __ldg(sc.light_pick + i);
-    if (coin < a.x) {
-        sx = __fdiv_rn(coin, a.x);
-        return i;
-    }
-    sx = __fdiv_rn(__fsub_rn(coin, a.x), __fsub_rn(1.f, a.x));
-    return __float_as_int(a.y);
-}
-
-// pdf of direction sample `pdf` of emitter `l` times its pick probability
-// (pdfEmitterDirection, scene.cpp:171-179).
-__device__ __forceinline__ float with_pick_pdf(const DevRequest& R, int l, float pdf) {
-    if (R.flags & DL_RENDER_POWER_LIGHT_PICK) return __fmul_rn(pdf, __ldg(R.sc.light_pick + l).z);
-    return R.sc.num_lights != 1 ? __fdiv_rn(pdf, (float)R.sc.num_lights) : pdf;
-}
-
-// Three fresh numbers for an envmap NEE sample, drawn after the NEE 2D sample.
-__device__ __forceinline__ float3 env_xi(Pcg32& g) {
-    float3 xi;
-    xi.x = g.next_float();
-    xi.y = g.next_float();
-    xi.z = g.next_float();
-    return xi;
-}
-
-// Scene::sampleEmitterDirection without the visibility test (the caller
-// traces the shadow ray).  Returns the unoccluded spectrum.  An envmap pick
-// draws three more numbers from `g`.
-__device__ __forceinline__ float3 sample_emitter(const DevRequest& R, float3 its_p, float3 sh_n, float2 s,
-                                                 Pcg32& g, float3& d, float& dist, float& pdf, bool& delta) {
-    const DevScene& sc = R.sc;
-    int N = sc.num_lights;
-    float3 zero = f3(0.f, 0.f, 0.f);
-    delta = false;
-    pdf = 0.f;
-    dist = 0.f;
-    d = zero;
-    if (N == 0) return zero;
-    const int idx = pick_light(R, s.x);
-    const DevLight& L = sc.lights[idx];
-    float3 spec;
-    if (L.type == LIGHT_AREA) {
-        float3 lp, ln;
-        sample_area(sc, L, s, lp, ln);
-        float3 vec = sub(lp, its_p);
-        d = normalize(vec);
-        dist = length(vec);
-        float dp = fmaxf(dot(ln, neg(d)), 0.f);
-        float pw = dp != 0.f ? __fdiv_rn(__fmul_rn(__fmul_rn(L.pA, dist), dist), dp) : 0.f;
-        pdf = pw;
-        spec = pw != 0.f ? divs(scale(ld3(L.radiance), fmaxf(dot(sh_n, d), 0.f)), pw) : zero;
-    } else if (L.type == LIGHT_POINT) {
-        float3 vec = sub(ld3(L.position), its_p);
-        d = normalize(vec);
-        dist = length(vec);
-        pdf = 1.f;
-        delta = true;
-        float inv = __fdiv_rn(1.0f, dist);
-        if (R.flags & DL_RENDER_FIX_POINT_LIGHT) {
-            float c = fmaxf(dot(sh_n, d), 0.f);
-            spec = c > 0.f ? scale(scale(scale(ld3(L.radiance), c), inv), inv) : zero;
-        } else {
-            spec = scale(scale(ld3(L.radiance), inv), inv);
-        }
-    } else if (L.type == LIGHT_ENVMAP) {
-        spec = env_sample(sc, sh_n, env_xi(g), d, pdf);
-        dist = 1e16f;  // envmap.h:67
-    } else {
-        spec = zero;
-    }
-    if (R.flags & DL_RENDER_POWER_LIGHT_PICK) {
-        const float pl = __ldg(sc.light_pick + idx).z;
-        spec = divs(spec, pl);
-        pdf = __fmul_rn(pdf, pl);
-    } else if (N > 1) {
-        spec = scale(spec, (float)N);
-        pdf = __fmul_rn(pdf, __fdiv_rn(1.f, (float)N));
-    }
-    return spec;
-}
 
 // ---------------------------------------------------------------- kernels
 // First camera paths of a pass: slot i starts path i (no claiming needed),
@@ -507,10 +62,6 @@ __global__ void k_init(RenderParams P, int capacity) {
         P.ext_q[0][slot] = slot;
     }
 }
-
-// traversal state: ray finished (below every leaf reference: scenes hold
-// fewer than 2^27 triangles)
-constexpr int kDone = INT_MIN;
 
 // Persistent traversal over a ray queue.  Each lane holds one ray's
 // traversal state (node, stack); a lane whose ray finishes takes the next ray
@@ -793,9 +344,7 @@ __global__ void __launch_bounds__(128) k_traverse(RenderParams P, int p) {
 }
 
 // Rays that hit nothing (path.cpp:23-25, 85-87): with an envmap, add its
-// radiance first (miss.cu:11-49: camera rays see it if "visual", else the
-// background colour; later rays weight it by MIS against the BSDF pdf after
-// a diffuse bounce).  Store the sample, then start new camera paths in the
+// radiance first.  Store the sample, then start new camera paths in the
 // freed slots.
 template <bool kMulti, int kThreads>
 __global__ void __launch_bounds__(kThreads) k_miss(RenderParams P, int p) {
@@ -836,26 +385,16 @@ __global__ void __launch_bounds__(kThreads) k_miss(RenderParams P, int p) {
             int4 m = P.rec[slot].meta.m;
             const DevRequest& R = request<kMulti>(P, m.y >> kReqShift);
             const DevScene& sc = R.sc;
-            float3 L = f3(pr.L.x, pr.L.y, pr.L.z);
-            // (the normals integrator returns 0 on a miss, normal.cpp:13-14)
-            if (sc.env_light >= 0 && !(R.flags & DL_RENDER_NORMALS)) {
-                float3 dir = xyz(P.rec[slot].ray.d);
-                if (m.y & PF_CAMERA) {
-                    L = add(L, sc.env_visual ? env_lookup_dir(sc, dir) : ld3(sc.env_bg));
-                } else {
-                    float3 le = env_lookup_dir(sc, dir);
-                    float w = 1.f;
-                    if (m.y & PF_PREV_DIFFUSE) {
-                        float ep = env_pdf(sc, dir);
-                        ep = with_pick_pdf(R, sc.env_light, ep);
-                        w = mis_weight(pr.L.w, ep);
-                    }
-                    float3 c = mul(scale(f3(pr.tp.x, pr.tp.y, pr.tp.z), w), le);
-                    L = add(L, c);
+            PathState S;
+            S.tp = f3(pr.tp.x, pr.tp.y, pr.tp.z);
+            S.L = f3(pr.L.x, pr.L.y, pr.L.z);
+            S.prev_pdf = pr.L.w;
+            S.flags = m.y;
+            if (sc.env_light >= 0 && !(R.flags & DL_RENDER_NORMALS))
+                add_miss(R, xyz(P.rec[slot].ray.d), S, [&](float3 c) {
                     if (P.guided) credit(P, P.grec[slot], c, true);
-                }
-            }
-            store_sample(P, path_index(m), L, slot);
+                });
+            store_sample(P, path_index(m), S.L, slot);
         }
         const int r = done_before + lane_id();
         const unsigned long long pid = pid0 + (unsigned long long)r;
@@ -867,13 +406,10 @@ __global__ void __launch_bounds__(kThreads) k_miss(RenderParams P, int p) {
     }
 }
 
-// One BSDF type, the whole rest of the path iteration for hits on it:
-// emitter hit + MIS (path.cpp:72-84) or first-hit emission (27-29), Russian
-// roulette (89-97), depth limit, next-event estimation (36-56) and BSDF
-// sampling (60-69).  A path that ends here stores its sample and its slot
-// starts a new camera path at once; a shadow ray it emitted on the way adds
-// to the stored sample when traced.  Mirror and dielectric still draw the NEE
-// sample (their eval and pdf are zero: no contribution, no shadow ray).
+// One BSDF type, the whole rest of the path iteration for hits on it
+// (enter_vertex, scatter_vertex).  A path that ends here stores its sample
+// and its slot starts a new camera path at once; a shadow ray it emitted on
+// the way adds to the stored sample when traced.
 //
 // kGuided (diffuse, Beckmann, GGX in a guided render): blocks of two
 // warpgroups; each warpgroup takes 128 queued hits at a time and evaluates
@@ -914,238 +450,96 @@ __global__ void __launch_bounds__(kGuided ? kTcThreads : kThreads) k_material(Re
         bool cont = false, emit = false, done = false;
         float4 sh_o = make_float4(0.f, 0.f, 0.f, 0.f), sh_d = sh_o, sh_c = sh_o;
         // ---- phase 1: emitter hit, Russian roulette, depth limit
-        RayRec ray;
-        PathRec pr;
-        MetaRec mr;
-        Pcg32 g;
+        PathState S;
         HitInfo h;
         GuideRec gr;
         float2 tuv = make_float2(0.f, 0.f);  // texture coordinates (textured materials)
         float3 s_tan = f3(0.f, 0.f, 0.f);    // aniso_ggx: shading tangent from a tangent map
-        float3 tp = f3(0.f, 0.f, 0.f), Lr = tp, dir = tp;
-        float eta = 1.f;
-        int depth = 0, flags = 0, rid = 0;
-        unsigned long long pid = 0;
+        float3 dir = f3(0.f, 0.f, 0.f);
+        int rid = 0;
+        S.tp = dir;
+        S.pid = 0;
+        S.depth = 0;
         if (active) {
             float4 hit = P.rec[slot].hit.h;
-            ray = P.rec[slot].ray;
-            pr = P.rec[slot].path;
-            mr = P.rec[slot].meta;
+            const RayRec ray = P.rec[slot].ray;
+            const PathRec pr = P.rec[slot].path;
+            const MetaRec mr = P.rec[slot].meta;
             if (guided) gr = P.grec[slot];
-            g = load_rng(mr.rng);
-            pid = path_index(mr.m);
-            tp = f3(pr.tp.x, pr.tp.y, pr.tp.z);
-            eta = pr.tp.w;
-            Lr = f3(pr.L.x, pr.L.y, pr.L.z);
+            S.g = load_rng(mr.rng);
+            S.pid = path_index(mr.m);
+            S.tp = f3(pr.tp.x, pr.tp.y, pr.tp.z);
+            S.eta = pr.tp.w;
+            S.L = f3(pr.L.x, pr.L.y, pr.L.z);
+            S.prev_pdf = pr.L.w;
+            S.depth = mr.m.x;
+            S.flags = mr.m.y;
             dir = xyz(ray.d);
-            depth = mr.m.x;
-            flags = mr.m.y;
-            rid = flags >> kReqShift;
+            rid = S.flags >> kReqShift;
             const DevRequest& R = request<kMulti>(P, rid);
-            const DevScene& sc = R.sc;
-            if (!DL_IN_BOUNDS(__float_as_int(hit.w) >= 0 && __float_as_int(hit.w) < sc.num_tris, &P.cnt->err))
+            if (!DL_IN_BOUNDS(__float_as_int(hit.w) >= 0 && __float_as_int(hit.w) < R.sc.num_tris, &P.cnt->err))
                 hit.w = __int_as_float(0);
-            h = hit_info(sc, __float_as_int(hit.w), hit.y, hit.z);
-            if (T == MAT_DIFFUSE || T == MAT_ANISO_GGX) {
-                const DevMaterial& mt = sc.materials[sc.meshes[h.mesh].material];
-                if (mt.has_tex) {
-                    tuv = hit_texcoord(sc, __float_as_int(hit.w), hit.y, hit.z);
-                    // world-space normal / tangent maps (shader_common.h:62-64,
-                    // 104-107): normalize(2 rgb - 1) replaces the shading normal
-                    if (T == MAT_ANISO_GGX && mt.tex[TEX_NORMAL] >= 0) {
-                        const float3 c = tex_lookup(sc, mt.tex[TEX_NORMAL], tuv);
-                        h.sh.n = normalize(f3(__fsub_rn(__fmul_rn(c.x, 2.f), 1.f), __fsub_rn(__fmul_rn(c.y, 2.f), 1.f),
-                                              __fsub_rn(__fmul_rn(c.z, 2.f), 1.f)));
-                    }
-                    if (T == MAT_ANISO_GGX && mt.tex[TEX_TANGENT] >= 0) {
-                        const float3 c = tex_lookup(sc, mt.tex[TEX_TANGENT], tuv);
-                        s_tan = normalize(f3(__fsub_rn(__fmul_rn(c.x, 2.f), 1.f), __fsub_rn(__fmul_rn(c.y, 2.f), 1.f),
-                                             __fsub_rn(__fmul_rn(c.z, 2.f), 1.f)));
-                    }
-                }
-            }
-            int light = sc.meshes[h.mesh].light;
-            if (R.flags & DL_RENDER_NORMALS) {
-                // the normals integrator (normal.cpp:10-20): |shading normal|
-                // of the first hit, and the path ends
-                Lr = f3(fabsf(h.sh.n.x), fabsf(h.sh.n.y), fabsf(h.sh.n.z));
-                done = true;
-            } else if (flags & PF_CAMERA) {
-                if (light >= 0 && dot(h.sh.n, neg(dir)) > 0.f) Lr = add(Lr, mul(tp, ld3(sc.lights[light].radiance)));
-                depth = 0;
-            } else {
-                if (light >= 0) {
-                    const DevLight& Lt = sc.lights[light];
-                    float3 le = dot(h.sh.n, neg(dir)) > 0.f ? ld3(Lt.radiance) : f3(0.f, 0.f, 0.f);
-                    float3 vec = sub(h.p, xyz(ray.o));
-                    float3 dd = normalize(vec);
-                    float dist = length(vec);
-                    float dp = fmaxf(dot(h.sh.n, neg(dd)), 0.f);
-                    float ep = dp != 0.f ? __fdiv_rn(__fmul_rn(__fmul_rn(Lt.pA, dist), dist), dp) : 0.f;
-                    ep = with_pick_pdf(R, light, ep);
-                    float w = (flags & PF_PREV_DIFFUSE) ? mis_weight(pr.L.w, ep) : 1.f;
-                    float3 c = mul(scale(tp, w), le);
-                    Lr = add(Lr, c);
-                    if (guided) credit(P, gr, c, true);
-                }
-                if (depth > R.rr_depth) {
-                    float pq = fminf(maxc(scale(scale(tp, eta), eta)), 0.99f);
-                    if (g.next_float() > pq) done = true;
-                    else tp = divs(tp, pq);
-                }
-                depth += 1;
-            }
-            if (!done && R.max_depth > 0 && depth >= R.max_depth) done = true;
+            done = enter_vertex<T>(R, T, __float_as_int(hit.w), hit.y, hit.z, xyz(ray.o), dir, S, h, tuv, s_tan,
+                                   [&](float3 c) {
+                                       if (guided) credit(P, gr, c, true);
+                                   });
         }
         // ---- phase 2 (guided): the network on the block's 128 shading points
         const bool sampling = active && !done;
-        bool use_guide = kGuided && sampling && depth < P.gnet.max_depth;
+        bool use_guide = kGuided && sampling && S.depth < P.gnet.max_depth;
         float in6[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         float* lob = nullptr;
         if (kGuided) {
-            GuideTcSmem& S = *reinterpret_cast<GuideTcSmem*>(dyn_smem);
+            GuideTcSmem& Sm = *reinterpret_cast<GuideTcSmem*>(dyn_smem);
             const int grp = tc_group();
-            lob = tc_out_row(S, grp, tc_row());
+            lob = tc_out_row(Sm, grp, tc_row());
             if (use_guide) guide_input(request<kMulti>(P, rid).sc, h.p, normalize(h.sh.n), in6);
             // (also the barrier after which the previous tile's lobes are dead)
             if (wg_or(grp, use_guide) && net_ok) {
-                encode_row_tc(in6, S.act[grp], tc_row());
-                net_ok = guide_tc_forward(S, grp, mma_phase, &P.cnt->err);
+                encode_row_tc(in6, Sm.act[grp], tc_row());
+                net_ok = guide_tc_forward(Sm, grp, mma_phase, &P.cnt->err);
             }
             if (!net_ok) use_guide = false;  // a wait ran out: sample the BSDF alone
             if (use_guide) decode_lobes_inplace(lob);
         }
         // ---- phase 3: NEE and the next direction
         bool record = false, rotate = false;
-        float rec_pdf = 0.f;
         float3 nd = f3(0.f, 0.f, 0.f);
         if (active) {
-            const DevRequest& R = request<kMulti>(P, rid);
-            const DevScene& sc = R.sc;
-            float prev_pdf = pr.L.w;
             int target = slot;
             if (!done) {
-                DevMaterial m = sc.materials[sc.meshes[h.mesh].material];
-                if ((T == MAT_DIFFUSE || T == MAT_ANISO_GGX) && m.has_tex) {
-                    // texture lookups replace the constants (diffuse.cu:15-20,
-                    // aniso_ggx.cu:19-35)
-                    if (m.tex[TEX_ALBEDO] >= 0) {
-                        const float3 a = tex_lookup(sc, m.tex[TEX_ALBEDO], tuv);
-                        m.albedo[0] = a.x;
-                        m.albedo[1] = a.y;
-                        m.albedo[2] = a.z;
-                    }
-                    if (T == MAT_ANISO_GGX && m.tex[TEX_SPECULAR] >= 0) {
-                        const float3 a = tex_lookup(sc, m.tex[TEX_SPECULAR], tuv);
-                        m.specular[0] = a.x;
-                        m.specular[1] = a.y;
-                        m.specular[2] = a.z;
-                    }
-                    if (T == MAT_ANISO_GGX && m.tex[TEX_ALPHA] >= 0) {
-                        const float3 a = tex_lookup(sc, m.tex[TEX_ALPHA], tuv);
-                        m.ax = a.x;
-                        m.ay = a.y;
-                    }
-                }
-                Frame fr = T == MAT_ANISO_GGX ? make_onb_t(normalize(h.sh.n), s_tan) : h.sh;
-                float3 wi = to_local(fr, neg(normalize(dir)));
-                if (T == MAT_ANISO_GGX) wi = normalize(wi);
-                const float alpha = use_guide ? P.gnet.fraction : 0.f;
-                float2 s_nee = g.next2d();
-                float3 c = f3(0.f, 0.f, 0.f);
-                float3 ld = c;
-                float ldist = 0.f;
-                if (T == MAT_MIRROR || T == MAT_DIELECTRIC) {
-                    // no NEE contribution, but an envmap pick still draws its numbers
-                    float sx = s_nee.x;
-                    if (sc.env_light >= 0 && sc.num_lights > 0 && pick_light(R, sx) == sc.env_light) (void)env_xi(g);
-                } else {
-                    float lpdf;
-                    bool delta;
-                    float3 espec = sample_emitter(R, h.p, h.sh.n, s_nee, g, ld, ldist, lpdf, delta);
-                    if (__fadd_rn(__fadd_rn(espec.x, espec.y), espec.z) > 0.f && lpdf > 0.f) {
-                        BRec q1;
-                        q1.wi = wi;
-                        q1.wo = to_local(fr, ld);
-                        q1.measure = M_SOLID;
-                        q1.eta = 1.f;
-                        float3 bv = bsdf_eval<T>(m, q1);
-                        float bp = bsdf_pdf<T>(m, q1);
-                        if (use_guide) bp = alpha * stored_mixture_pdf(lob, ld) + (1.f - alpha) * bp;
-                        float w = (delta && (R.flags & DL_RENDER_FIX_POINT_LIGHT)) ? 1.f : mis_weight(lpdf, bp);
-                        c = mul(mul(scale(tp, w), bv), espec);
-                        emit = c.x != 0.f || c.y != 0.f || c.z != 0.f;
-                    }
-                }
-                BRec q2;
-                q2.wi = wi;
-                q2.wo = f3(0.f, 0.f, 0.f);
-                q2.eta = 1.f;
-                q2.measure = M_UNKNOWN;
-                if (use_guide) {
-                    // one-sample MIS between the learned mixture and the BSDF
-                    float3 fcos_over_p;
-                    if (g.next_float() < alpha) {
-                        float u0 = g.next_float();
-                        nd = stored_mixture_sample(lob, u0, g.next2d());
-                        q2.wo = to_local(fr, nd);
-                        q2.measure = M_SOLID;
-                        float3 fv = bsdf_eval<T>(m, q2);
-                        float pb = bsdf_pdf<T>(m, q2);
-                        prev_pdf = alpha * stored_mixture_pdf(lob, nd) + (1.f - alpha) * pb;
-                        fcos_over_p = prev_pdf > 0.f ? scale(fv, fmaxf(q2.wo.z, 0.f) / prev_pdf) : f3(0.f, 0.f, 0.f);
-                    } else {
-                        const float2 s2 = g.next2d();
-                        const float lobe = T == MAT_ANISO_GGX ? g.next_float() : 0.f;
-                        float3 wgt = bsdf_sample<T>(m, q2, s2, lobe);
-                        float pb = bsdf_pdf<T>(m, q2);
-                        nd = to_world(fr, q2.wo);
-                        if (T == MAT_ANISO_GGX) nd = normalize(nd);
-                        prev_pdf = alpha * stored_mixture_pdf(lob, nd) + (1.f - alpha) * pb;
-                        fcos_over_p = prev_pdf > 0.f ? scale(wgt, pb / prev_pdf) : f3(0.f, 0.f, 0.f);
-                    }
-                    tp = mul(tp, fcos_over_p);
-                    rec_pdf = prev_pdf;
-                } else {
-                    const float2 s2 = g.next2d();
-                    const float lobe = T == MAT_ANISO_GGX ? g.next_float() : 0.f;
-                    float3 f = bsdf_sample<T>(m, q2, s2, lobe);
-                    tp = mul(tp, f);
-                    eta = __fmul_rn(eta, q2.eta);
-                    prev_pdf = bsdf_pdf<T>(m, q2);
-                    nd = to_world(fr, q2.wo);
-                    if (T == MAT_ANISO_GGX) nd = normalize(nd);
-                }
-                flags = (rid << kReqShift) | (is_diffuse(T) ? PF_PREV_DIFFUSE : 0);
-                if (tp.x == 0.f && tp.y == 0.f && tp.z == 0.f) {
-                    done = true;  // every later contribution is zero
-                } else {
+                Scatter sc;
+                done = scatter_vertex<T, kGuided>(request<kMulti>(P, rid), T, rid, h, dir, tuv, s_tan, use_guide, lob,
+                                                  use_guide ? P.gnet.fraction : 0.f, S, sc);
+                nd = sc.nd;
+                emit = sc.emit;
+                if (!done) {
                     RayRec nr;
                     nr.o = make_float4(h.p.x, h.p.y, h.p.z, __int_as_float(rid));
                     nr.d = make_float4(nd.x, nd.y, nd.z, __int_as_float(0x7f800000));
                     P.rec[slot].ray = nr;
                     cont = true;
                     rotate = use_guide && P.grecords != nullptr;
-                    record = rotate && (uint32_t)(splitmix64(pid * 64ull + (unsigned long long)depth) >> 40) <
+                    record = rotate && (uint32_t)(splitmix64(S.pid * 64ull + (unsigned long long)S.depth) >> 40) <
                                            P.cnt->pass_keep;
                 }
                 if (emit) {
-                    if (done) target = -1 - (int)pid;  // lands in the stored sample
+                    if (done) target = -1 - (int)S.pid;  // lands in the stored sample
                     sh_o = make_float4(h.p.x, h.p.y, h.p.z, __int_as_float(rid));
-                    sh_d = make_float4(ld.x, ld.y, ld.z, __fsub_rn(ldist, kRayEps));
-                    sh_c = make_float4(c.x, c.y, c.z, __int_as_float(target));
+                    sh_d = make_float4(sc.ld.x, sc.ld.y, sc.ld.z, __fsub_rn(sc.ldist, kRayEps));
+                    sh_c = make_float4(sc.c.x, sc.c.y, sc.c.z, __int_as_float(target));
                 }
             }
             if (done) {
-                store_sample(P, pid, Lr, slot);
+                store_sample(P, S.pid, S.L, slot);
             } else {
                 PathRec npr;
-                npr.tp = make_float4(tp.x, tp.y, tp.z, eta);
-                npr.L = make_float4(Lr.x, Lr.y, Lr.z, prev_pdf);
+                npr.tp = make_float4(S.tp.x, S.tp.y, S.tp.z, S.eta);
+                npr.L = make_float4(S.L.x, S.L.y, S.L.z, S.prev_pdf);
                 P.rec[slot].path = npr;
                 MetaRec nmr;
-                nmr.m = make_int4(depth, flags, mr.m.z, mr.m.w);
-                nmr.rng = store_rng(g);
+                nmr.m = make_int4(S.depth, S.flags, (int)(S.pid & 0xffffffffu), (int)(S.pid >> 32));
+                nmr.rng = store_rng(S.g);
                 P.rec[slot].meta = nmr;
             }
         }
@@ -1161,14 +555,14 @@ __global__ void __launch_bounds__(kGuided ? kTcThreads : kThreads) k_material(Re
                     rc.w[0] = nd.x;
                     rc.w[1] = nd.y;
                     rc.w[2] = nd.z;
-                    rc.pdf = rec_pdf;
+                    rc.pdf = S.prev_pdf;
                     rc.L = 0.f;
                     rc.pad = 0.f;
                     static_cast<GuideRecord*>(P.cnt->pass_recs)[idx] = rc;
                 }
                 GuideRec ngr;
                 ngr.a = gr.b;
-                ngr.b = make_float4(tp.x, tp.y, tp.z, __int_as_float(idx));
+                ngr.b = make_float4(S.tp.x, S.tp.y, S.tp.z, __int_as_float(idx));
                 P.grec[slot] = ngr;
             }
         }
@@ -1510,6 +904,13 @@ struct PassValues {
 };
 static_assert(sizeof(PassValues) == 24, "pass values layout");
 
+static void check_render_error(unsigned int err) {
+    if (err & kErrBounds) throw Error(DL_ERR_QUEUE_OVERFLOW, kBoundsMessage);
+    if (err & kErrTensorWait) throw Error(DL_ERR_TIMEOUT, "tensor-core wait timed out in a guided kernel");
+    if (err & kErrRounds) throw Error(DL_ERR_TIMEOUT, "render did not converge");
+    if (err) throw Error(DL_ERR_QUEUE_OVERFLOW, "traversal stack overflow");
+}
+
 // Wavefront loop over the paths [0, total) of one pass, until every path and
 // every shadow ray has finished.  Adds the pass's counters into `acc` and
 // per-kernel times into kms.  `multi`: paths of a request table.
@@ -1595,9 +996,7 @@ static void run_wavefront(dl_context* ctx, RenderParams& P, int64_t cap, bool mu
                     kms[j] += ms;
                 }
         }
-        if (hc->err & kErrBounds) throw Error(DL_ERR_QUEUE_OVERFLOW, kBoundsMessage);
-        if (hc->err & kErrTensorWait) throw Error(DL_ERR_TIMEOUT, "tensor-core wait timed out in a guided kernel");
-        if (hc->err) throw Error(DL_ERR_QUEUE_OVERFLOW, "traversal stack overflow");
+        check_render_error(hc->err);
         if (hc->ext[0] == 0 && hc->shadow[0] == 0 && hc->next_path >= total) break;
         if (iters > 1000000) throw Error(DL_ERR_TIMEOUT, "render did not converge");
     }
@@ -1608,6 +1007,38 @@ static void run_wavefront(dl_context* ctx, RenderParams& P, int64_t cap, bool mu
     acc.stat_tris_ext += hc->stat_tris_ext;
     acc.stat_nodes_sh += hc->stat_nodes_sh;
     acc.stat_tris_sh += hc->stat_tris_sh;
+}
+
+// A pass of `total` paths runs in the resident kernel: few paths, no pool
+// size asked for, and no need for the wavefront's separate kernels (their
+// times or traversal counts, or the tuning of their launch shape).
+static bool use_resident(const dl_context* ctx, int64_t pool, unsigned long long total, bool count_traversal) {
+    return total <= kResidentMaxPaths && pool == 0 && !count_traversal && !ctx->kernel_timing && !ctx->tuning;
+}
+
+// One pass as one k_resident launch; its counters are added to `acc`.
+static void run_resident(dl_context* ctx, const RenderParams& P, bool multi, int64_t& launches, int64_t& iters,
+                         RenderCounters& acc, unsigned long long total, int spp_offset) {
+    cudaStream_t st = ctx->stream;
+    RenderBuffers& B = ctx->render;
+    DL_CUDA(cudaMemsetAsync(P.cnt, 0, sizeof(RenderCounters), st));
+    B.host_pass.ensure(sizeof(PassValues));
+    PassValues* pv = B.host_pass.as<PassValues>();
+    pv->total = total;
+    pv->spp_offset = spp_offset;
+    pv->keep = 0;
+    pv->recs = nullptr;
+    DL_CUDA(cudaMemcpyAsync(&P.cnt->pass_total, pv, sizeof(PassValues), cudaMemcpyHostToDevice, st));
+    resident_launch(ctx->num_sms > 0 ? ctx->num_sms : 152, P, multi, total, st);
+    launches += 1;
+    iters += 1;
+    RenderCounters* hc = B.host_counters.as<RenderCounters>();
+    DL_CUDA(cudaMemcpyAsync(hc, P.cnt, sizeof(RenderCounters), cudaMemcpyDeviceToHost, st));
+    DL_CUDA(cudaStreamSynchronize(st));
+    check_render_error(hc->err);
+    acc.stat_camera += total;
+    acc.stat_ext += hc->stat_ext;
+    acc.stat_shadow += hc->stat_shadow;
 }
 
 // Budget of the per-path sample buffer; larger frames render in passes of
@@ -1672,7 +1103,8 @@ void render_run(dl_scene* S, const dl_render_opts& o, float* d_film, int64_t li_
     const int spp = std::max(o.spp, 1);
     int chunk_spp = P.mode == 1 ? 1 : (int)std::max<size_t>(1, std::min<size_t>(spp, kSampleBufferBytes / (npix * 16)));
     unsigned long long chunk_total = P.mode == 1 ? (unsigned long long)li_n : npix * (unsigned long long)chunk_spp;
-    const int64_t cap = pool_capacity(ctx, o.max_paths_in_flight, chunk_total);
+    const bool resident = use_resident(ctx, o.max_paths_in_flight, chunk_total, count_traversal);
+    const int64_t cap = resident ? 32 : pool_capacity(ctx, o.max_paths_in_flight, chunk_total);
     RenderBuffers& B = ctx->render;
     B.ensure(cap);
     bind_pool(P, B);
@@ -1689,7 +1121,9 @@ void render_run(dl_scene* S, const dl_render_opts& o, float* d_film, int64_t li_
     std::memset(&acc, 0, sizeof(acc));
     DL_CUDA(cudaEventRecord(ctx->ev0, st));
     unsigned long long invalid = 0;
-    if (P.mode == 1) {
+    if (P.mode == 1 && resident) {
+        run_resident(ctx, P, false, launches, iters, acc, (unsigned long long)li_n, 0);
+    } else if (P.mode == 1) {
         run_wavefront(ctx, P, cap, false, count_traversal, kms, launches, iters, acc, (unsigned long long)li_n, 0,
                       1u << 24);
     } else {
@@ -1698,8 +1132,11 @@ void render_run(dl_scene* S, const dl_render_opts& o, float* d_film, int64_t li_
         dim3 fgrid((F.cols + kFilmTile - 1) / kFilmTile, (F.rows + kFilmTile - 1) / kFilmTile);
         for (int s0 = 0; s0 < spp; s0 += chunk_spp) {
             int ns = std::min(chunk_spp, spp - s0);
-            run_wavefront(ctx, P, cap, false, count_traversal, kms, launches, iters, acc,
-                          npix * (unsigned long long)ns, o.spp_offset + s0, 1u << 24);
+            if (resident)
+                run_resident(ctx, P, false, launches, iters, acc, npix * (unsigned long long)ns, o.spp_offset + s0);
+            else
+                run_wavefront(ctx, P, cap, false, count_traversal, kms, launches, iters, acc,
+                              npix * (unsigned long long)ns, o.spp_offset + s0, 1u << 24);
             F.nspp = ns;
             F.s_first = o.spp_offset + s0;
             F.accumulate = s0 > 0;
@@ -1888,7 +1325,8 @@ void render_batch(dl_context* ctx, const BatchItem* items, int n, bool count_tra
     }
     int64_t requested = 0;
     for (int r = 0; r < n; r++) requested = std::max<int64_t>(requested, items[r].opts.max_paths_in_flight);
-    const int64_t cap = pool_capacity(ctx, requested, max_pass);
+    const bool resident = use_resident(ctx, requested, max_pass, count_traversal);
+    const int64_t cap = resident ? 32 : pool_capacity(ctx, requested, max_pass);
     B.ensure(cap);
     B.samples.ensure((size_t)std::max<unsigned long long>(max_pass, 1) * 16);
     B.requests.ensure(sizeof(DevRequest) * (size_t)std::max(n, 1));
@@ -1928,7 +1366,8 @@ void render_batch(dl_context* ctx, const BatchItem* items, int n, bool count_tra
         // the pass's request table; the copy is ordered before the pass's kernels
         DL_CUDA(cudaMemcpyAsync(B.requests.ptr, hreq, sizeof(DevRequest) * na, cudaMemcpyHostToDevice, st));
         P.num_reqs = na;
-        run_wavefront(ctx, P, cap, true, count_traversal, kms, launches, iters, acc, first, 0, 1u << 24);
+        if (resident) run_resident(ctx, P, true, launches, iters, acc, first, 0);
+        else run_wavefront(ctx, P, cap, true, count_traversal, kms, launches, iters, acc, first, 0, 1u << 24);
         for (int a = 0; a < na; a++) {
             const int r = active[a];
             const DevCamera& cam = items[r].cam;
