@@ -421,9 +421,45 @@ __global__ void __launch_bounds__(kThreads) k_miss(RenderParams P, int p) {
 // same combined pdf.  The vertex becomes a training record.
 constexpr size_t kGuidedSmem = sizeof(GuideTcSmem);
 
+// A warp's 32 slot records on their way to shared memory: eight lanes fetch
+// one 128-byte line each, four lines an instruction, and chunk c of lane l's
+// record lands at chunk c ^ (l & 7) of line l (no bank conflicts when each
+// lane reads its own record).
+__device__ __forceinline__ void fetch_slots(const SlotRec* rec, int slot, float4* line) {
+    const int lane = lane_id(), c = lane & 7;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const int l = 4 * j + (lane >> 3);
+        const int s = __shfl_sync(0xffffffffu, slot, l);
+        if (s >= 0)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::
+                         "r"((uint32_t)__cvta_generic_to_shared(line + 8 * l + (c ^ (l & 7)))),
+                         "l"(reinterpret_cast<const float4*>(rec + s) + c) : "memory");
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+__device__ __forceinline__ float4 fetched(const float4* line, int c) {
+    const int l = lane_id();
+    return line[8 * l + (c ^ (l & 7))];
+}
+
+// Threads per SM of the plain kernels (80 registers each).  The records of a
+// warp's next 32 entries travel to shared memory while it shades the present
+// ones; loaded where they were used, DRAM latency left the kernels at 40 % of
+// the issue slots (shading, serialised, before -> with 768 | 896 | 1024
+// threads: material spheres 11.5 -> 10.5 | 11.6 | 12.0 ms, MIS plates 64 spp
+// 11.7 -> 10.4 | 10.8 | 9.5, Cornell 512x512 32 spp 2.9 -> 2.6 | 2.9 | 3.0,
+// window-lit room 4.4 -> 3.9 | 4.2 | 3.9; the smaller register budgets spill
+// in the GGX kernel).
+constexpr int kMaterialThreads = 768;
+
 template <int T, bool kMulti, bool kGuided, int kThreads>
-__global__ void __launch_bounds__(kGuided ? kTcThreads : kThreads) k_material(RenderParams P, int p) {
+__global__ void __launch_bounds__(kGuided ? kTcThreads : kThreads, kGuided ? 2 : kMaterialThreads / kThreads)
+    k_material(RenderParams P, int p) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
+    // the warps' next records (not in the guided kernels, whose shared memory
+    // holds the network)
+    __shared__ __align__(128) float4 s_line[kGuided ? 1 : kThreads / 32][kGuided ? 1 : 8 * 32];
     const int q = p ^ 1;
     const int lane = lane_id();
     int n = P.cnt->mat[p][T].n;
@@ -442,11 +478,19 @@ __global__ void __launch_bounds__(kGuided ? kTcThreads : kThreads) k_material(Re
         if ((int)blockIdx.x * kTcThreads >= n) return;
         net_ok = guide_tc_begin(*reinterpret_cast<GuideTcSmem*>(dyn_smem), P.gnet.image, &P.cnt->err);
     }
-    for (int i0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~(kSpan - 1); i0 < n; i0 += gridDim.x * blockDim.x) {
-        int i = i0 + (kGuided ? tc_row() : lane);
-        bool active = i < n;
-        int slot = active ? P.mat_q[T][i] : 0;
-        if (active && !slot_ok(P, slot)) active = false;
+    const int first = (blockIdx.x * blockDim.x + threadIdx.x) & ~(kSpan - 1), stride = gridDim.x * blockDim.x;
+    // queue entry i's slot, -1 past the queue's end
+    auto queued = [&](int i) {
+        const int s = i < n ? P.mat_q[T][i] : -1;
+        return s < 0 || slot_ok(P, s) ? s : -1;
+    };
+    float4* const line = s_line[kGuided ? 0 : threadIdx.x >> 5];
+    int next = kGuided ? -1 : queued(first + lane), after = kGuided ? -1 : queued(first + stride + lane);
+    if (!kGuided && first < n) fetch_slots(P.rec, next, line);
+    for (int i0 = first; i0 < n; i0 += stride) {
+        int slot = kGuided ? queued(i0 + tc_row()) : next;
+        const bool active = slot >= 0;
+        if (!active) slot = 0;
         bool cont = false, emit = false, done = false;
         float4 sh_o = make_float4(0.f, 0.f, 0.f, 0.f), sh_d = sh_o, sh_c = sh_o;
         // ---- phase 1: emitter hit, Russian roulette, depth limit
@@ -460,11 +504,37 @@ __global__ void __launch_bounds__(kGuided ? kTcThreads : kThreads) k_material(Re
         S.tp = dir;
         S.pid = 0;
         S.depth = 0;
+        float4 hit;
+        RayRec ray;
+        PathRec pr;
+        MetaRec mr;
+        if (kGuided) {
+            if (active) {
+                hit = P.rec[slot].hit.h;
+                ray = P.rec[slot].ray;
+                pr = P.rec[slot].path;
+                mr = P.rec[slot].meta;
+            }
+        } else {
+            // this round's records have arrived; the next round's travel
+            // while this one is computed
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+            __syncwarp();
+            ray.o = fetched(line, 0);
+            ray.d = fetched(line, 1);
+            hit = fetched(line, 2);
+            pr.tp = fetched(line, 4);
+            pr.L = fetched(line, 5);
+            const float4 m0 = fetched(line, 6), m1 = fetched(line, 7);
+            mr.m = make_int4(__float_as_int(m0.x), __float_as_int(m0.y), __float_as_int(m0.z), __float_as_int(m0.w));
+            mr.rng = make_uint4(__float_as_uint(m1.x), __float_as_uint(m1.y), __float_as_uint(m1.z),
+                                __float_as_uint(m1.w));
+            __syncwarp();
+            next = after;
+            if (i0 + stride < n) fetch_slots(P.rec, next, line);
+            after = queued(i0 + 2 * stride + lane);
+        }
         if (active) {
-            float4 hit = P.rec[slot].hit.h;
-            const RayRec ray = P.rec[slot].ray;
-            const PathRec pr = P.rec[slot].path;
-            const MetaRec mr = P.rec[slot].meta;
             if (guided) gr = P.grec[slot];
             S.g = load_rng(mr.rng);
             S.pid = path_index(mr.m);
