@@ -651,23 +651,33 @@ __global__ void __launch_bounds__(kGuided ? kTcThreads : kThreads, kGuided ? 2 :
 }
 
 // Film accumulation as a gather (the reference splats each sample with
-// ImageBlock::put, src/core/bitmap/block.cpp:81-113).  One block owns a
-// 32x32 tile of film pixels; per sample index it stages the samples of the
-// 36x36 image pixels around it (radiance from the sample buffer, film
-// position recomputed from the path's pcg32 stream: its first 2D draw) in
-// shared memory together with their 5 x and 5 y filter weights (the
-// reference's table lookup).  Each thread then owns four film pixels of one
-// column and sums the weighted samples of their 5x5 neighbourhoods; a staged
-// sample's radiance and x weight are read once for all four.  Every pixel
-// sums in a fixed order (sample index, then row, then column): no atomics,
-// bit-reproducible films.  Samples the film rejects (NaN, Inf or negative:
-// ImageBlock::put block.cpp:82-88) get zero weight and are counted.
-constexpr int kFilmTile = 32, kFilmApron = 2, kFilmRegion = kFilmTile + 2 * kFilmApron, kFilmRows = 4;
-constexpr int kFilmCells = kFilmRegion * kFilmRegion;
+// ImageBlock::put, src/core/bitmap/block.cpp:81-113).  One block of 256
+// threads owns a tile of kTile x kTile film pixels; per sample index it
+// stages the samples of the (kTile + 4)^2 image pixels around it (radiance
+// from the sample buffer, film position recomputed from the path's pcg32
+// stream: its first 2D draw) in shared memory together with their 5 x and 5 y
+// filter weights (the reference's table lookup).  Each thread then owns
+// kFilmRows film pixels of one column and sums the weighted samples of their
+// 5x5 neighbourhoods; a staged sample's radiance and x weight are read once
+// for all of them.  Every pixel sums in a fixed order (sample index, then
+// row, then column): no atomics, bit-reproducible films.  Samples the film
+// rejects (NaN, Inf or negative: ImageBlock::put block.cpp:82-88) get zero
+// weight and are counted.
+//
+// The next sample's radiances are loaded while the present one is summed.
+// Two tile sizes: 32 (four rows a thread) moves the fewest bytes and
+// instructions a pixel, 16 (one row a thread) has four times the blocks and a
+// shorter chain a sample, for frames whose tiles of 32 leave the chip idle.
+constexpr int kFilmApron = 2, kFilmThreads = 256;
 constexpr int kFilmTaps = 2 * kFilmApron + 1;  // 5 film pixels per axis around a sample
-constexpr int kFilmThreads = kFilmTile * kFilmTile / kFilmRows;
-// staged per cell: r, g, b, 5 x weights, 5 y weights
-constexpr size_t kFilmSmem = (size_t)(3 + 2 * kFilmTaps) * kFilmCells * sizeof(float);
+template <int kTile>
+struct FilmTile {
+    static constexpr int kRegion = kTile + 2 * kFilmApron, kCells = kRegion * kRegion;
+    static constexpr int kRows = kTile * kTile / kFilmThreads;                       // film pixels of a thread
+    static constexpr int kOwn = (kCells + kFilmThreads - 1) / kFilmThreads;          // staged cells of a thread
+    // staged per cell: r, g, b, 5 x weights, 5 y weights
+    static constexpr size_t kSmem = (size_t)(3 + 2 * kFilmTaps) * kCells * sizeof(float);
+};
 
 struct FilmParams {
     float4* film;
@@ -682,56 +692,68 @@ struct FilmParams {
     int accumulate;       // add to the film instead of overwriting it
 };
 
-__global__ void __launch_bounds__(kFilmThreads) k_film_gather(FilmParams F) {
+template <int kTile>
+__global__ void __launch_bounds__(kFilmThreads, kTile == 32 ? 3 : 4)
+    k_film_gather(FilmParams F) {
+    using Tile = FilmTile<kTile>;
+    constexpr int kRows = Tile::kRows, kCells = Tile::kCells, kRegion = Tile::kRegion;
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     float* const s_r = reinterpret_cast<float*>(dyn_smem);
-    float* const s_g = s_r + kFilmCells;
-    float* const s_b = s_g + kFilmCells;
-    float* const s_wx = s_b + kFilmCells;               // [kFilmTaps][kFilmCells]
-    float* const s_wy = s_wx + kFilmTaps * kFilmCells;  // [kFilmTaps][kFilmCells]
+    float* const s_g = s_r + kCells;
+    float* const s_b = s_g + kCells;
+    float* const s_wx = s_b + kCells;               // [kFilmTaps][kCells]
+    float* const s_wy = s_wx + kFilmTaps * kCells;  // [kFilmTaps][kCells]
     __shared__ float s_table[33];
     __shared__ unsigned int s_invalid;
-    const int tx = threadIdx.x % kFilmTile, ty = threadIdx.x / kFilmTile;  // column, group of 4 rows
-    const int X0 = blockIdx.x * kFilmTile, Y0 = blockIdx.y * kFilmTile;
-    const int X = X0 + tx, Yb = Y0 + kFilmRows * ty;
+    const int tx = threadIdx.x % kTile, ty = threadIdx.x / kTile;  // column, group of kRows rows
+    const int X0 = blockIdx.x * kTile, Y0 = blockIdx.y * kTile;
+    const int X = X0 + tx, Yb = Y0 + kRows * ty;
     const int IX0 = X0 - F.border - kFilmApron, IY0 = Y0 - F.border - kFilmApron;
     const size_t npix = (size_t)F.w * F.h;
     if (threadIdx.x < 33) s_table[threadIdx.x] = F.table[threadIdx.x];
     if (threadIdx.x == 0) s_invalid = 0;
-    __syncthreads();
-    float ar[kFilmRows], ag[kFilmRows], ab[kFilmRows], aw[kFilmRows];
+    // the thread's cells' samples of index k (w = 0 outside the image)
+    float4 L[Tile::kOwn];
+    auto load = [&](int k) {
 #pragma unroll
-    for (int j = 0; j < kFilmRows; j++) ar[j] = ag[j] = ab[j] = aw[j] = 0.f;
+        for (int j = 0; j < Tile::kOwn; j++) {
+            const int e = threadIdx.x + j * kFilmThreads;
+            const int sx = IX0 + e % kRegion, sy = IY0 + e / kRegion;
+            L[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (e < kCells && sx >= 0 && sx < F.w && sy >= 0 && sy < F.h)
+                L[j] = F.samples[(size_t)k * npix + (size_t)sy * F.w + sx];
+        }
+    };
+    load(0);
+    __syncthreads();
+    float ar[kRows], ag[kRows], ab[kRows], aw[kRows];
+#pragma unroll
+    for (int j = 0; j < kRows; j++) ar[j] = ag[j] = ab[j] = aw[j] = 0.f;
     for (int k = 0; k < F.nspp; k++) {
-        for (int e = threadIdx.x; e < kFilmCells; e += kFilmThreads) {
-            const int rx = e % kFilmRegion, ry = e / kFilmRegion;
+#pragma unroll
+        for (int j = 0; j < Tile::kOwn; j++) {
+            const int e = threadIdx.x + j * kFilmThreads;
+            if (e >= kCells) break;
+            const int rx = e % kRegion, ry = e / kRegion;
             const int sx = IX0 + rx, sy = IY0 + ry;
-            float L0 = 0.f, L1 = 0.f, L2 = 0.f;
-            bool ok = false;
+            const bool ok = L[j].w != 0.f && L[j].x >= 0.f && L[j].y >= 0.f && L[j].z >= 0.f && isfinite(L[j].x) &&
+                            isfinite(L[j].y) && isfinite(L[j].z);
+            // each sample is counted by the tile that owns its pixel
+            if (!ok && L[j].w != 0.f && rx >= kFilmApron && rx < kFilmApron + kTile && ry >= kFilmApron &&
+                ry < kFilmApron + kTile)
+                atomicAdd(&s_invalid, 1u);
             float px = 0.f, py = 0.f;
-            if (sx >= 0 && sx < F.w && sy >= 0 && sy < F.h) {
-                float4 L = F.samples[(size_t)k * npix + (size_t)sy * F.w + sx];
-                ok = L.w != 0.f && L.x >= 0.f && L.y >= 0.f && L.z >= 0.f && isfinite(L.x) && isfinite(L.y) &&
-                     isfinite(L.z);
-                // each sample is counted by the tile that owns its pixel
-                if (!ok && L.w != 0.f && rx >= kFilmApron && rx < kFilmApron + kFilmTile && ry >= kFilmApron &&
-                    ry < kFilmApron + kFilmTile)
-                    atomicAdd(&s_invalid, 1u);
-                if (ok) {
-                    Pcg32 g;
-                    seed_path(g, F.seed_mix, F.w, F.h, sx, sy, F.s_first + k);
-                    float2 ps = g.next2d();
-                    float fx = __fadd_rn((float)sx, ps.x), fy = __fadd_rn((float)sy, ps.y);
-                    px = __fsub_rn(__fsub_rn(fx, 0.5f), (float)(-F.border));
-                    py = __fsub_rn(__fsub_rn(fy, 0.5f), (float)(-F.border));
-                    L0 = L.x;
-                    L1 = L.y;
-                    L2 = L.z;
-                }
+            if (ok) {
+                Pcg32 g;
+                seed_path(g, F.seed_mix, F.w, F.h, sx, sy, F.s_first + k);
+                float2 ps = g.next2d();
+                float fx = __fadd_rn((float)sx, ps.x), fy = __fadd_rn((float)sy, ps.y);
+                px = __fsub_rn(__fsub_rn(fx, 0.5f), (float)(-F.border));
+                py = __fsub_rn(__fsub_rn(fy, 0.5f), (float)(-F.border));
             }
-            s_r[e] = L0;
-            s_g[e] = L1;
-            s_b[e] = L2;
+            s_r[e] = ok ? L[j].x : 0.f;
+            s_g[e] = ok ? L[j].y : 0.f;
+            s_b[e] = ok ? L[j].z : 0.f;
             // weights of this sample for film columns X0 + rx - d and rows Y0 + ry - d
 #pragma unroll
             for (int d = 0; d < kFilmTaps; d++) {
@@ -741,25 +763,26 @@ __global__ void __launch_bounds__(kFilmThreads) k_film_gather(FilmParams F) {
                     wx = s_table[min((int)__fmul_rn(fabsf(__fsub_rn((float)cx, px)), F.lookup), 32)];
                 if (ok && cy >= 0 && cy < F.rows)
                     wy = s_table[min((int)__fmul_rn(fabsf(__fsub_rn((float)cy, py)), F.lookup), 32)];
-                s_wx[d * kFilmCells + e] = wx;
-                s_wy[d * kFilmCells + e] = wy;
+                s_wx[d * kCells + e] = wx;
+                s_wy[d * kCells + e] = wy;
             }
         }
         __syncthreads();
-        // region rows kFilmRows*ty + r reach this thread's pixel j when
+        if (k + 1 < F.nspp) load(k + 1);
+        // region rows kRows*ty + r reach this thread's pixel j when
         // dy = r - j is a filter tap; per pixel the order is dy, then dx
 #pragma unroll
-        for (int r = 0; r < kFilmRows + kFilmTaps - 1; r++) {
+        for (int r = 0; r < kRows + kFilmTaps - 1; r++) {
 #pragma unroll
             for (int dx = 0; dx < kFilmTaps; dx++) {
-                const int c = (kFilmRows * ty + r) * kFilmRegion + tx + dx;
-                const float wx = s_wx[dx * kFilmCells + c];
+                const int c = (kRows * ty + r) * kRegion + tx + dx;
+                const float wx = s_wx[dx * kCells + c];
                 const float R = __fmul_rn(s_r[c], wx), G = __fmul_rn(s_g[c], wx), B = __fmul_rn(s_b[c], wx);
 #pragma unroll
-                for (int j = 0; j < kFilmRows; j++) {
+                for (int j = 0; j < kRows; j++) {
                     const int dy = r - j;
                     if (dy < 0 || dy >= kFilmTaps) continue;
-                    const float wy = s_wy[dy * kFilmCells + c];
+                    const float wy = s_wy[dy * kCells + c];
                     ar[j] = __fmaf_rn(R, wy, ar[j]);
                     ag[j] = __fmaf_rn(G, wy, ag[j]);
                     ab[j] = __fmaf_rn(B, wy, ab[j]);
@@ -772,7 +795,7 @@ __global__ void __launch_bounds__(kFilmThreads) k_film_gather(FilmParams F) {
     if (threadIdx.x == 0 && s_invalid) atomicAdd(F.invalid, (unsigned long long)s_invalid);
     if (X >= F.cols) return;
 #pragma unroll
-    for (int j = 0; j < kFilmRows; j++) {
+    for (int j = 0; j < kRows; j++) {
         const int Y = Yb + j;
         if (Y >= F.rows) break;
         float4* o = F.film + (size_t)Y * F.cols + X;
@@ -786,10 +809,29 @@ __global__ void __launch_bounds__(kFilmThreads) k_film_gather(FilmParams F) {
     }
 }
 
+template <int kTile>
+static void launch_film(const FilmParams& F, cudaStream_t st) {
+    const dim3 grid((F.cols + kTile - 1) / kTile, (F.rows + kTile - 1) / kTile);
+    k_film_gather<kTile><<<grid, kFilmThreads, FilmTile<kTile>::kSmem, st>>>(F);
+    DL_CUDA(cudaGetLastError());
+}
+
+// The gather of F's samples, on tiles of 32 when there is at least one per
+// SM.  Whole renders of an empty scene, device ms (tiles of 16 | of 32 | of
+// 32 before the prefetch): 64x64 64 spp 0.22 | 0.46 | 0.49; 256x256 16 spp
+// 0.14 | 0.19 | 0.27; 400x300 17 spp 0.22 | 0.22; 517x389 9 spp 0.19 | 0.17;
+// 1080p 64 spp 19.6 | 16.8 | 17.0.
+static void film_gather(const FilmParams& F, int sms, cudaStream_t st) {
+    const int64_t tiles = (int64_t)((F.cols + 31) / 32) * ((F.rows + 31) / 32);
+    if (tiles >= sms) launch_film<32>(F, st);
+    else launch_film<16>(F, st);
+}
+
 // Per device, once per context: kernels whose shared memory exceeds the
 // default 48 KB limit.
 void render_setup_device() {
-    DL_CUDA(cudaFuncSetAttribute(k_film_gather, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFilmSmem));
+    DL_CUDA(cudaFuncSetAttribute(k_film_gather<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)FilmTile<32>::kSmem));
 }
 
 // film -> rgb (ImageBlock::toBitmap, block.cpp:58-66)
@@ -1199,7 +1241,6 @@ void render_run(dl_scene* S, const dl_render_opts& o, float* d_film, int64_t li_
     } else {
         FilmParams F = film_params(cam, P.r0, o.filter, d_film, P.samples, B.invalid.as<unsigned long long>());
         DL_CUDA(cudaMemsetAsync(F.invalid, 0, sizeof(unsigned long long), st));
-        dim3 fgrid((F.cols + kFilmTile - 1) / kFilmTile, (F.rows + kFilmTile - 1) / kFilmTile);
         for (int s0 = 0; s0 < spp; s0 += chunk_spp) {
             int ns = std::min(chunk_spp, spp - s0);
             if (resident)
@@ -1210,9 +1251,8 @@ void render_run(dl_scene* S, const dl_render_opts& o, float* d_film, int64_t li_
             F.nspp = ns;
             F.s_first = o.spp_offset + s0;
             F.accumulate = s0 > 0;
-            k_film_gather<<<fgrid, kFilmThreads, kFilmSmem, st>>>(F);
+            film_gather(F, ctx->num_sms, st);
             launches += 1;
-            DL_CUDA(cudaGetLastError());
         }
         unsigned long long* hinv =
             reinterpret_cast<unsigned long long*>(B.host_counters.as<char>() + sizeof(RenderCounters));
@@ -1304,7 +1344,6 @@ void render_guided(dl_scene* S, const dl_render_opts& o, dl_guide* G, float* d_f
     DL_CUDA(cudaEventRecord(ctx->ev0, st));
     FilmParams F = film_params(cam, P.r0, o.filter, d_film, P.samples, B.invalid.as<unsigned long long>());
     DL_CUDA(cudaMemsetAsync(F.invalid, 0, sizeof(unsigned long long), st));
-    dim3 fgrid((F.cols + kFilmTile - 1) / kFilmTile, (F.rows + kFilmTile - 1) / kFilmTile);
     RenderCounters* hc = B.host_counters.as<RenderCounters>();
     int done = 0;
     bool trained[2] = {false, false};
@@ -1328,9 +1367,8 @@ void render_guided(dl_scene* S, const dl_render_opts& o, dl_guide* G, float* d_f
         F.nspp = ns;
         F.s_first = o.spp_offset + done;
         F.accumulate = done > 0;
-        k_film_gather<<<fgrid, kFilmThreads, kFilmSmem, st>>>(F);
+        film_gather(F, ctx->num_sms, st);
         launches += 1;
-        DL_CUDA(cudaGetLastError());
         done += ns;
         const int steps = G->cfg.steps_per_pass;
         if (train && nrec >= 16 * (int64_t)std::max(1, steps) && done < spp) {
@@ -1446,10 +1484,8 @@ void render_batch(dl_context* ctx, const BatchItem* items, int n, bool count_tra
             F.nspp = ns[a];
             F.s_first = hreq[a].spp_offset;
             F.accumulate = done[r] > 0;
-            dim3 fgrid((F.cols + kFilmTile - 1) / kFilmTile, (F.rows + kFilmTile - 1) / kFilmTile);
-            k_film_gather<<<fgrid, kFilmThreads, kFilmSmem, st>>>(F);
+                film_gather(F, ctx->num_sms, st);
             launches += 1;
-            DL_CUDA(cudaGetLastError());
             done[r] += ns[a];
         }
         // host_requests is rewritten next pass: wait for this pass's copy
