@@ -2,6 +2,7 @@
 // staging and dispatch to the scene builder, the trace kernels and the
 // wavefront renderer.
 #include <cuda_runtime.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cmath>
@@ -105,6 +106,10 @@ int dl_context_create(int device, dl_context** out) {
         DL_CUDA(cudaEventCreate(&ctx->ev0));
         DL_CUDA(cudaEventCreate(&ctx->ev1));
         DL_CUDA(cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device));
+        int direct = 0;
+        DL_CUDA(cudaDeviceGetAttribute(&direct, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device));
+        ctx->host_direct = direct != 0;
+        ctx->words.ensure(64);
         for (int i = 0; i < dl_context::kAux; i++) {
             DL_CUDA(cudaStreamCreateWithFlags(&ctx->aux[i], cudaStreamNonBlocking));
             DL_CUDA(cudaEventCreateWithFlags(&ctx->join_ev[i], cudaEventDisableTiming));
@@ -188,7 +193,7 @@ int dl_trace_closest_device(dl_scene* S, const float* d_rays, int64_t n, float* 
     return guard(ctx, [&] {
         need(n >= 0 && (n == 0 || (d_rays && d_hits)), "bad ray buffers");
         ctx->trace.occ.ensure(64);
-        dl::trace_closest_launch(S, d_rays, n, d_hits, ctx->trace.occ.ptr, false);
+        dl::trace_closest_launch(S, d_rays, n, d_hits, ctx->trace.occ.ptr);
     });
 }
 
@@ -198,9 +203,66 @@ int dl_trace_any_device(dl_scene* S, const float* d_rays, int64_t n, uint8_t* d_
     return guard(ctx, [&] {
         need(n >= 0 && (n == 0 || (d_rays && d_occ)), "bad ray buffers");
         ctx->trace.occ.ensure(64);
-        dl::trace_any_launch(S, d_rays, n, d_occ, ctx->trace.occ.ptr, false);
+        dl::trace_any_launch(S, d_rays, n, d_occ, ctx->trace.occ.ptr);
     });
 }
+
+}  // extern "C"
+
+namespace {
+
+// Whether the kernels take host array `p` of `bytes` bytes as it is: the
+// device shares the host's page tables and the array has the alignment of the
+// kernels' accesses.  An input's ends are read here, so that a bad pointer
+// fails on the host as it does in a copy.
+bool direct_in(const dl_context* ctx, const void* p, size_t bytes, size_t align) {
+    if (!ctx->host_direct || bytes == 0 || reinterpret_cast<uintptr_t>(p) % align != 0) return false;
+    const volatile char* c = static_cast<const char*>(p);
+    (void)c[0];
+    (void)c[bytes - 1];
+    return true;
+}
+bool direct_out(const dl_context* ctx, const void* p, size_t align) {
+    return ctx->host_direct && reinterpret_cast<uintptr_t>(p) % align == 0;
+}
+// Before a kernel writes host array `p`: touches each of its pages.  A fresh
+// page costs 2.5 us here, 20 us when the device is the first to write it (and
+// a bad pointer fails on the host).
+void touch_pages(void* p, size_t bytes) {
+    static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    volatile char* c = static_cast<char*>(p);
+    for (size_t i = 0; i < bytes; i += page) c[i] = 0;
+    c[bytes - 1] = 0;
+}
+
+// `rays` where the traversal kernel reads them: in place, or copied.
+const float* rays_on_device(dl_context* ctx, const float* rays, int64_t n) {
+    const size_t bytes = (size_t)n * 32;
+    if (direct_in(ctx, rays, bytes, 16)) return rays;
+    ctx->trace.rays.ensure(bytes);
+    DL_CUDA(cudaMemcpyAsync(ctx->trace.rays.ptr, rays, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    return ctx->trace.rays.as<float>();
+}
+
+// The end of a host ray batch: waits for the stream and checks the error word.
+void finish_rays(dl_context* ctx) {
+    cudaStream_t st = ctx->stream;
+    unsigned* err = ctx->words.as<unsigned>();
+    DL_CUDA(cudaMemcpyAsync(err, ctx->trace.occ.ptr, 4, cudaMemcpyDeviceToHost, st));
+    DL_CUDA(cudaEventRecord(ctx->ev1, st));
+    DL_CUDA(cudaStreamSynchronize(st));
+    if (*err & 4u)
+        throw dl::Error(DL_ERR_QUEUE_OVERFLOW, "bounds check failed: a node or triangle index outside its array "
+                                               "(bounds-checked build)");
+    if (*err) throw dl::Error(DL_ERR_QUEUE_OVERFLOW, "traversal stack overflow");
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
+    ctx->stats.trace_ms = ms;
+}
+
+}  // namespace
+
+extern "C" {
 
 int dl_trace_closest(dl_scene* S, const float* rays, int64_t n, int32_t* prim_id, float* t, float* u, float* v) {
     if (!S) return DL_ERR_INVALID_ARG;
@@ -210,32 +272,26 @@ int dl_trace_closest(dl_scene* S, const float* rays, int64_t n, int32_t* prim_id
         if (n == 0) return;
         cudaStream_t st = ctx->stream;
         dl::TraceBuffers& B = ctx->trace;
-        B.rays.ensure((size_t)n * 32);
-        B.hits.ensure((size_t)n * 16);
+        const size_t f = (size_t)n * 4;
+        B.hits.ensure(4 * f);
         B.occ.ensure(64);
-        B.stage.ensure((size_t)n * 16);
+        const bool direct = direct_out(ctx, prim_id, 4) && direct_out(ctx, t, 4) && direct_out(ctx, u, 4) &&
+                            direct_out(ctx, v, 4);
+        if (!direct) B.split.ensure(4 * f);
         DL_CUDA(cudaEventRecord(ctx->ev0, st));
-        DL_CUDA(cudaMemcpyAsync(B.rays.ptr, rays, (size_t)n * 32, cudaMemcpyHostToDevice, st));
-        dl::trace_closest_launch(S, B.rays.as<float>(), n, B.hits.as<float>(), B.occ.ptr, false);
-        DL_CUDA(cudaMemcpyAsync(B.stage.ptr, B.hits.ptr, (size_t)n * 16, cudaMemcpyDeviceToHost, st));
-        unsigned int err = 0;
-        DL_CUDA(cudaMemcpyAsync(&err, B.occ.ptr, 4, cudaMemcpyDeviceToHost, st));
-        DL_CUDA(cudaEventRecord(ctx->ev1, st));
-        DL_CUDA(cudaStreamSynchronize(st));
-        if (err & 4u)
-            throw dl::Error(DL_ERR_QUEUE_OVERFLOW, "bounds check failed: a node or triangle index outside its array "
-                                                   "(bounds-checked build)");
-        if (err) throw dl::Error(DL_ERR_QUEUE_OVERFLOW, "traversal stack overflow");
-        const float* h = B.stage.as<float>();
-        for (int64_t i = 0; i < n; i++) {
-            t[i] = h[4 * i];
-            u[i] = h[4 * i + 1];
-            v[i] = h[4 * i + 2];
-            std::memcpy(&prim_id[i], &h[4 * i + 3], 4);
+        dl::trace_closest_launch(S, rays_on_device(ctx, rays, n), n, B.hits.as<float>(), B.occ.ptr);
+        if (direct) {
+            for (void* p : {(void*)prim_id, (void*)t, (void*)u, (void*)v}) touch_pages(p, f);  // (while the rays are traced)
+            dl::split_hits_launch(ctx, B.hits.as<float>(), n, prim_id, t, u, v);
+        } else {
+            float* s = B.split.as<float>();
+            dl::split_hits_launch(ctx, B.hits.as<float>(), n, reinterpret_cast<int32_t*>(s), s + n, s + 2 * n, s + 3 * n);
+            DL_CUDA(cudaMemcpyAsync(prim_id, s, f, cudaMemcpyDeviceToHost, st));
+            DL_CUDA(cudaMemcpyAsync(t, s + n, f, cudaMemcpyDeviceToHost, st));
+            DL_CUDA(cudaMemcpyAsync(u, s + 2 * n, f, cudaMemcpyDeviceToHost, st));
+            DL_CUDA(cudaMemcpyAsync(v, s + 3 * n, f, cudaMemcpyDeviceToHost, st));
         }
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-        ctx->stats.trace_ms = ms;
+        finish_rays(ctx);
     });
 }
 
@@ -247,26 +303,21 @@ int dl_trace_any(dl_scene* S, const float* rays, int64_t n, uint8_t* occluded) {
         if (n == 0) return;
         cudaStream_t st = ctx->stream;
         dl::TraceBuffers& B = ctx->trace;
-        B.rays.ensure((size_t)n * 32);
         B.hits.ensure((size_t)n);
         B.occ.ensure(64);
         DL_CUDA(cudaEventRecord(ctx->ev0, st));
-        DL_CUDA(cudaMemcpyAsync(B.rays.ptr, rays, (size_t)n * 32, cudaMemcpyHostToDevice, st));
-        dl::trace_any_launch(S, B.rays.as<float>(), n, B.hits.as<uint8_t>(), B.occ.ptr, false);
-        DL_CUDA(cudaMemcpyAsync(occluded, B.hits.ptr, (size_t)n, cudaMemcpyDeviceToHost, st));
-        unsigned int err = 0;
-        DL_CUDA(cudaMemcpyAsync(&err, B.occ.ptr, 4, cudaMemcpyDeviceToHost, st));
-        DL_CUDA(cudaEventRecord(ctx->ev1, st));
-        DL_CUDA(cudaStreamSynchronize(st));
-        if (err & 4u)
-            throw dl::Error(DL_ERR_QUEUE_OVERFLOW, "bounds check failed: a node or triangle index outside its array "
-                                                   "(bounds-checked build)");
-        if (err) throw dl::Error(DL_ERR_QUEUE_OVERFLOW, "traversal stack overflow");
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-        ctx->stats.trace_ms = ms;
+        dl::trace_any_launch(S, rays_on_device(ctx, rays, n), n, B.hits.as<uint8_t>(), B.occ.ptr);
+        if (direct_out(ctx, occluded, 1)) {
+            touch_pages(occluded, (size_t)n);
+            dl::copy_bytes_launch(ctx, B.hits.as<uint8_t>(), n, occluded);
+        } else {
+            DL_CUDA(cudaMemcpyAsync(occluded, B.hits.ptr, (size_t)n, cudaMemcpyDeviceToHost, st));
+        }
+        finish_rays(ctx);
     });
 }
+
+}  // extern "C"
 
 namespace {
 // Rays through the renderer's own traversal kernels (render.cu): every ray
@@ -299,6 +350,8 @@ void trace_wavefront_host(dl_scene* S, bool any, const float* rays, int64_t n, f
     ctx->stats.trace_ms = ms;
 }
 }  // namespace
+
+extern "C" {
 
 int dl_trace_closest_wavefront(dl_scene* S, const float* rays, int64_t n, int32_t* prim_id, float* t, float* u,
                                float* v) {
@@ -648,10 +701,10 @@ void guide_err_reset(dl_guide* G, cudaStream_t st) {
     DL_CUDA(cudaMemsetAsync(G->scratch.as<char>() + dl::kGuideErrOffset, 0, 4, st));
 }
 void guide_err_check(dl_guide* G, cudaStream_t st) {
-    unsigned err = 0;
-    DL_CUDA(cudaMemcpyAsync(&err, G->scratch.as<char>() + dl::kGuideErrOffset, 4, cudaMemcpyDeviceToHost, st));
+    unsigned* err = G->ctx->words.as<unsigned>();
+    DL_CUDA(cudaMemcpyAsync(err, G->scratch.as<char>() + dl::kGuideErrOffset, 4, cudaMemcpyDeviceToHost, st));
     DL_CUDA(cudaStreamSynchronize(st));
-    if (err) throw dl::Error(DL_ERR_TIMEOUT, "tensor-core wait timed out in a network kernel");
+    if (*err) throw dl::Error(DL_ERR_TIMEOUT, "tensor-core wait timed out in a network kernel");
 }
 }  // namespace
 
@@ -733,18 +786,23 @@ int dl_guide_forward(dl_guide* G, int64_t n, const float* inputs, float* outputs
     return guard(ctx, [&] {
         need(n >= 0 && n < ((int64_t)1 << 31) && (n == 0 || (inputs && outputs)), "bad buffers");
         if (n == 0) return;
-        G->io_in.ensure((size_t)n * 6 * 4);
-        G->io_out.ensure((size_t)n * 40 * 4);
-        DL_CUDA(cudaMemcpyAsync(G->io_in.ptr, inputs, (size_t)n * 24, cudaMemcpyHostToDevice, ctx->stream));
+        // the network's kernel reads the caller's rows in place where it may
+        const size_t in_bytes = (size_t)n * 24;
+        const bool in_place = direct_in(ctx, inputs, in_bytes, 4);
+        if (!in_place) {
+            G->io_in.ensure(in_bytes);
+            DL_CUDA(cudaMemcpyAsync(G->io_in.ptr, inputs, in_bytes, cudaMemcpyHostToDevice, ctx->stream));
+        }
+        G->io_out.ensure((size_t)n * 160);
         DL_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
-        dl::guide_forward(G, G->io_in.as<float>(), G->io_out.as<float>(), n);
+        dl::guide_forward(G, in_place ? inputs : G->io_in.as<float>(), G->io_out.as<float>(), n);
         DL_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
         DL_CUDA(cudaMemcpyAsync(outputs, G->io_out.ptr, (size_t)n * 160, cudaMemcpyDeviceToHost, ctx->stream));
-        unsigned err = 0;
-        DL_CUDA(cudaMemcpyAsync(&err, G->scratch.as<char>() + dl::kGuideErrOffset, 4, cudaMemcpyDeviceToHost,
+        unsigned* err = ctx->words.as<unsigned>();
+        DL_CUDA(cudaMemcpyAsync(err, G->scratch.as<char>() + dl::kGuideErrOffset, 4, cudaMemcpyDeviceToHost,
                                 ctx->stream));
         DL_CUDA(cudaStreamSynchronize(ctx->stream));
-        if (err) throw dl::Error(DL_ERR_TIMEOUT, "tensor-core wait timed out in the network kernel");
+        if (*err) throw dl::Error(DL_ERR_TIMEOUT, "tensor-core wait timed out in the network kernel");
         float ms = 0.f;
         DL_CUDA(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
         ctx->stats.guide_ms = ms;

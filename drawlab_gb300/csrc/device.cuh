@@ -126,6 +126,13 @@ __device__ __forceinline__ bool intersect_tri(float3 v0, float3 v1, float3 v2, f
     return t >= tmin && t <= tmax;
 }
 
+// 32 bytes (32-byte aligned) of read-only global data in one load.
+__device__ __forceinline__ void ld_nc_256(const float4* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+
 struct RayBox {
     float3 idir, ood;
 };
@@ -157,146 +164,6 @@ __device__ __forceinline__ void box2(const RayBox& rb, float tmin, float tmax, f
     h1 = n1 <= f1;
     t0 = n0;
     t1 = n1;
-}
-
-struct TraversalCounters {
-    unsigned long long nodes;
-    unsigned long long tris;
-};
-
-// Closest hit over the BVH.  Returns the leaf-order triangle index or -1;
-// t/u/v as the reference's Moller-Trumbore computes them.  `err` is set when
-// the stack would overflow (cannot happen for depth <= kStackSize builds).
-template <bool kCount>
-__device__ __forceinline__ int trace_closest(const DevScene& sc, float3 o, float3 d, float tmin,
-                                             float tmax, float& ht, float& hu, float& hv,
-                                             uint32_t& err, uint32_t& n_nodes, uint32_t& n_tris) {
-    int hit = -1;
-    if (sc.num_tris == 0) return -1;
-    RayBox rb = make_raybox(o, d);
-    int stack[kStackSize];
-    int sp = 0;
-    int node = 0;
-    for (;;) {
-        if (node >= 0) {
-#ifdef DL_CHECKS
-            if (node >= sc.num_nodes) {  // bounds-checked build: bit 4 of the error word
-                err |= 4u;
-                break;
-            }
-#endif
-            const float4* np = sc.nodes + 4 * node;
-            float4 a = __ldg(np), b = __ldg(np + 1), c = __ldg(np + 2);
-            int4 ch = __ldg(reinterpret_cast<const int4*>(np + 3));
-            if (kCount) n_nodes++;
-            bool h0, h1;
-            float t0, t1;
-            box2(rb, tmin, tmax, a, b, c, h0, h1, t0, t1);
-            h0 = h0 && ch.x != kEmptyChild;
-            h1 = h1 && ch.y != kEmptyChild;
-            if (h0 && h1) {
-                int near = ch.x, far = ch.y;
-                if (t1 < t0) { near = ch.y; far = ch.x; }
-                if (sp < kStackSize) stack[sp++] = far; else err |= 1u;
-                node = near;
-                continue;
-            } else if (h0) {
-                node = ch.x;
-                continue;
-            } else if (h1) {
-                node = ch.y;
-                continue;
-            }
-        } else {
-            int ref = ~node;
-            int first = ref >> 4, count = (ref & 15) + 1;
-#ifdef DL_CHECKS
-            if (first < 0 || first + count > sc.num_tris) {
-                err |= 4u;
-                count = 0;
-            }
-#endif
-            for (int k = 0; k < count; k++) {
-                const float4* tp = sc.tris + 3 * (first + k);
-                float4 p0 = __ldg(tp), p1 = __ldg(tp + 1), p2 = __ldg(tp + 2);
-                if (kCount) n_tris++;
-                float t, u, v;
-                if (intersect_tri(xyz(p0), xyz(p1), xyz(p2), o, d, tmin, tmax, t, u, v)) {
-                    tmax = t;
-                    ht = t;
-                    hu = u;
-                    hv = v;
-                    hit = first + k;
-                }
-            }
-        }
-        if (sp == 0) break;
-        node = stack[--sp];
-    }
-    return hit;
-}
-
-// Any hit (shadow rays), first accepted triangle ends the query.
-template <bool kCount>
-__device__ __forceinline__ bool trace_any(const DevScene& sc, float3 o, float3 d, float tmin,
-                                          float tmax, uint32_t& err, uint32_t& n_nodes,
-                                          uint32_t& n_tris) {
-    if (sc.num_tris == 0) return false;
-    RayBox rb = make_raybox(o, d);
-    int stack[kStackSize];
-    int sp = 0;
-    int node = 0;
-    for (;;) {
-        if (node >= 0) {
-#ifdef DL_CHECKS
-            if (node >= sc.num_nodes) {  // bounds-checked build: bit 4 of the error word
-                err |= 4u;
-                break;
-            }
-#endif
-            const float4* np = sc.nodes + 4 * node;
-            float4 a = __ldg(np), b = __ldg(np + 1), c = __ldg(np + 2);
-            int4 ch = __ldg(reinterpret_cast<const int4*>(np + 3));
-            if (kCount) n_nodes++;
-            bool h0, h1;
-            float t0, t1;
-            box2(rb, tmin, tmax, a, b, c, h0, h1, t0, t1);
-            h0 = h0 && ch.x != kEmptyChild;
-            h1 = h1 && ch.y != kEmptyChild;
-            if (h0 && h1) {
-                int near = ch.x, far = ch.y;
-                if (t1 < t0) { near = ch.y; far = ch.x; }
-                if (sp < kStackSize) stack[sp++] = far; else err |= 1u;
-                node = near;
-                continue;
-            } else if (h0) {
-                node = ch.x;
-                continue;
-            } else if (h1) {
-                node = ch.y;
-                continue;
-            }
-        } else {
-            int ref = ~node;
-            int first = ref >> 4, count = (ref & 15) + 1;
-#ifdef DL_CHECKS
-            if (first < 0 || first + count > sc.num_tris) {
-                err |= 4u;
-                count = 0;
-            }
-#endif
-            for (int k = 0; k < count; k++) {
-                const float4* tp = sc.tris + 3 * (first + k);
-                float4 p0 = __ldg(tp), p1 = __ldg(tp + 1), p2 = __ldg(tp + 2);
-                if (kCount) n_tris++;
-                float t, u, v;
-                if (intersect_tri(xyz(p0), xyz(p1), xyz(p2), o, d, tmin, tmax, t, u, v)) return true;
-            }
-        }
-        if (sp == 0) break;
-        node = stack[--sp];
-    }
-    return false;
 }
 
 // ------------------------------------------------------------------ frames

@@ -120,12 +120,6 @@ __device__ __forceinline__ bool in_bounds(bool ok, unsigned int* err) {
 #endif
 constexpr const char* kBoundsMessage = "bounds check failed: a queue, slot, path, node or triangle index "
                                         "outside its array (bounds-checked build)";
-// 32 bytes (32-byte aligned) of read-only global data in one load.
-__device__ __forceinline__ void ld_nc_256(const float4* p, float4& a, float4& b) {
-    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-        : "l"(p));
-}
 __device__ __forceinline__ bool slot_ok(const RenderParams& P, int slot) {
     return DL_IN_BOUNDS(slot >= 0 && slot < P.capacity, &P.cnt->err);
 }

@@ -12,8 +12,13 @@ void validate_scene(const dl_mesh_desc* meshes, int32_t nm, const dl_material_de
 void build_scene(dl_scene* S, const dl_mesh_desc* meshes, int32_t nm, const dl_material_desc* mats, int32_t nmat,
                  const dl_light_desc* lights, int32_t nl, const dl_camera_desc* cam);
 
-void trace_closest_launch(dl_scene* S, const float* d_rays, int64_t n, float* d_hits, void* scratch, bool count);
-void trace_any_launch(dl_scene* S, const float* d_rays, int64_t n, uint8_t* d_occ, void* scratch, bool count);
+void trace_closest_launch(dl_scene* S, const float* d_rays, int64_t n, float* d_hits, void* scratch);
+void trace_any_launch(dl_scene* S, const float* d_rays, int64_t n, uint8_t* d_occ, void* scratch);
+// Results into the caller's arrays, on the context stream: host memory that
+// the device may write (host_direct), or device memory.
+void split_hits_launch(const dl_context* ctx, const float* d_hits, int64_t n, int32_t* prim, float* t, float* u,
+                       float* v);
+void copy_bytes_launch(const dl_context* ctx, const uint8_t* from, int64_t n, uint8_t* to);
 // The same queries through the renderer's own k_traverse kernels (render.cu);
 // every ray starts at t = kRayEps.  Synchronises; `work` holds
 // wavefront_rays_bytes(n).
