@@ -492,7 +492,7 @@ int dl_guide_train(dl_guide* guide, int64_t n, const float* records, int32_t ste
  * records (radiance gathered later on the path is credited to the two most
  * recent ones) and the guide takes steps_per_pass Adam steps on interleaved
  * subsets of them before the next pass.  With `train` 0 the network is
- * frozen.  All samples add to one film. */
+ * frozen, and one pass renders all samples.  All samples add to one film. */
 int dl_render_guided(dl_scene* scene, const dl_render_opts* opts, dl_guide* guide, int32_t train, float* rgb_out);
 
 /* --------------------------------------------------------------- statistics */
