@@ -440,9 +440,9 @@ int dl_render_film(dl_scene* S, const dl_render_opts* opts, float* film_out) {
         need(film_out != nullptr, "film_out is NULL");
         int64_t nf = dl::film_floats(S->dev.cam.w, S->dev.cam.h, opts->filter);
         ctx->render.film.ensure((size_t)nf * 4);
-        dl::render_run(S, *opts, ctx->render.film.as<float>(), 0, nullptr, nullptr, nullptr, false, nullptr);
-        DL_CUDA(cudaMemcpyAsync(film_out, ctx->render.film.ptr, (size_t)nf * 4, cudaMemcpyDeviceToHost, ctx->stream));
-        DL_CUDA(cudaStreamSynchronize(ctx->stream));
+        dl::render_run(S, *opts, ctx->render.film.as<float>(), 0, nullptr, nullptr, nullptr, false, nullptr, [&] {
+            DL_CUDA(cudaMemcpyAsync(film_out, ctx->render.film.ptr, (size_t)nf * 4, cudaMemcpyDeviceToHost, ctx->stream));
+        });
     });
 }
 
@@ -456,10 +456,10 @@ int dl_render(dl_scene* S, const dl_render_opts* opts, float* rgb_out) {
         size_t nrgb = (size_t)S->dev.cam.w * S->dev.cam.h * 3;
         ctx->render.film.ensure((size_t)nf * 4);
         ctx->render.rgb.ensure(nrgb * 4);
-        dl::render_run(S, *opts, ctx->render.film.as<float>(), 0, nullptr, nullptr, nullptr, false, nullptr);
-        dl::resolve_film(S, ctx->render.film.as<float>(), opts->filter, ctx->render.rgb.as<float>());
-        DL_CUDA(cudaMemcpyAsync(rgb_out, ctx->render.rgb.ptr, nrgb * 4, cudaMemcpyDeviceToHost, ctx->stream));
-        DL_CUDA(cudaStreamSynchronize(ctx->stream));
+        dl::render_run(S, *opts, ctx->render.film.as<float>(), 0, nullptr, nullptr, nullptr, false, nullptr, [&] {
+            dl::resolve_film(S, ctx->render.film.as<float>(), opts->filter, ctx->render.rgb.as<float>());
+            DL_CUDA(cudaMemcpyAsync(rgb_out, ctx->render.rgb.ptr, nrgb * 4, cudaMemcpyDeviceToHost, ctx->stream));
+        });
     });
 }
 
@@ -472,10 +472,11 @@ int dl_li(dl_scene* S, const dl_render_opts* opts, int64_t n, const int32_t* xys
         need(n < ((int64_t)1 << 31), "at most 2^31 - 1 paths per call");
         if (n == 0) return;
         const dl::DevCamera& cam = S->dev.cam;
+        unsigned bad = 0;  // (no branch a path: the loop vectorises)
         for (int64_t i = 0; i < n; i++)
-            need(xys[3 * i] >= 0 && xys[3 * i] < cam.w && xys[3 * i + 1] >= 0 && xys[3 * i + 1] < cam.h &&
-                     xys[3 * i + 2] >= 0,
-                 "path (x, y, s) out of range");
+            bad |= (unsigned)((unsigned)xys[3 * i] >= (unsigned)cam.w) |
+                   (unsigned)((unsigned)xys[3 * i + 1] >= (unsigned)cam.h) | (unsigned)(xys[3 * i + 2] < 0);
+        need(!bad, "path (x, y, s) out of range");
         dl_render_opts o = *opts;
         o.spp = 1;
         check_opts(&o);
@@ -485,11 +486,12 @@ int dl_li(dl_scene* S, const dl_render_opts* opts, int64_t n, const int32_t* xys
         B.li_out.ensure((size_t)n * 12);
         B.li_pos.ensure((size_t)n * 8);
         DL_CUDA(cudaMemcpyAsync(B.li_xys.ptr, xys, (size_t)n * 12, cudaMemcpyHostToDevice, st));
-        dl::render_run(S, o, nullptr, n, B.li_xys.as<int>(), B.li_out.as<float>(), B.li_pos.as<float>(), false,
-                       nullptr);
-        DL_CUDA(cudaMemcpyAsync(L_out, B.li_out.ptr, (size_t)n * 12, cudaMemcpyDeviceToHost, st));
-        if (pos_out) DL_CUDA(cudaMemcpyAsync(pos_out, B.li_pos.ptr, (size_t)n * 8, cudaMemcpyDeviceToHost, st));
-        DL_CUDA(cudaStreamSynchronize(st));
+        dl::render_run(S, o, nullptr, n, B.li_xys.as<int>(), B.li_out.as<float>(), B.li_pos.as<float>(), false, nullptr,
+                       [&] {
+                           DL_CUDA(cudaMemcpyAsync(L_out, B.li_out.ptr, (size_t)n * 12, cudaMemcpyDeviceToHost, st));
+                           if (pos_out)
+                               DL_CUDA(cudaMemcpyAsync(pos_out, B.li_pos.ptr, (size_t)n * 8, cudaMemcpyDeviceToHost, st));
+                       });
     });
 }
 
@@ -568,19 +570,19 @@ int dl_render_batch(dl_context* ctx, const dl_request* reqs, int32_t n) {
         std::vector<int64_t> off;
         std::vector<dl::BatchItem> items = batch_items(ctx, reqs, n, true, -1, off);
         if (n == 0) return;
-        dl::render_batch(ctx, items.data(), n, false);
         size_t maxrgb = 0;
         for (int32_t r = 0; r < n; r++)
             if (reqs[r].rgb) maxrgb = std::max(maxrgb, (size_t)items[r].cam.w * items[r].cam.h * 3);
         ctx->render.rgb.ensure(std::max<size_t>(maxrgb, 1) * 4);
-        for (int32_t r = 0; r < n; r++) {
-            if (!reqs[r].rgb) continue;
-            size_t nrgb = (size_t)items[r].cam.w * items[r].cam.h * 3;
-            dl::resolve_film_cam(items[r].cam, ctx->stream, items[r].d_film, items[r].opts.filter,
-                                 ctx->render.rgb.as<float>());
-            DL_CUDA(cudaMemcpyAsync(reqs[r].rgb, ctx->render.rgb.ptr, nrgb * 4, cudaMemcpyDeviceToHost, ctx->stream));
-            DL_CUDA(cudaStreamSynchronize(ctx->stream));
-        }
+        dl::render_batch(ctx, items.data(), n, false, [&] {
+            for (int32_t r = 0; r < n; r++) {  // (one after another on the stream)
+                if (!reqs[r].rgb) continue;
+                size_t nrgb = (size_t)items[r].cam.w * items[r].cam.h * 3;
+                dl::resolve_film_cam(items[r].cam, ctx->stream, items[r].d_film, items[r].opts.filter,
+                                     ctx->render.rgb.as<float>());
+                DL_CUDA(cudaMemcpyAsync(reqs[r].rgb, ctx->render.rgb.ptr, nrgb * 4, cudaMemcpyDeviceToHost, ctx->stream));
+            }
+        });
     });
 }
 

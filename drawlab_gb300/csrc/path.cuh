@@ -88,6 +88,7 @@ struct RenderParams {
     const int* xys;
     float* li_L;
     float* li_pos;
+    unsigned long long total;  // resident kernel: paths of the pass
     // guided renders
     int guided;
     GuideNet gnet;
@@ -194,8 +195,10 @@ struct PathState {
 };
 
 // Path `pid` of request `rid`: camera sample (film position `ps`) and ray
-// (cpu_renderer.cpp:36-44).
-template <bool kMulti>
+// (cpu_renderer.cpp:36-44).  kPass: a single render's first sample index is
+// among the pass values on the device (the wavefront's captured graph), else
+// in the request.
+template <bool kMulti, bool kPass>
 __device__ __forceinline__ void camera_path(const RenderParams& P, unsigned long long pid, int rid, PathState& S,
                                             float2& ps, float3& o, float3& d, float& tmax) {
     const DevRequest& R = request<kMulti>(P, rid);
@@ -219,7 +222,7 @@ __device__ __forceinline__ void camera_path(const RenderParams& P, unsigned long
             x = (int)(pix % cam.w);
             y = (int)(pix / cam.w);
         }
-        s += kMulti ? R.spp_offset : P.cnt->pass_spp_offset;
+        s += kMulti || !kPass ? R.spp_offset : P.cnt->pass_spp_offset;
     }
     seed_path(S.g, R.seed_mix, cam.w, cam.h, x, y, s);
     ps = S.g.next2d();
@@ -246,7 +249,7 @@ __device__ void start_path(const RenderParams& P, int slot, unsigned long long p
     float2 ps;
     float3 o, d;
     float tmax;
-    camera_path<kMulti>(P, pid, rid, S, ps, o, d, tmax);
+    camera_path<kMulti, true>(P, pid, rid, S, ps, o, d, tmax);
     RayRec r;
     r.o = make_float4(o.x, o.y, o.z, __int_as_float(rid));
     r.d = make_float4(d.x, d.y, d.z, tmax);
@@ -730,8 +733,7 @@ __device__ __forceinline__ bool scatter_vertex(const DevRequest& R, int type, in
 constexpr unsigned long long kResidentMaxPaths = 1ull << 21, kResidentFewPaths = 1ull << 18;
 constexpr unsigned kErrRounds = 8u;  // error-word bit: the resident kernel gave up (a wait or a warp's turns ran out)
 
-// One pass of `total` paths as one launch on `st`; P.cnt reset and its pass
-// values set before.
-void resident_launch(int sms, const RenderParams& P, bool multi, unsigned long long total, cudaStream_t st);
+// One pass of P.total paths as one launch on `st`; P.cnt reset before.
+void resident_launch(int sms, const RenderParams& P, bool multi, cudaStream_t st);
 
 }  // namespace dl

@@ -1134,31 +1134,6 @@ static bool use_resident(const dl_context* ctx, int64_t pool, unsigned long long
     return total <= kResidentMaxPaths && pool == 0 && !count_traversal && !ctx->kernel_timing && !ctx->tuning;
 }
 
-// One pass as one k_resident launch; its counters are added to `acc`.
-static void run_resident(dl_context* ctx, const RenderParams& P, bool multi, int64_t& launches, int64_t& iters,
-                         RenderCounters& acc, unsigned long long total, int spp_offset) {
-    cudaStream_t st = ctx->stream;
-    RenderBuffers& B = ctx->render;
-    DL_CUDA(cudaMemsetAsync(P.cnt, 0, sizeof(RenderCounters), st));
-    B.host_pass.ensure(sizeof(PassValues));
-    PassValues* pv = B.host_pass.as<PassValues>();
-    pv->total = total;
-    pv->spp_offset = spp_offset;
-    pv->keep = 0;
-    pv->recs = nullptr;
-    DL_CUDA(cudaMemcpyAsync(&P.cnt->pass_total, pv, sizeof(PassValues), cudaMemcpyHostToDevice, st));
-    resident_launch(ctx->num_sms > 0 ? ctx->num_sms : 152, P, multi, total, st);
-    launches += 1;
-    iters += 1;
-    RenderCounters* hc = B.host_counters.as<RenderCounters>();
-    DL_CUDA(cudaMemcpyAsync(hc, P.cnt, sizeof(RenderCounters), cudaMemcpyDeviceToHost, st));
-    DL_CUDA(cudaStreamSynchronize(st));
-    check_render_error(hc->err);
-    acc.stat_camera += total;
-    acc.stat_ext += hc->stat_ext;
-    acc.stat_shadow += hc->stat_shadow;
-}
-
 // Budget of the per-path sample buffer; larger frames render in passes of
 // whole samples per pixel.
 constexpr size_t kSampleBufferBytes = (size_t)4 << 30;
@@ -1180,11 +1155,33 @@ static FilmParams film_params(const DevCamera& cam, const DevRequest& R, int fil
     return F;
 }
 
+// The end of a render, in two halves around the caller's results: reads the
+// counters of a resident pass (`resident`), or the count of invalid samples,
+// and marks the end of the render's time; then, after one wait, checks the
+// error word of a resident pass and adds its counters.
+static void end_render(dl_context* ctx, bool resident, const RenderParams& P, const void* d_invalid,
+                       const std::function<void()>& results, RenderCounters& acc) {
+    cudaStream_t st = ctx->stream;
+    RenderCounters* hc = ctx->render.host_counters.as<RenderCounters>();
+    unsigned long long* hinv = reinterpret_cast<unsigned long long*>(hc + 1);
+    *hinv = 0;
+    if (resident) DL_CUDA(cudaMemcpyAsync(hc, P.cnt, sizeof(RenderCounters), cudaMemcpyDeviceToHost, st));
+    else if (d_invalid) DL_CUDA(cudaMemcpyAsync(hinv, d_invalid, sizeof(*hinv), cudaMemcpyDeviceToHost, st));
+    DL_CUDA(cudaEventRecord(ctx->ev1, st));
+    if (results) results();
+    DL_CUDA(cudaStreamSynchronize(st));
+    if (resident) {
+        check_render_error(hc->err);
+        acc.stat_camera += P.total;
+        acc.stat_ext += hc->stat_ext;
+        acc.stat_shadow += hc->stat_shadow;
+        *hinv = hc->stat_invalid;
+    }
+    acc.stat_invalid = *hinv;
+}
+
 static void finish_stats(dl_context* ctx, const RenderCounters& acc, unsigned long long invalid, int64_t iters,
                          int64_t launches, const double* kms) {
-    cudaStream_t st = ctx->stream;
-    DL_CUDA(cudaEventRecord(ctx->ev1, st));
-    DL_CUDA(cudaEventSynchronize(ctx->ev1));
     float ms = 0.f;
     DL_CUDA(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
     ctx->stats.camera_rays = (int64_t)acc.stat_camera;
@@ -1209,7 +1206,8 @@ static int64_t pool_capacity(dl_context* ctx, int64_t requested, unsigned long l
 // Runs one render.  mode 0: the film (d_film) receives every sample through
 // the gather kernel; mode 1: Li of li_n explicit paths (d_xys -> d_L, d_pos).
 void render_run(dl_scene* S, const dl_render_opts& o, float* d_film, int64_t li_n, const int* d_xys,
-                float* d_L, float* d_pos, bool count_traversal, RenderCounters* out_counters) {
+                float* d_L, float* d_pos, bool count_traversal, RenderCounters* out_counters,
+                const std::function<void()>& results) {
     dl_context* ctx = S->ctx;
     cudaStream_t st = ctx->stream;
     const DevCamera& cam = S->dev.cam;
@@ -1238,20 +1236,27 @@ void render_run(dl_scene* S, const dl_render_opts& o, float* d_film, int64_t li_
     RenderCounters acc;
     std::memset(&acc, 0, sizeof(acc));
     DL_CUDA(cudaEventRecord(ctx->ev0, st));
-    unsigned long long invalid = 0;
-    if (P.mode == 1 && resident) {
-        run_resident(ctx, P, false, launches, iters, acc, (unsigned long long)li_n, 0);
-    } else if (P.mode == 1) {
-        run_wavefront(ctx, P, cap, false, count_traversal, kms, launches, iters, acc, (unsigned long long)li_n, 0,
-                      1u << 24);
+    FilmParams F;
+    if (P.mode == 0) {
+        // (a resident pass counts invalid samples among its counters)
+        F = film_params(cam, P.r0, o.filter, d_film, P.samples,
+                        resident ? &P.cnt->stat_invalid : B.invalid.as<unsigned long long>());
+        if (!resident) DL_CUDA(cudaMemsetAsync(F.invalid, 0, sizeof(unsigned long long), st));
+    }
+    if (resident) {   // (a whole render: its samples fit the buffer)
+        P.total = chunk_total;
+        DL_CUDA(cudaMemsetAsync(P.cnt, 0, sizeof(RenderCounters), st));
+        resident_launch(ctx->num_sms > 0 ? ctx->num_sms : 152, P, false, st);
+        launches = iters = 1;
+    }
+    if (P.mode == 1) {
+        if (!resident)
+            run_wavefront(ctx, P, cap, false, count_traversal, kms, launches, iters, acc, (unsigned long long)li_n, 0,
+                          1u << 24);
     } else {
-        FilmParams F = film_params(cam, P.r0, o.filter, d_film, P.samples, B.invalid.as<unsigned long long>());
-        DL_CUDA(cudaMemsetAsync(F.invalid, 0, sizeof(unsigned long long), st));
         for (int s0 = 0; s0 < spp; s0 += chunk_spp) {
             int ns = std::min(chunk_spp, spp - s0);
-            if (resident)
-                run_resident(ctx, P, false, launches, iters, acc, npix * (unsigned long long)ns, o.spp_offset + s0);
-            else
+            if (!resident)
                 run_wavefront(ctx, P, cap, false, count_traversal, kms, launches, iters, acc,
                               npix * (unsigned long long)ns, o.spp_offset + s0, 1u << 24);
             F.nspp = ns;
@@ -1260,14 +1265,9 @@ void render_run(dl_scene* S, const dl_render_opts& o, float* d_film, int64_t li_
             film_gather(F, ctx->num_sms, st);
             launches += 1;
         }
-        unsigned long long* hinv =
-            reinterpret_cast<unsigned long long*>(B.host_counters.as<char>() + sizeof(RenderCounters));
-        DL_CUDA(cudaMemcpyAsync(hinv, F.invalid, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-        DL_CUDA(cudaStreamSynchronize(st));
-        invalid = *hinv;
     }
-    acc.stat_invalid = invalid;
-    finish_stats(ctx, acc, invalid, iters, launches, kms);
+    end_render(ctx, resident, P, P.mode == 0 ? F.invalid : nullptr, results, acc);
+    finish_stats(ctx, acc, acc.stat_invalid, iters, launches, kms);
     if (out_counters) *out_counters = acc;
 }
 
@@ -1408,12 +1408,8 @@ void render_guided(dl_scene* S, const dl_render_opts& o, dl_guide* G, float* d_f
         DL_CUDA(cudaStreamSynchronize(ts));
         DL_CUDA(cudaEventElapsedTime(&train_ms, G->t0, G->t1));  // the last round's device time
     }
-    unsigned long long* hinv =
-        reinterpret_cast<unsigned long long*>(B.host_counters.as<char>() + sizeof(RenderCounters));
-    DL_CUDA(cudaMemcpyAsync(hinv, F.invalid, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-    DL_CUDA(cudaStreamSynchronize(st));
-    acc.stat_invalid = *hinv;
-    finish_stats(ctx, acc, *hinv, iters, launches, kms);
+    end_render(ctx, false, P, F.invalid, nullptr, acc);
+    finish_stats(ctx, acc, acc.stat_invalid, iters, launches, kms);
     ctx->stats.guide_records = records;
     ctx->stats.guide_train_ms = train_ms;
 }
@@ -1423,7 +1419,8 @@ void render_guided(dl_scene* S, const dl_render_opts& o, dl_guide* G, float* d_f
 // share the path pool and the material queues (each path carries its
 // request), and after the pass one gather per request adds the slice to its
 // film.  Slices are sized so a pass fits the sample buffer.
-void render_batch(dl_context* ctx, const BatchItem* items, int n, bool count_traversal) {
+void render_batch(dl_context* ctx, const BatchItem* items, int n, bool count_traversal,
+                  const std::function<void()>& results) {
     cudaStream_t st = ctx->stream;
     RenderBuffers& B = ctx->render;
     std::vector<int> done(n, 0);
@@ -1455,13 +1452,14 @@ void render_batch(dl_context* ctx, const BatchItem* items, int n, bool count_tra
     P.mode = 0;
     P.samples = B.samples.as<float4>();
     P.reqs = B.requests.as<DevRequest>();
-    unsigned long long* d_invalid = B.invalid.as<unsigned long long>();
+    // (a resident pass counts invalid samples among its counters)
+    unsigned long long* d_invalid = resident ? &P.cnt->stat_invalid : B.invalid.as<unsigned long long>();
     double kms[4] = {0, 0, 0, 0};
     int64_t launches = 0, iters = 0;
     RenderCounters acc;
     std::memset(&acc, 0, sizeof(acc));
     DL_CUDA(cudaEventRecord(ctx->ev0, st));
-    DL_CUDA(cudaMemsetAsync(d_invalid, 0, sizeof(unsigned long long), st));
+    if (!resident) DL_CUDA(cudaMemsetAsync(d_invalid, 0, sizeof(unsigned long long), st));
     std::vector<int> active(n), ns(n);
     for (;;) {
         int na = 0;
@@ -1483,8 +1481,14 @@ void render_batch(dl_context* ctx, const BatchItem* items, int n, bool count_tra
         // the pass's request table; the copy is ordered before the pass's kernels
         DL_CUDA(cudaMemcpyAsync(B.requests.ptr, hreq, sizeof(DevRequest) * na, cudaMemcpyHostToDevice, st));
         P.num_reqs = na;
-        if (resident) run_resident(ctx, P, true, launches, iters, acc, first, 0);
-        else run_wavefront(ctx, P, cap, true, count_traversal, kms, launches, iters, acc, first, 0, 1u << 24);
+        if (resident) {   // (one pass: every request's samples fit the buffer)
+            P.total = first;
+            DL_CUDA(cudaMemsetAsync(P.cnt, 0, sizeof(RenderCounters), st));
+            resident_launch(ctx->num_sms > 0 ? ctx->num_sms : 152, P, true, st);
+            launches = iters = 1;
+        } else {
+            run_wavefront(ctx, P, cap, true, count_traversal, kms, launches, iters, acc, first, 0, 1u << 24);
+        }
         for (int a = 0; a < na; a++) {
             const int r = active[a];
             const DevCamera& cam = items[r].cam;
@@ -1497,15 +1501,11 @@ void render_batch(dl_context* ctx, const BatchItem* items, int n, bool count_tra
             launches += 1;
             done[r] += ns[a];
         }
-        // host_requests is rewritten next pass: wait for this pass's copy
-        DL_CUDA(cudaStreamSynchronize(st));
+        // (host_requests is rewritten next pass, after the wavefront's wait)
+        if (resident) break;
     }
-    unsigned long long* hinv =
-        reinterpret_cast<unsigned long long*>(B.host_counters.as<char>() + sizeof(RenderCounters));
-    DL_CUDA(cudaMemcpyAsync(hinv, d_invalid, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-    DL_CUDA(cudaStreamSynchronize(st));
-    acc.stat_invalid = *hinv;
-    finish_stats(ctx, acc, *hinv, iters, launches, kms);
+    end_render(ctx, resident, P, d_invalid, results, acc);
+    finish_stats(ctx, acc, acc.stat_invalid, iters, launches, kms);
 }
 
 // Li of explicit paths with every piece of path state in caller-provided

@@ -150,7 +150,7 @@ __device__ __forceinline__ uint32_t ring_take(Ring<N>& r, uint32_t at, int* abor
 // camera sample's film position (its stream's first 2D draw).
 template <bool kMulti>
 __device__ __forceinline__ void resident_store(const RenderParams& P, uint32_t pid, float3 L) {
-    if (!DL_IN_BOUNDS(pid < P.cnt->pass_total, &P.cnt->err)) return;
+    if (!DL_IN_BOUNDS(pid < P.total, &P.cnt->err)) return;
     if (P.mode == 1) {
         const size_t i = pid;
         P.li_L[3 * i] = L.x;
@@ -410,7 +410,7 @@ __device__ __forceinline__ void resident_shade(const RenderParams& P, Sm& sm, in
 // lane's slot starts the next path of the pass, 32 consecutive ones a warp.
 template <bool kMulti, class Sm>
 __device__ __forceinline__ void resident_restart(const RenderParams& P, Sm& sm, uint32_t entry, bool active,
-                                                 unsigned long long total, uint32_t& err) {
+                                                 uint32_t& err) {
     const int slot = (int)(entry & ~kFreeEntry);
     if (active && !(entry & kFreeEntry)) {
         PathState S;
@@ -425,14 +425,14 @@ __device__ __forceinline__ void resident_restart(const RenderParams& P, Sm& sm, 
         resident_store<kMulti>(P, sm.pid[slot], S.L);
     }
     const unsigned long long pid = warp_claim(&P.cnt->next_path, active);
-    const bool start = active && pid < total;
+    const bool start = active && pid < P.total;
     if (start) {
         const int rid = kMulti ? find_request(P, pid) : 0;
         PathState S;
         float2 ps;
         float3 o, d;
         float tmax;
-        camera_path<kMulti>(P, pid, rid, S, ps, o, d, tmax);
+        camera_path<kMulti, false>(P, pid, rid, S, ps, o, d, tmax);
         sm.o[0][slot] = o.x;
         sm.o[1][slot] = o.y;
         sm.o[2][slot] = o.z;
@@ -463,7 +463,7 @@ __device__ __forceinline__ void resident_restart(const RenderParams& P, Sm& sm, 
 
 // `slots`: path slots each block uses (a multiple of 32, at most kSlots).
 template <bool kMulti, int kThreads, int kSlots, int kBlocks>
-__global__ void __launch_bounds__(kThreads, kBlocks) k_resident(RenderParams P, unsigned long long total, int slots) {
+__global__ void __launch_bounds__(kThreads, kBlocks) k_resident(RenderParams P, int slots) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     auto& sm = *reinterpret_cast<ResidentSmem<kThreads, kSlots>*>(dyn_smem);
     const int lane = lane_id();
@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_resident(RenderParams P, 
             if (n > 0) {
                 const uint32_t e = lane < n ? ring_take(sm.queue[best], base + lane, &sm.abort, err) : kNoEntry;
                 const bool active = e != kNoEntry;
-                if (best == kEndedQueue) resident_restart<kMulti>(P, sm, e, active, total, err);
+                if (best == kEndedQueue) resident_restart<kMulti>(P, sm, e, active, err);
                 else resident_shade<kMulti>(P, sm, best, active ? (int)e : 0, active, err);
                 idle = 0;
                 if (++turn == kResMaxTurns) st_shared(&sm.abort, 1);
@@ -532,7 +532,8 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_resident(RenderParams P, 
 
 // One shape of the kernel, its blocks per SM found on first use.
 template <bool kMulti, int kThreads, int kSlots, int kBlocks>
-static void launch_shape(int sms, const RenderParams& P, unsigned long long total, cudaStream_t st) {
+static void launch_shape(int sms, const RenderParams& P, cudaStream_t st) {
+    const unsigned long long total = P.total;
     auto* fn = k_resident<kMulti, kThreads, kSlots, kBlocks>;
     constexpr size_t smem = sizeof(ResidentSmem<kThreads, kSlots>);
     static_assert(kSlots % 32 == 0 && kSlots < (int)kFreeEntry && kBlocks * (smem + 1024) <= 228 * 1024, "shared memory");
@@ -547,18 +548,18 @@ static void launch_shape(int sms, const RenderParams& P, unsigned long long tota
     const int64_t share = (int64_t)((total + blocks - 1) / blocks);
     const int slots = (int)std::min<int64_t>(kSlots, (share + 31) / 32 * 32);
     const int grid = (int)std::min<int64_t>(blocks, (int64_t)((total + slots - 1) / slots));
-    fn<<<grid, kThreads, smem, st>>>(P, total, slots);
+    fn<<<grid, kThreads, smem, st>>>(P, slots);
     DL_CUDA(cudaGetLastError());
 }
 
-void resident_launch(int sms, const RenderParams& P, bool multi, unsigned long long total, cudaStream_t st) {
+void resident_launch(int sms, const RenderParams& P, bool multi, cudaStream_t st) {
     // (the shapes cross between 0.2 and 0.4 M paths: see the top)
-    if (total <= kResidentFewPaths) {
-        if (multi) launch_shape<true, 256, 640, 2>(sms, P, total, st);
-        else launch_shape<false, 256, 640, 2>(sms, P, total, st);
+    if (P.total <= kResidentFewPaths) {
+        if (multi) launch_shape<true, 256, 640, 2>(sms, P, st);
+        else launch_shape<false, 256, 640, 2>(sms, P, st);
     } else {
-        if (multi) launch_shape<true, 448, 640, 2>(sms, P, total, st);
-        else launch_shape<false, 448, 640, 2>(sms, P, total, st);
+        if (multi) launch_shape<true, 448, 640, 2>(sms, P, st);
+        else launch_shape<false, 448, 640, 2>(sms, P, st);
     }
 }
 

@@ -1,6 +1,8 @@
 // Scene construction (scene.cpp) and the launchers of trace.cu / render.cu.
 #pragma once
 
+#include <functional>
+
 #include "internal.h"
 
 namespace dl {
@@ -38,8 +40,11 @@ void emitter_query(dl_scene* S, uint32_t flags, int64_t n, const float* pts, con
 double measure_l2_read(dl_context* ctx, int64_t bytes, int passes);
 
 int64_t film_floats(int w, int h, int filter);
+// `results` puts what follows the render (resolving, copies to the host) on
+// the stream before the call waits for it; an error is thrown after the wait.
 void render_run(dl_scene* S, const dl_render_opts& o, float* d_film, int64_t li_n, const int* d_xys, float* d_L,
-                float* d_pos, bool count_traversal, RenderCounters* out_counters);
+                float* d_pos, bool count_traversal, RenderCounters* out_counters,
+                const std::function<void()>& results = nullptr);
 void resolve_film(dl_scene* S, const float* d_film, int filter, float* d_rgb);
 // One-time kernel attributes of the current device (called by context creation).
 void render_setup_device();
@@ -52,7 +57,8 @@ struct BatchItem {
     DevCamera cam;   // the scene's camera or the request's override
 };
 void resolve_film_cam(const DevCamera& cam, cudaStream_t st, const float* d_film, int filter, float* d_rgb);
-void render_batch(dl_context* ctx, const BatchItem* items, int n, bool count_traversal);
+void render_batch(dl_context* ctx, const BatchItem* items, int n, bool count_traversal,
+                  const std::function<void()>& results = nullptr);
 
 // Learned guiding (guide.cu).
 constexpr int kGuideParams = 16560;
