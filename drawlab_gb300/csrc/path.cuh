@@ -240,7 +240,8 @@ __device__ __forceinline__ void camera_path(const RenderParams& P, unsigned long
 }
 
 // Start path `pid` in `slot`.  Ray records carry the request index in o.w
-// (every render ray starts at tmin = kRayEps).
+// (every render ray starts at tmin = kRayEps).  The path record of a camera
+// ray (PF_CAMERA) is not written: throughput 1, no radiance yet.
 template <bool kMulti>
 __device__ void start_path(const RenderParams& P, int slot, unsigned long long pid) {
     if (!slot_ok(P, slot) || !DL_IN_BOUNDS(pid < P.cnt->pass_total, &P.cnt->err)) return;
@@ -254,10 +255,6 @@ __device__ void start_path(const RenderParams& P, int slot, unsigned long long p
     r.o = make_float4(o.x, o.y, o.z, __int_as_float(rid));
     r.d = make_float4(d.x, d.y, d.z, tmax);
     P.rec[slot].ray = r;
-    PathRec pr;
-    pr.tp = make_float4(S.tp.x, S.tp.y, S.tp.z, S.eta);
-    pr.L = make_float4(S.L.x, S.L.y, S.L.z, S.prev_pdf);
-    P.rec[slot].path = pr;
     MetaRec mr;
     mr.m = make_int4(S.depth, S.flags, (int)(pid & 0xffffffffu), (int)(pid >> 32));
     mr.rng = store_rng(S.g);
@@ -269,6 +266,14 @@ __device__ void start_path(const RenderParams& P, int slot, unsigned long long p
         gr.b = gr.a;
         P.grec[slot] = gr;
     }
+}
+
+// The path record of a camera ray.
+__device__ __forceinline__ PathRec camera_record() {
+    PathRec r;
+    r.tp = make_float4(1.f, 1.f, 1.f, 1.f);
+    r.L = make_float4(0.f, 0.f, 0.f, 0.f);
+    return r;
 }
 
 // Radiance of ended path `pid` (slot `slot`): into the sample buffer at its

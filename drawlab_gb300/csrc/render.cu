@@ -391,8 +391,9 @@ __global__ void __launch_bounds__(kThreads) k_miss(RenderParams P, int p) {
         int slot = active ? P.mat_q[kMissQueue][i] : 0;
         if (active && !slot_ok(P, slot)) active = false;
         if (active) {
-            PathRec pr = P.rec[slot].path;
             int4 m = P.rec[slot].meta.m;
+            PathRec pr = camera_record();
+            if (!(m.y & PF_CAMERA)) pr = P.rec[slot].path;
             const DevRequest& R = request<kMulti>(P, m.y >> kReqShift);
             const DevScene& sc = R.sc;
             PathState S;
@@ -546,6 +547,7 @@ __global__ void __launch_bounds__(kGuided ? kTcThreads : kThreads, kGuided ? 2 :
         }
         if (active) {
             if (guided) gr = P.grec[slot];
+            if (mr.m.y & PF_CAMERA) pr = camera_record();
             S.g = load_rng(mr.rng);
             S.pid = path_index(mr.m);
             S.tp = f3(pr.tp.x, pr.tp.y, pr.tp.z);
