@@ -115,12 +115,13 @@ __global__ void __launch_bounds__(kWsumThreads) k_guide_weight_sum(const GuideRe
 // the renderer's sampling keeps the accurate forms.  The mixture's
 // normalisation needs both halves: each thread publishes, in `mine`, its
 // largest logit, its sum of exp(logit - that) and the same sum weighted by
-// the lobes' pdfs, and reads the other half's from `other` after a barrier
-// of the whole block (every thread of the block calls this together; both
-// halves then hold the same sums, added in the same order).  Writes the 20
-// gradients, times `scale`, to d; returns the record's loss, -scale log q.
-__device__ __forceinline__ float record_grad_half(const float* o, float3 w, float scale, float4* mine,
-                                                  const float4* other, float* d) {
+// the lobes' pdfs, and reads the other half's from `other` after `exchange`,
+// which waits for it and returns the record's loss weight (both halves then
+// hold the same sums, added in the same order).  Writes the 20 gradients,
+// times that weight, to d; returns the record's loss, -weight log q.
+template <typename F>
+__device__ __forceinline__ float record_grad_half(const float* o, float3 w, float4* mine, const float4* other,
+                                                  F exchange, float* d) {
     constexpr int kH = kGLobes / 2;
     float mx = -1e30f;
 #pragma unroll
@@ -154,7 +155,7 @@ __device__ __forceinline__ float record_grad_half(const float* o, float3 w, floa
         sq += e[j] * pdf[j];
     }
     *mine = make_float4(mx, se, sq, 0.f);
-    __syncthreads();
+    const float scale = exchange();
     const float4 x = *other;
     const float M = fmaxf(mx, x.x);
     const float am = __expf(mx - M), ao = __expf(x.x - M);
@@ -190,11 +191,11 @@ __device__ __forceinline__ float record_grad_half(const float* o, float3 w, floa
 //
 //   k_guide_weight_sum  per-block sums of the records' L / pdf (the loss's
 //                    target normalisation).
-//   k_guide_train    one block per SM, two warpgroups (256 threads), over a
-//                    range of 128-record tiles, one tile at a time.  Per tile,
-//                    every product a tcgen05.mma issued by thread 0 with both
-//                    operands in shared memory and the fp32 accumulator in
-//                    tensor memory:
+//   k_guide_train    one block per SM over a range of 128-record tiles, two
+//                    tiles at a time: two groups of 256 threads walk one tile
+//                    each and one thread of a seventeenth warp issues every
+//                    tcgen05.mma of both, both operands in shared memory and
+//                    the fp32 accumulator in tensor memory.  Per tile:
 //                      forward  x -> h1 -> h2 -> outputs (3 products);
 //                      the loss and dLoss/dOutput of each record (d0, fp16);
 //                      backward d2 = (d0 W3) * [h2 > 0], d1 = (d2 W2) *
@@ -202,23 +203,20 @@ __device__ __forceinline__ float record_grad_half(const float* o, float3 w, floa
 //                               weight image);
 //                      the tile's share of the weight and bias gradients,
 //                               accumulated in tensor memory over the
-//                               block's tiles (K = the tile's records), in
-//                               two products: [d2 | d0]^T [h1 | 1 | h2]
-//                               (dW2, b2, b3, dW3), issued as soon as d2
-//                               exists, and [d1 | .]^T [x | 1] (dW1, b1).
-//                    The activations stay in shared memory in the canonical
-//                    layout, which the forward and backward products read as
-//                    K-major operands and the weight-gradient products as
-//                    MN-major ones (M or N = features, K = records).  The two
-//                    warpgroups split each epilogue's 64 accumulator columns
-//                    and each record's loss (four lobes each); while a
-//                    product runs, each thread encodes one of its three
-//                    inputs of the next tile into the second x buffer; the
-//                    tile's weight-gradient products run while the backward
-//                    epilogues and the next tile's first product go on.  At
-//                    the end each block writes its gradient sums from tensor
-//                    memory to global memory, feature-major (coalesced
-//                    stores; layout below).
+//                               block's tiles (K = the tile's records):
+//                               d0^T [1 | h2] (b3, dW3), d2^T [h1 | 1] (dW2,
+//                               b2) and d1^T [x | 1] (dW1, b1).
+//                    A tile's activations are one matrix of 128 records in the
+//                    canonical layout, which the forward and backward products
+//                    read as a K-major operand and the gradient products as
+//                    an MN-major one (M or N = features, K = records); d2
+//                    takes h2's place and d1 takes h1's, each when the
+//                    gradient product that reads the activation is done.
+//                    A group splits each epilogue's 64 accumulator columns
+//                    over its two warpgroups, and each record's loss (four
+//                    lobes each).  At the end each block writes its gradient
+//                    sums from tensor memory to global memory, feature-major
+//                    (coalesced stores; layout below).
 //   k_guide_grad_reduce  sums the blocks' partials in a fixed order (no
 //                    atomics) into the gradient, in the parameter layout,
 //                    applying the loss's 1/n.
@@ -227,16 +225,35 @@ __device__ __forceinline__ float record_grad_half(const float* o, float3 w, floa
 // (with n ~ 1e5 records most of them would be fp16 subnormals); they
 // saturate at the fp16 range, and the 1/n is applied, in fp32, in the
 // reduction.
-constexpr int kTrThreads = 2 * kTcRows;                // two warpgroups
-// operand matrices in shared memory (halves per record, feature offsets)
-constexpr int kXK = kGEnc + 16, kXones = kGEnc;        // X = [x | 1]
-constexpr int kHK = 144, kHh1 = 0, kHones = 64, kHh2 = 80;  // H = [h1 | 1 | h2]
-constexpr int kDK = 192, kDd1 = 0, kDd2 = 64, kDd0 = 128;   // D = [d1 | d2 | d0 | 0]
-// tensor memory: the gradient sums (columns 0..303) and the forward /
-// backward accumulator (64 columns, reused by every product)
+//
+// What bounds it: a tile is a chain of six dependent steps -- products, their
+// completion, an epilogue over 128 rows, a barrier -- of 10600 cycles when a
+// block works on one tile, the tensor cores busy for 2600 of them (55
+// products of 128 rows, 48 to 82 cycles each: at these widths the operands'
+// way from shared memory sets the time).  The second tile in the first one's
+// waits makes it 13400 cycles for two.  The issuing warp keeps its control
+// flow converged and predicates the instructions on one lane: descriptors
+// then stay in uniform registers (issued from one lane's branch, a product
+// took 100 cycles).  131072 records: 51.8 us for the batch's kernels with one
+// tile at a time and its two warpgroups, 41.5 with two; 64 records 15 us
+// either way.  Shared memory holds two tiles, not three (88 KB each, beside
+// 47 KB of weights).
+// The two chains' products are issued in a fixed order (step by step, the
+// first group's before the second's), so that the gradient sums are added
+// tile by tile in the same order whatever the groups' timing.
+constexpr int kTrGroup = 2 * kTcRows;                  // threads of a group: two warpgroups
+constexpr int kTrGroups = 2;
+constexpr int kTrThreads = kTrGroups * kTrGroup + 32;  // and the issuing warp
+// a tile's operand matrix [x | 1 | h1, then d1 | 1 | h2, then d2 | d0]
+// (halves per record, feature offsets)
+constexpr int kR1x = kGEnc, kRh1 = kR1x + 16, kR1h = kRh1 + kGHid, kRh2 = kR1h + 16, kRd0 = kRh2 + kGHid;
+constexpr int kRK = kRd0 + kGOutPad;
+// tensor memory: the gradient sums -- [dW1 | b1], [dW2 | b2], [b3 | dW3] --
+// and each group's forward / backward accumulator (64 columns, reused by
+// every product)
 constexpr int kTrCols = 512;
-constexpr int kAccA = 0, kAccB = kXK, kAccF = 384;
-static_assert(kAccB + kHK <= kAccF && kAccF + kGHid <= kTrCols, "tensor-memory columns");
+constexpr int kAcc1 = 0, kAcc2 = kAcc1 + kGEnc + 16, kAcc3 = kAcc2 + kGHid + 16, kAccF = kAcc3 + kGHid + 16;
+static_assert(kAccF + kTrGroups * kGHid <= kTrCols, "tensor-memory columns");
 constexpr float kHalfMax = 65504.f;
 // A block's gradient sums in global memory, feature-major so that a warp's
 // 32 units (accumulator lanes) of one feature are 32 consecutive floats:
@@ -258,38 +275,42 @@ static_assert(guide_sum_param(kPSums - 1) == kGB3 + kGOut - 1 && guide_sum_param
               "sum layout");
 
 struct GuideTrSmem {
-    __half w[kGImgHalves];                    // the weight image: weights, biases,
+    // (a gradient product's 128 rows of A may start at a tile's last features
+    // and reach up to 1.3 KB past it -- the other tile or the weights -- in
+    // rows of the accumulator that nobody reads)
+    alignas(128) __half rec[kTrGroups][kTcRows * kRK];
+    alignas(128) __half w[kGImgHalves];       // the weight image: weights, biases,
     float bias[kGImgBiases];                  // W2^T and W3^T
     __half w2t[kGHid * kGHid];
     __half w3t[kGHid * kGOutPad];
-    alignas(128) __half x[2][kTcRows * kXK];  // this tile's X and the next tile's
-    alignas(128) __half h[kTcRows * kHK];
-    alignas(128) __half d[kTcRows * kDK];
-    float4 ex[2][kTcRows];                    // the two halves' mixture sums of each record
-    uint64_t bar_w, bar_mma;
+    uint64_t bar_w;                           // the weight image has landed
+    uint64_t bar_ready[kTrGroups];            // the group's step is written (8 warps)
+    uint64_t bar_done[kTrGroups];             // its product is in the accumulator
+    uint64_t bar_grad[kTrGroups];             // its gradient products have read their operands
+    uint64_t bar_ex[kTrGroups];               // the mixture sums are written (8 warps)
+    uint64_t bar_end;                         // every product of the block is complete
     uint32_t tmem;
-    float mean;
+    float mean[kTrGroups];
     int fail;
 };
-static_assert(offsetof(GuideTrSmem, w2t) == kGImgW2T && offsetof(GuideTrSmem, w3t) == kGImgW3T, "image layout");
+static_assert(offsetof(GuideTrSmem, w2t) - offsetof(GuideTrSmem, w) == kGImgW2T &&
+                  offsetof(GuideTrSmem, w3t) - offsetof(GuideTrSmem, w) == kGImgW3T, "image layout");
 static_assert(sizeof(GuideTrSmem) + 1024 <= 227 * 1024, "one training block per SM");
 // no other tensor-memory user of this library (the guided material blocks,
 // 107 KB; the inference block, 218 KB) fits beside a block: its 512 columns
 // are free
 static_assert(sizeof(GuideTrSmem) + 1024 + 107 * 1024 > 228 * 1024, "one tensor-memory user per SM");
 
-__device__ __forceinline__ uint32_t pack_h2(float a, float b) {
-    __half2 h = __floats2half2_rn(a, b);
-    return *reinterpret_cast<const uint32_t*>(&h);
-}
-__device__ __forceinline__ uint32_t pack_h2_sat(float a, float b) {
-    return pack_h2(fminf(fmaxf(a, -kHalfMax), kHalfMax), fminf(fmaxf(b, -kHalfMax), kHalfMax));
+__device__ __forceinline__ uint32_t as_u32(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
+__device__ __forceinline__ __half2 as_h2(uint32_t u) { return *reinterpret_cast<const __half2*>(&u); }
+// Two values as fp16, saturated at the fp16 range (NaN: the lower end).
+__device__ __forceinline__ __half2 pack_h2_sat(float a, float b) {
+    const __half2 lim = __float2half2_rn(kHalfMax);
+    return __hmin2(__hmax2(__floats2half2_rn(a, b), __hneg2(lim)), lim);
 }
 
-// Input i of a record, encoded into features 24 i .. 24 i + 23 of row r of X.
-__device__ __forceinline__ void tr_encode(float v, __half* x, int r, int i) {
-    __half2 h[kGFreq];
-    encode_scalar_h2(v, h);
+// An encoded input into features 24 i .. 24 i + 23 of row r.
+__device__ __forceinline__ void tr_store_input(const __half2* h, __half* rec, int r, int i) {
 #pragma unroll
     for (int c = 0; c < 3; c++) {
         uint4 q;
@@ -297,75 +318,113 @@ __device__ __forceinline__ void tr_encode(float v, __half* x, int r, int i) {
         q.y = *reinterpret_cast<const uint32_t*>(&h[4 * c + 1]);
         q.z = *reinterpret_cast<const uint32_t*>(&h[4 * c + 2]);
         q.w = *reinterpret_cast<const uint32_t*>(&h[4 * c + 3]);
-        *reinterpret_cast<uint4*>(x + canon_index(r, i * 2 * kGFreq + 8 * c, kXK)) = q;
+        *reinterpret_cast<uint4*>(rec + canon_index(r, i * 2 * kGFreq + 8 * c, kRK)) = q;
     }
 }
 
 // Bias + ReLU of the 32 accumulator columns c0 .. c0 + 31 (at t, the warp's
-// lanes) into H at feature hf + c0; returns the mask of the outputs that are
-// > 0 after rounding (bit j: column c0 + j).
-__device__ __forceinline__ uint32_t tr_hidden_epilogue(uint32_t t, int c0, const float* bias, __half* H, int hf) {
-    const int r = threadIdx.x & (kTcRows - 1);
+// lanes) into the record's features hf + c0.
+__device__ __forceinline__ void tr_hidden_epilogue(uint32_t t, int c0, const float* bias, __half* rec, int r, int hf) {
     float v[32];
     tc::ld_32x32b_x32(t + c0, v);
-    uint32_t mask = 0, p[16];
+    const __half2 zero = __float2half2_rn(0.f);
+    auto act = [&](int j) {
+        return as_u32(__hmax2(__floats2half2_rn(v[j] + bias[c0 + j], v[j + 1] + bias[c0 + j + 1]), zero));
+    };
 #pragma unroll
-    for (int j = 0; j < 16; j++) {
-        __half2 h = __floats2half2_rn(fmaxf(v[2 * j] + bias[c0 + 2 * j], 0.f),
-                                      fmaxf(v[2 * j + 1] + bias[c0 + 2 * j + 1], 0.f));
-        if (__low2float(h) > 0.f) mask |= 1u << (2 * j);
-        if (__high2float(h) > 0.f) mask |= 1u << (2 * j + 1);
-        p[j] = *reinterpret_cast<const uint32_t*>(&h);
+    for (int q = 0; q < 32; q += 8)
+        *reinterpret_cast<uint4*>(rec + canon_index(r, hf + c0 + q, kRK)) =
+            make_uint4(act(q), act(q + 2), act(q + 4), act(q + 6));
+}
+
+// The gradients in the 32 accumulator columns c0 .. c0 + 31, as fp16
+// (saturated), where the activation they belong to (the record's features hf
+// + c0, which they will replace) is positive.
+__device__ __forceinline__ void tr_masked(uint32_t t, int c0, const __half* rec, int r, int hf, uint4* p) {
+    float v[32];
+    tc::ld_32x32b_x32(t + c0, v);
+    const __half2 zero = __float2half2_rn(0.f);
+    auto grad = [&](int j, uint32_t h) { return as_u32(pack_h2_sat(v[j], v[j + 1])) & __hgt2_mask(as_h2(h), zero); };
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const uint4 h = *reinterpret_cast<const uint4*>(rec + canon_index(r, hf + c0 + 8 * q, kRK));
+        p[q] = make_uint4(grad(8 * q, h.x), grad(8 * q + 2, h.y), grad(8 * q + 4, h.z), grad(8 * q + 6, h.w));
     }
+}
+__device__ __forceinline__ void tr_store_features(const uint4* p, __half* rec, int r, int f) {
 #pragma unroll
-    for (int q = 0; q < 4; q++)
-        *reinterpret_cast<uint4*>(H + canon_index(r, hf + c0 + 8 * q, kHK)) =
-            make_uint4(p[4 * q], p[4 * q + 1], p[4 * q + 2], p[4 * q + 3]);
-    return mask;
+    for (int q = 0; q < 4; q++) *reinterpret_cast<uint4*>(rec + canon_index(r, f + 8 * q, kRK)) = p[q];
 }
 
-// The 32 accumulator columns c0 .. c0 + 31, masked by `mask`, into D at
-// feature df + c0 (fp16, saturated).
-__device__ __forceinline__ void tr_backward_epilogue(uint32_t t, int c0, uint32_t mask, __half* D, int df) {
-    const int r = threadIdx.x & (kTcRows - 1);
-    float v[32];
-    tc::ld_32x32b_x32(t + c0, v);
-    uint32_t p[16];
-#pragma unroll
-    for (int j = 0; j < 16; j++)
-        p[j] = pack_h2_sat((mask >> (2 * j)) & 1u ? v[2 * j] : 0.f, (mask >> (2 * j + 1)) & 1u ? v[2 * j + 1] : 0.f);
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-        *reinterpret_cast<uint4*>(D + canon_index(r, df + c0 + 8 * q, kDK)) =
-            make_uint4(p[4 * q], p[4 * q + 1], p[4 * q + 2], p[4 * q + 3]);
-}
-
-// acc (128 x N) = A x W^T: A = K features of the tile's rows, starting at
-// byte address a in a matrix with rows of `arow` halves (K-major); W [N][K]
-// at w (rows of K halves).  Completion on `bar`.
+// acc (128 x N) = A x W^T: A = K features from af of the tile at rec
+// (K-major); W [N][K] at w (rows of K halves).  A descriptor's address field
+// counts 16 bytes and the tiles end below 2^18, so that steps along K add to it.
 template <int K, int N>
-__device__ __forceinline__ void tr_issue(uint32_t acc, uint32_t a, int arow, uint32_t w, uint64_t* bar) {
+__device__ __forceinline__ void tr_issue(bool leader, uint32_t acc, uint32_t rec, int af, uint32_t w) {
     constexpr uint32_t idesc = tc::idesc_f16_f32(kTcRows, N);
-    tc::fence_after_sync();
+    const uint64_t a = tc::smem_desc(rec + (af / 8) * 128, 128, kRK * 16), b = tc::smem_desc(w, 128, K * 16);
 #pragma unroll
     for (int ks = 0; ks < K / 16; ks++)
-        tc::mma_f16(acc, tc::smem_desc(a + ks * 256, 128, arow * 16), tc::smem_desc(w + ks * 256, 128, K * 16), idesc,
-                    ks > 0 ? 1u : 0u);
-    tc::commit(bar);
+        tc::mma_f16_by(leader, acc, a + ks * (256 / 16), b + ks * (256 / 16), idesc, ks > 0 ? 1u : 0u);
 }
 
 // Gradient sums (acc, N columns) += A^T B over the tile's 128 records, 16
 // per instruction (the block's first tile initialises them): A = 128
-// features of D from feature af, B = N features of a matrix of `brow`
-// halves per record at b, both MN-major.  No completion signal of its own:
-// the next product's commit covers it.
+// features of the tile from af (those past the wanted ones fill accumulator
+// lanes that are never read), B = N features from bf, both MN-major.
 template <int N>
-__device__ __forceinline__ void tr_issue_grad(uint32_t acc, uint32_t da, int af, uint32_t b, int brow, bool first) {
+__device__ __forceinline__ void tr_issue_grad(bool leader, uint32_t acc, uint32_t rec, int af, int bf, bool first) {
     constexpr uint32_t idesc = tc::idesc_f16_f32(kTcRows, N, true, true);
+    const uint64_t a = tc::smem_desc(rec + (af / 8) * 128, kRK * 16, 128);
+    const uint64_t b = tc::smem_desc(rec + (bf / 8) * 128, kRK * 16, 128);
 #pragma unroll
     for (int ks = 0; ks < kTcRows / 16; ks++)
-        tc::mma_f16(acc, tc::smem_desc(da + (af / 8) * 128 + ks * 2 * kDK * 16, kDK * 16, 128),
-                    tc::smem_desc(b + ks * 2 * brow * 16, brow * 16, 128), idesc, first && ks == 0 ? 0u : 1u);
+        tc::mma_f16_by(leader, acc, a + ks * 2 * kRK, b + ks * 2 * kRK, idesc, first && ks == 0 ? 0u : 1u);
+}
+
+// The block's products, step by step of each pair of tiles, the first
+// group's before the second's: one converged warp, one lane of which issues
+// them.  Returns false when a wait ran out.
+__device__ __forceinline__ bool tr_issue_all(GuideTrSmem& S, int ntiles) {
+    constexpr int kSteps = 6;
+    const bool leader = tc::elect_one();
+    const uint32_t T = S.tmem, wa = tc::smem_addr(S.w);
+    auto wait = [](uint64_t* bar, uint32_t ph) {
+        return __any_sync(0xffffffffu, !tc::mbar_wait(bar, ph, kTcWaitNs)) == 0;
+    };
+    bool ok = wait(&S.bar_w, 0);
+    uint32_t ph = 0;
+    for (int tile = blockIdx.x, pair = 0; ok && tile < ntiles; tile += kTrGroups * gridDim.x, pair++) {
+        for (int step = 0; ok && step < kSteps; step++, ph ^= 1u) {
+            for (int g = 0; g < kTrGroups && tile + g * (int)gridDim.x < ntiles; g++) {
+                ok = wait(&S.bar_ready[g], ph);
+                if (!ok) break;
+                tc::fence_after_sync();
+                const uint32_t F = T + kAccF + g * kGHid, rec = tc::smem_addr(S.rec[g]);
+                const bool first = pair == 0 && g == 0;
+                if (step == 0) {          // x -> h1
+                    tr_issue<kGEnc, kGHid>(leader, F, rec, 0, wa + 2 * kGImgW1);
+                } else if (step == 1) {   // h1 -> h2
+                    tr_issue<kGHid, kGHid>(leader, F, rec, kRh1, wa + 2 * kGImgW2);
+                } else if (step == 2) {   // h2 -> outputs
+                    tr_issue<kGHid, kGOutPad>(leader, F, rec, kRh2, wa + 2 * kGImgW3);
+                } else if (step == 3) {   // d0 W3 -> d2; d0^T [1 | h2]
+                    tr_issue<kGOutPad, kGHid>(leader, F, rec, kRd0, wa + kGImgW3T);
+                    tc::commit_by(leader, &S.bar_done[g]);
+                    tr_issue_grad<kGHid + 16>(leader, T + kAcc3, rec, kRd0, kR1h, first);
+                } else if (step == 4) {   // d2 W2 -> d1; d2^T [h1 | 1]
+                    tr_issue<kGHid, kGHid>(leader, F, rec, kRh2, wa + kGImgW2T);
+                    tc::commit_by(leader, &S.bar_done[g]);
+                    tr_issue_grad<kGHid + 16>(leader, T + kAcc2, rec, kRh2, kRh1, first);
+                } else {                  // d1^T [x | 1]
+                    tr_issue_grad<kGEnc + 16>(leader, T + kAcc1, rec, kRh1, 0, first);
+                }
+                tc::commit_by(leader, step < 3 ? &S.bar_done[g] : &S.bar_grad[g]);
+            }
+        }
+    }
+    tc::commit_by(leader, &S.bar_end);
+    return ok;
 }
 
 __global__ void __launch_bounds__(kTrThreads, 1) k_guide_train(const void* image, const GuideRecord* s, int n,
@@ -373,184 +432,180 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_guide_train(const void* image
                                                                 float* partial, float* loss, unsigned* err) {
     extern __shared__ __align__(128) unsigned char dyn_smem[];
     GuideTrSmem& S = *reinterpret_cast<GuideTrSmem*>(dyn_smem);
-    const int tid = threadIdx.x, g = tid >> 7, r = tid & (kTcRows - 1);
+    const int tid = threadIdx.x, lane = tid & 31;
+    const bool issuer = tid >= kTrGroups * kTrGroup;                // the issuing warp
+    const int grp = (tid / kTrGroup) % kTrGroups, gt = tid % kTrGroup;
+    const int g = gt >> 7, r = gt & (kTcRows - 1);                  // half of the group, record of the tile
     const int ntiles = (n + kTcRows - 1) / kTcRows;
-    if (tid == 0) {
+    if (tid == kTrGroups * kTrGroup) {
         tc::mbar_init(&S.bar_w, 1);
-        tc::mbar_init(&S.bar_mma, 1);
+        tc::mbar_init(&S.bar_end, 1);
+        for (int i = 0; i < kTrGroups; i++) {
+            tc::mbar_init(&S.bar_ready[i], kTrGroup / 32);
+            tc::mbar_init(&S.bar_done[i], 1);
+            tc::mbar_init(&S.bar_grad[i], 1);
+            tc::mbar_init(&S.bar_ex[i], kTrGroup / 32);
+        }
         S.fail = 0;
     }
-    if (tid < 32) tc::tmem_alloc(&S.tmem, kTrCols);
+    if (issuer) tc::tmem_alloc(&S.tmem, kTrCols);
     tc::pdl_launch_dependents();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    // the weight copy lands while the first tile's records load and encode
-    if (tid == 0) tc::bulk_load(S.w, image, kGImgTrainBytes, &S.bar_w);
-    {   // the constant columns, the same for every tile: ones of X (both
-        // buffers) and H, zeros of D after d0's 40 outputs
-        const uint32_t one2 = pack_h2(1.f, 1.f);
-        const uint4 ones = make_uint4(one2, one2, one2, one2), zeros = make_uint4(0u, 0u, 0u, 0u);
-        for (int c = 0; c < 16; c += 8) {
-            *reinterpret_cast<uint4*>(S.x[g] + canon_index(r, kXones + c, kXK)) = ones;
-            if (g == 0) *reinterpret_cast<uint4*>(S.h + canon_index(r, kHones + c, kHK)) = ones;
-        }
-        for (int c = kDd0 + kGOut + 8 * g; c < kDK; c += 16)
-            *reinterpret_cast<uint4*>(S.d + canon_index(r, c, kDK)) = zeros;
-    }
-    bool failed = false;
-    uint32_t ph = 0;
-    auto wait = [&]() {
-        if (!tc::mbar_wait(&S.bar_mma, ph, kTcWaitNs)) {
-            failed = true;
-            S.fail = 1;
-            atomicOr(err, kErrTensorWait);
-        } else {
-            ph ^= 1u;
-        }
-        tc::fence_after_sync();
-    };
-    // all threads done with the step's shared and tensor memory: returns
-    // true (in every thread) when a wait has failed
-    auto step_sync = [&]() {
-        tc::fence_smem_to_async();
-        tc::fence_before_sync();
-        return __syncthreads_or(failed) != 0;
-    };
+    // the weight copy lands while the first tiles' records load and encode
+    if (tid == kTrGroups * kTrGroup) tc::bulk_load(S.w, image, kGImgTrainBytes, &S.bar_w);
     const uint32_t T = S.tmem;
-    const uint32_t tf = T + kAccF + ((uint32_t)(tid & 96) << 16);   // forward accumulator, this warp's lanes
-    const int ch = 32 * g;                                          // this warpgroup's epilogue columns
-    const uint32_t xa0 = tc::smem_addr(S.x[0]), ha = tc::smem_addr(S.h), da = tc::smem_addr(S.d);
-    const uint32_t wa = tc::smem_addr(S.w);
-    constexpr uint32_t kXBytes = kTcRows * kXK * 2;
+    const uint32_t lanes = (uint32_t)(tid & 96) << 16;              // this warp's accumulator lanes
     float lacc = 0.f;
-    bool any = false;
-    // a record as three float4: in[0..3] | in[4], in[5], w[0], w[1] | w[2], pdf, L, pad
-    auto load_rec = [&](int row, float4* q) {
-        if (row < n) {
-            const float4* p = reinterpret_cast<const float4*>(s + (size_t)row * stride);
-            q[0] = p[0];
-            q[1] = p[1];
-            q[2] = p[2];
-        } else {
-            q[0] = q[1] = q[2] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+    bool failed = false;
+    // bounded wait of the whole warp; a warp whose wait ran out leaves its
+    // loop, and the waits of the others then run out in turn
+    auto wait = [&](uint64_t* bar, uint32_t& ph) {
+        const bool ok = tc::mbar_wait(bar, ph, kTcWaitNs);
+        ph ^= 1u;
+        failed = __any_sync(0xffffffffu, !ok) != 0;
+        tc::fence_after_sync();
+        return !failed;
     };
-    // input 3g + i of a record
-    auto input = [&](const float4* q, int i) {
-        const int j = 3 * g + i;
-        return j == 0 ? q[0].x : j == 1 ? q[0].y : j == 2 ? q[0].z : j == 3 ? q[0].w : j == 4 ? q[1].x : q[1].y;
-    };
-    float4 cur[3], nxt[3];
-    int k = 0;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, k++) {
-        const int row = tile * kTcRows + r;
-        const int b = k & 1;
-        const bool more = tile + (int)gridDim.x < ntiles;
-        if (k == 0) {
-            // the first tile's encoding: inputs 3g .. 3g + 2 of each record
-            load_rec(row, cur);
+    if (issuer) {
+        failed = !tr_issue_all(S, ntiles);
+    } else {
+        __half* rec = S.rec[grp];
+        const uint32_t tf = T + kAccF + grp * kGHid + lanes;        // the group's accumulator, this warp's lanes
+        const int ch = 32 * g;                                      // this warpgroup's epilogue columns
+        uint32_t ph_w = 0, ph_done = 0, ph_grad = 0, ph_ex = 0;
+        // this warp's part of a step is written and its accumulator reads are done
+        auto ready = [&]() {
+            tc::fence_smem_to_async();
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&S.bar_ready[grp]);
+        };
+        // inputs 3g .. 3g + 2 of a record (zeros past the last one); each is
+        // loaded a product or two before it is used
+        auto load_inputs = [&](int row, float* in) {
+            const float* q = reinterpret_cast<const float*>(s + (size_t)row * stride);
 #pragma unroll
-            for (int i = 0; i < 3; i++) tr_encode(input(cur, i), S.x[0], r, 3 * g + i);
-            if (!tc::mbar_wait(&S.bar_w, 0, kTcWaitNs)) {
-                failed = true;
-                S.fail = 1;
-                atomicOr(err, kErrTensorWait);
+            for (int i = 0; i < 3; i++) in[i] = row < n ? q[3 * g + i] : 0.f;
+        };
+        const int step = kTrGroups * gridDim.x;
+        int tile = blockIdx.x + grp * (int)gridDim.x;
+        if (tile < ntiles) {
+            // what every tile shares -- the columns of ones, the zeros after
+            // d0's 40 outputs -- and the first tile's encoding
+            const uint32_t one2 = as_u32(__float2half2_rn(1.f));
+            const uint4 ones = make_uint4(one2, one2, one2, one2);
+            *reinterpret_cast<uint4*>(rec + canon_index(r, kR1x + 8 * g, kRK)) = ones;
+            *reinterpret_cast<uint4*>(rec + canon_index(r, kR1h + 8 * g, kRK)) = ones;
+            if (g == 0) *reinterpret_cast<uint4*>(rec + canon_index(r, kRd0 + kGOut, kRK)) = make_uint4(0u, 0u, 0u, 0u);
+            float in[3];
+            load_inputs(tile * kTcRows + r, in);
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                __half2 h[kGFreq];
+                encode_scalar_h2(in[i], h);
+                tr_store_input(h, rec, r, 3 * g + i);
             }
-            if (step_sync()) break;
-        }
-        // (later tiles: their X was complete at the previous tile's last barrier)
-        // the next tile's records arrive while this tile's first products run
-        if (more) load_rec((tile + (int)gridDim.x) * kTcRows + r, nxt);
-        const uint32_t xa = xa0 + b * kXBytes;
-        // layer 1: x -> h1 (after the previous tile's gradient products,
-        // which read H and D: the commit covers them)
-        if (tid == 0) tr_issue<kGEnc, kGHid>(T + kAccF, xa, kXK, wa + 2 * kGImgW1, &S.bar_mma);
-        if (k == 0) {
+            ready();
             tc::pdl_wait();   // k_guide_weight_sum has finished
-            if (tid < 32) {   // the batch's mean weight, summed the same way in every block
+            if (gt < 32) {    // the batch's mean weight, summed the same way in every block
                 float sum = 0.f;
-                for (int j = tid; j < nwsum; j += 32) sum += wsum[j];
+                for (int j = lane; j < nwsum; j += 32) sum += wsum[j];
                 for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-                if (tid == 0) S.mean = sum / (float)n;
+                if (lane == 0) S.mean[grp] = sum / (float)n;
+            }
+            (void)wait(&S.bar_w, ph_w);   // the biases
+        }
+        for (; tile < ntiles && !failed; tile += step) {
+            const int row = tile * kTcRows + r;
+            const bool more = tile + step < ntiles;
+            if (!wait(&S.bar_done[grp], ph_done)) break;
+            tr_hidden_epilogue(tf, ch, S.bias + kGImgB1, rec, r, kRh1);
+            ready();
+            if (!wait(&S.bar_done[grp], ph_done)) break;
+            tr_hidden_epilogue(tf, ch, S.bias + kGImgB2, rec, r, kRh2);
+            ready();
+            // the record's direction, pdf and radiance: in[6] | w[3], pdf, L
+            float2 q0 = make_float2(0.f, 0.f), q1 = q0, q2 = q0;
+            if (row < n) {
+                const float2* q = reinterpret_cast<const float2*>(s + (size_t)row * stride) + 3;
+                q0 = q[0];
+                q1 = q[1];
+                q2 = q[2];
+            }
+            if (!wait(&S.bar_done[grp], ph_done)) break;
+            {   // loss and dLoss/dOutput (times n) of the record, lobes 4g .. 4g + 3, into d0 (features 20g ..)
+                float o[20];
+                float v[32];
+                tc::ld_32x32b_x32(tf + 16 * g, v);   // columns 16g .. 16g + 31 hold outputs 20g .. 20g + 19
+#pragma unroll
+                for (int j = 0; j < 20; j++) o[j] = (g ? v[4 + j] : v[j]) + S.bias[kGImgB3 + 20 * g + j];
+                float dd[20];
+                // the halves' sums change hands in d0's place: each half's lie
+                // where the other half, having read them, writes its gradients
+                float4* ex_mine = reinterpret_cast<float4*>(rec + canon_index(r, kRd0 + (g ? 0 : 24), kRK));
+                const float4* ex_other = reinterpret_cast<float4*>(rec + canon_index(r, kRd0 + (g ? 24 : 0), kRK));
+                const float lr = record_grad_half(
+                    o, f3(q0.x, q0.y, q1.x), ex_mine, ex_other,
+                    [&]() {
+                        __syncwarp();
+                        if (lane == 0) tc::mbar_arrive(&S.bar_ex[grp]);
+                        (void)wait(&S.bar_ex[grp], ph_ex);
+                        // the record's loss weight times n (the mean was written before the exchange)
+                        const float mean = S.mean[grp], pdf = q1.y, Lr = q2.x;
+                        return row < n && pdf > 0.f && mean > 0.f ? fminf(Lr / pdf / mean, kGTargetClamp) : 0.f;
+                    },
+                    dd);
+                if (failed) break;
+                if (g == 0) lacc += lr;
+#pragma unroll
+                for (int c = 0; c < 20; c += 4)
+                    *reinterpret_cast<uint2*>(rec + canon_index(r, kRd0 + 20 * g + c, kRK)) =
+                        make_uint2(as_u32(pack_h2_sat(dd[c], dd[c + 1])), as_u32(pack_h2_sat(dd[c + 2], dd[c + 3])));
+            }
+            ready();
+            float in[3] = {0.f, 0.f, 0.f};   // of the next tile
+            if (more) load_inputs(row + step * kTcRows, in);
+            uint4 p[4];
+            if (!wait(&S.bar_done[grp], ph_done)) break;
+            tr_masked(tf, ch, rec, r, kRh2, p);
+            if (!wait(&S.bar_grad[grp], ph_grad)) break;   // dW3's product has read h2
+            tr_store_features(p, rec, r, kRh2 + ch);
+            ready();
+            if (!wait(&S.bar_done[grp], ph_done)) break;
+            tr_masked(tf, ch, rec, r, kRh1, p);
+            if (!wait(&S.bar_grad[grp], ph_grad)) break;   // dW2's product has read h1
+            tr_store_features(p, rec, r, kRh1 + ch);
+            ready();
+            if (!wait(&S.bar_grad[grp], ph_grad)) break;
+            if (more) {
+#pragma unroll
+                for (int i = 0; i < 3; i++) { __half2 h[kGFreq]; encode_scalar_h2(in[i], h); tr_store_input(h, rec, r, 3 * g + i); }
+                ready();
             }
         }
-        wait();
-        const uint32_t m1 = tr_hidden_epilogue(tf, ch, S.bias + kGImgB1, S.h, kHh1);
-        if (step_sync()) break;
-        // the record's loss weight times n (the mean is visible after the barrier)
-        const float mean = S.mean;
-        const float pdf = cur[2].y, Lr = cur[2].z;
-        const float sc = row < n && pdf > 0.f && mean > 0.f ? fminf(Lr / pdf / mean, kGTargetClamp) : 0.f;
-        // layer 2: h1 -> h2.  While a product runs, each thread encodes one
-        // of its three inputs of the next tile into the other X buffer (its
-        // last reader, the previous tile's gradient product, has completed)
-        if (tid == 0) tr_issue<kGHid, kGHid>(T + kAccF, ha + (kHh1 / 8) * 128, kHK, wa + 2 * kGImgW2, &S.bar_mma);
-        if (more) tr_encode(input(nxt, 0), S.x[b ^ 1], r, 3 * g);
-        wait();
-        const uint32_t m2 = tr_hidden_epilogue(tf, ch, S.bias + kGImgB2, S.h, kHh2);
-        if (step_sync()) break;
-        // layer 3: h2 -> outputs
-        if (tid == 0) tr_issue<kGHid, kGOutPad>(T + kAccF, ha + (kHh2 / 8) * 128, kHK, wa + 2 * kGImgW3, &S.bar_mma);
-        if (more) tr_encode(input(nxt, 1), S.x[b ^ 1], r, 3 * g + 1);
-        wait();
-        {   // loss and dLoss/dOutput (times n) of the record, lobes 4g .. 4g + 3, into D (d0 features 20g ..)
-            float o[20];
-            float v[32];
-            tc::ld_32x32b_x32(tf + 16 * g, v);   // columns 16g .. 16g + 31 hold outputs 20g .. 20g + 19
-#pragma unroll
-            for (int j = 0; j < 20; j++) o[j] = (g ? v[4 + j] : v[j]) + S.bias[kGImgB3 + 20 * g + j];
-            float dd[20];
-            const float lr = record_grad_half(o, f3(cur[1].z, cur[1].w, cur[2].x), sc, &S.ex[g][r], &S.ex[g ^ 1][r],
-                                              dd);
-            if (g == 0) lacc += lr;
-#pragma unroll
-            for (int c = 0; c < 20; c += 4)
-                *reinterpret_cast<uint2*>(S.d + canon_index(r, kDd0 + 20 * g + c, kDK)) =
-                    make_uint2(pack_h2_sat(dd[c], dd[c + 1]), pack_h2_sat(dd[c + 2], dd[c + 3]));
-        }
-        if (step_sync()) break;
-        // backward through layer 3: d0 W3 -> d2
-        if (tid == 0) tr_issue<kGOutPad, kGHid>(T + kAccF, da + (kDd0 / 8) * 128, kDK, wa + kGImgW3T, &S.bar_mma);
-        if (more) tr_encode(input(nxt, 2), S.x[b ^ 1], r, 3 * g + 2);
-        wait();
-        tr_backward_epilogue(tf, ch, m2, S.d, kDd2);
-        if (step_sync()) break;
-        // backward through layer 2: d2 W2 -> d1; then, behind it on the
-        // tensor cores, [d2 | d0]^T [h1 | 1 | h2] (its inputs are complete
-        // and nothing writes them before the next tile's first product)
-        if (tid == 0) {
-            tr_issue<kGHid, kGHid>(T + kAccF, da + (kDd2 / 8) * 128, kDK, wa + kGImgW2T, &S.bar_mma);
-            tr_issue_grad<kHK>(T + kAccB, da, kDd2, ha, kHK, k == 0);
-        }
-        wait();
-        tr_backward_epilogue(tf, ch, m1, S.d, kDd1);
-        if (step_sync()) break;
-        // [d1 | d2]^T [x | 1]; it completes before the next tile's first
-        // product does (one issuing thread, products in order), which every
-        // thread waits for before it writes H, D or this X buffer again
-        if (tid == 0) tr_issue_grad<kXK>(T + kAccA, da, kDd1, xa, kXK, k == 0);
-        any = true;
-#pragma unroll
-        for (int i = 0; i < 3; i++) cur[i] = nxt[i];
     }
-    // every product of the block complete (after a failed wait: skipped)
-    tc::fence_before_sync();
-    if (__syncthreads_or(failed) == 0 && any) {
-        if (tid == 0) tc::commit(&S.bar_mma);
-        wait();
+    if (failed && lane == 0) {
+        S.fail = 1;
+        atomicOr(err, kErrTensorWait);
     }
+    // every product of the block complete
+    __syncthreads();
+    uint32_t ph_end = 0;
+    if (!wait(&S.bar_end, ph_end) && lane == 0) {
+        S.fail = 1;
+        atomicOr(err, kErrTensorWait);
+    }
+    __syncthreads();
+    const bool live = S.fail == 0 && (int)blockIdx.x < ntiles;
     for (int o = 16; o; o >>= 1) lacc += __shfl_xor_sync(0xffffffffu, lacc, o);
-    if (g == 0 && (tid & 31) == 0 && any) atomicAdd(loss, lacc / (float)n);
-    tc::fence_before_sync();
-    const bool bad = __syncthreads_or(failed) != 0;
-    tc::fence_after_sync();
+    if (!issuer && g == 0 && lane == 0) atomicAdd(loss, lacc / (float)n);
     // the block's gradient sums (feature-major: each store of a warp writes
-    // one feature of its 32 units, 128 contiguous bytes); warps w and w + 4
-    // read the same accumulator lanes and split the columns
+    // one feature of its 32 units, 128 contiguous bytes): accumulator lanes
+    // 0..63 hold unit r of layer 1, unit r of layer 2 and output r (< 40);
+    // the four warpgroups split the columns
     float* out = partial + (size_t)blockIdx.x * kPSums;
-    const uint32_t tl = T + ((uint32_t)(tid & 96) << 16);
-    const bool live = any && !bad;
     // ncols (16 or 32) columns from col: column j to out[dst + j * stride];
     // stride 0: a bias (its 16 columns of ones hold the same sum), column 0 only
     auto run = [&](uint32_t col, int ncols, int dst, int stride, bool keep) {
@@ -559,36 +614,38 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_guide_train(const void* image
 #pragma unroll
             for (int j = 0; j < 32; j++) v[j] = 0.f;
         } else if (ncols == 32) {
-            tc::ld_32x32b_x32(tl + col, v);
+            tc::ld_32x32b_x32(T + lanes + col, v);
         } else {
-            tc::ld_32x32b_x16(tl + col, v);
+            tc::ld_32x32b_x16(T + lanes + col, v);
         }
         if (keep && stride == 0) out[dst] = v[0];
         if (keep && stride > 0)
             for (int j = 0; j < ncols; j++) out[dst + j * stride] = v[j];
     };
-    if (r < kGHid) {   // accumulator lanes 0..63: unit r of layer 1 (first sums), of layer 2 (second sums)
-        if (g == 0) {
-            for (int c0 = 0; c0 < 128; c0 += 32) run(kAccA + c0, 32, kPW1 + c0 * kGHid + r, kGHid, true);
-            run(kAccA + 128, 16, kPW1 + 128 * kGHid + r, kGHid, true);
-            run(kAccA + kXones, 16, kPB1 + r, 0, true);
+    if (!issuer && r < kGHid) {
+        const int wg = 2 * grp + g;
+        const int o = min(r, kGOut - 1);
+        const bool keep = r < kGOut;
+        run(kAcc1 + 32 * wg, 32, kPW1 + 32 * wg * kGHid + r, kGHid, true);
+        if (wg == 0) {
+            run(kAcc1 + 128, 16, kPW1 + 128 * kGHid + r, kGHid, true);
+            run(kAcc2, 32, kPW2 + r, kGHid, true);
+        } else if (wg == 1) {
+            run(kAcc1 + kGEnc, 16, kPB1 + r, 0, true);
+            run(kAcc2 + 32, 32, kPW2 + 32 * kGHid + r, kGHid, true);
+        } else if (wg == 2) {
+            run(kAcc2 + kGHid, 16, kPB2 + r, 0, true);
+            run(kAcc3 + 16, 32, kPW3 + o, kGOut, keep);
         } else {
-            for (int c0 = 0; c0 < kGHid; c0 += 32) run(kAccB + kHh1 + c0, 32, kPW2 + c0 * kGHid + r, kGHid, true);
-            run(kAccB + kHones, 16, kPB2 + r, 0, true);
+            run(kAcc3, 16, kPB3 + o, 0, keep);
+            run(kAcc3 + 48, 32, kPW3 + 32 * kGOut + o, kGOut, keep);
         }
-    } else {           // lanes 64..103 of the second sums: output r - 64 (b3, dW3 half by half)
-        const int o = min(r - kGHid, kGOut - 1);
-        const bool keep = r - kGHid < kGOut;
-        if (g == 0) run(kAccB + kHones, 16, kPB3 + o, 0, keep);
-        run(kAccB + kHh2 + ch, 32, kPW3 + ch * kGOut + o, kGOut, keep);
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (S.fail) {
-        (void)tc::mbar_wait(&S.bar_w, 0, kTcWaitNs);
-        (void)tc::mbar_wait(&S.bar_mma, ph, kTcWaitNs);
-    }
-    if (tid < 32) {
+    if (issuer) {
+        if (S.fail) (void)tc::mbar_wait(&S.bar_w, 0, kTcWaitNs);   // the weight copy, after a failed wait
+        __syncwarp();
         tc::fence_after_sync();
         tc::tmem_dealloc(T, kTrCols);
     }

@@ -69,11 +69,40 @@ __device__ __forceinline__ void mma_f16(uint32_t taddr, uint64_t adesc, uint64_t
         :: "r"(taddr), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
+// The same by the lane of a converged warp whose `leader` is set: control
+// flow, descriptors and addresses stay the warp's, in uniform registers.
+__device__ __forceinline__ void mma_f16_by(bool leader, uint32_t taddr, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                           uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+        :: "r"(taddr), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"((uint32_t)leader) : "memory");
+}
+
 // The mbarrier arrives once all tcgen05 operations this thread issued
 // before have completed.
 __device__ __forceinline__ void commit(uint64_t* mbar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
                  :: "r"(smem_addr(mbar)) : "memory");
+}
+
+__device__ __forceinline__ void commit_by(bool leader, uint64_t* mbar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n"
+        :: "r"(smem_addr(mbar)), "r"((uint32_t)leader) : "memory");
+}
+// True in one lane of the (converged) warp, always the same one.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t is;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(is));
+    return is != 0;
 }
 
 __device__ __forceinline__ void fence_before_sync() {
@@ -90,6 +119,12 @@ __device__ __forceinline__ void fence_smem_to_async() {
 __device__ __forceinline__ void mbar_init(uint64_t* mbar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" :: "r"(smem_addr(mbar)), "r"(count) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+}
+
+// One arrival (release): what the warp wrote before a __syncwarp is visible
+// to whoever waits for the phase.
+__device__ __forceinline__ void mbar_arrive(uint64_t* mbar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" :: "r"(smem_addr(mbar)) : "memory");
 }
 
 __device__ __forceinline__ uint64_t globaltimer_ns() {

@@ -58,6 +58,27 @@ def test_gradient_matches_oracle(ctx, n):
         assert e < 1e-2, (name, e)
 
 
+@pytest.mark.parametrize("tiles, rest", [(1, 1), (2, 0), (152, 0), (152, 1), (304, 0), (304, 5), (456, 127)])
+def test_gradient_over_the_blocks_tiles(ctx, tiles, rest):
+    """Blocks with one tile (the second group idle), with two, and with the
+    first group one ahead; a last tile of few records.  `rest` records are
+    past the last whole tile.  The reference is the fp64 gradient at the
+    kernel's fp16 rounding points; the bound is that of
+    test_gradient_matches_oracle."""
+    n = 128 * tiles + rest
+    g = api.Guide(ctx)
+    p = random_params(17).astype(np.float32)
+    g.set_params(p)
+    rec = random_records(n, 18)
+    loss, grad = g.gradient(rec)
+    wl, wg = go.gradient(p.astype(np.float64), rec.astype(np.float32).astype(np.float64), fp16=True)
+    assert abs(loss - wl) <= 1e-3 * abs(wl), (loss, wl)
+    for name, a, b in [("W1", go.W1, go.B1), ("b1", go.B1, go.W2), ("W2", go.W2, go.B2), ("b2", go.B2, go.W3),
+                       ("W3", go.W3, go.B3), ("b3", go.B3, go.N_PARAMS)]:
+        e = rel(grad[a:b], wg[a:b])
+        assert e < 1e-2, (name, e)
+
+
 def test_adam_step_matches_oracle(ctx):
     g = api.Guide(ctx, learning_rate=1e-3)
     p = random_params(9).astype(np.float32)
