@@ -6,14 +6,16 @@
 //   loss = -(1/n) sum_i min((L_i / p_i) / mean(L / p), 20) * log q(w_i)
 // (an estimate of the KL divergence from the normalised incident radiance to
 // the mixture q, up to a constant), then one Adam update.  Kernels:
-//   k_guide_weight_sum   mean(L / p) over the batch
+//   k_guide_weight_sum   mean(L / p) over the batch (once for the steps of a
+//                        call, which take the same records)
 //   k_guide_train        forward, loss gradient, backward and the weight
 //                        and bias gradients per 128-record tile (tcgen05.mma),
 //                        activations kept in shared memory, gradient sums in
 //                        tensor memory; one partial gradient per block
-//   k_guide_grad_reduce  the blocks' partial gradients summed
-//   k_guide_adam         Adam on the fp32 master weights; refreshes the fp16
-//                        copy and the tensor cores' weight image
+//   k_guide_grad_reduce  the blocks' partial gradients summed; in a training
+//                        step also Adam on the fp32 master weights, which
+//                        refreshes the fp16 copy and the tensor cores' weight
+//                        image
 // Inference (k_guide_infer, and the guided material kernels in render.cu)
 // runs on tcgen05 too (guide_tc.cuh).
 #include <cuda_fp16.h>
@@ -385,9 +387,15 @@ __device__ __forceinline__ void tr_issue_grad(bool leader, uint32_t acc, uint32_
 // The block's products, step by step of each pair of tiles, the first
 // group's before the second's: one converged warp, one lane of which issues
 // them.  Returns false when a wait ran out.
-__device__ __forceinline__ bool tr_issue_all(GuideTrSmem& S, int ntiles) {
+__device__ __forceinline__ bool tr_issue_all(GuideTrSmem& S, const void* image, int ntiles) {
     constexpr int kSteps = 6;
     const bool leader = tc::elect_one();
+    // the weights, once the kernel before (an Adam step, perhaps) has written
+    // them: they land while the first tiles' records load and encode
+    tc::pdl_wait();
+    tc::fence_global_to_async();
+    if (leader) tc::bulk_load(S.w, image, kGImgTrainBytes, &S.bar_w);
+    __syncwarp();
     const uint32_t T = S.tmem, wa = tc::smem_addr(S.w);
     auto wait = [](uint64_t* bar, uint32_t ph) {
         return __any_sync(0xffffffffu, !tc::mbar_wait(bar, ph, kTcWaitNs)) == 0;
@@ -453,8 +461,6 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_guide_train(const void* image
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    // the weight copy lands while the first tiles' records load and encode
-    if (tid == kTrGroups * kTrGroup) tc::bulk_load(S.w, image, kGImgTrainBytes, &S.bar_w);
     const uint32_t T = S.tmem;
     const uint32_t lanes = (uint32_t)(tid & 96) << 16;              // this warp's accumulator lanes
     float lacc = 0.f;
@@ -469,7 +475,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_guide_train(const void* image
         return !failed;
     };
     if (issuer) {
-        failed = !tr_issue_all(S, ntiles);
+        failed = !tr_issue_all(S, image, ntiles);
     } else {
         __half* rec = S.rec[grp];
         const uint32_t tf = T + kAccF + grp * kGHid + lanes;        // the group's accumulator, this warp's lanes
@@ -508,9 +514,12 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_guide_train(const void* image
                 tr_store_input(h, rec, r, 3 * g + i);
             }
             ready();
-            tc::pdl_wait();   // k_guide_weight_sum has finished
-            if (gt < 32) {    // the batch's mean weight, summed the same way in every block
+        }
+        tc::pdl_wait();   // the kernels before have finished: the weights are summed, `partial` is free
+        if (tile < ntiles) {
+            if (gt < 32) {   // the batch's mean weight, summed the same way in every block
                 float sum = 0.f;
+#pragma unroll 8
                 for (int j = lane; j < nwsum; j += 32) sum += wsum[j];
                 for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
                 if (lane == 0) S.mean[grp] = sum / (float)n;
@@ -651,52 +660,90 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_guide_train(const void* image
     }
 }
 
-// grad[p] = (1/n) sum over the training blocks of their gradient sums (the
-// slot t that holds parameter p = guide_sum_param(t)).  A block takes 32
-// consecutive slots; its 8 warps split the blocks' sums and add theirs in
-// shared memory.  The padding outputs of layer 3 (rows 40..47) have no
-// slots and stay as they are.
+// Adam's state and this step's constants.
+struct AdamStep {
+    float* w32;              // fp32 master weights
+    __half* w16;
+    unsigned char* image;    // the tensor cores' weight image
+    float *m, *v;
+    float lr, b1, b2, c1, c2, eps;
+};
+
+// The padding of layer 3 (rows 40..47 and their biases): parameters without
+// a slot in the blocks' sums, kept zero.
+constexpr int kPPads = kGParams - kPSums;
+__host__ __device__ constexpr int guide_pad_param(int t) {
+    return t < (kGOutPad - kGOut) * kGHid ? kGW3 + kGOut * kGHid + t : kGB3 + kGOut + t - (kGOutPad - kGOut) * kGHid;
+}
+static_assert(guide_pad_param(0) == kGW3 + kGOut * kGHid && guide_pad_param(kPPads - 1) == kGParams - 1, "padding");
+
+// The gradient of parameter p = guide_sum_param(t): (1/n) times the sum over
+// the training blocks of their sums' slot t.  A block takes 32 consecutive
+// slots; its 8 warps split the blocks' sums and add theirs in shared memory.
+// kAdam: the warp that has the gradients updates their parameters (fp32
+// master, fp16 copy, weight image) and clears the batch's loss if `loss` is
+// given (for the next batch of a call).  Otherwise grad[p] is written.  The
+// padding parameters have no slots: Adam clears them.
+//
+// The sums (9.7 MB over 152 blocks, in the L2 cache) wait on latency, not on
+// bandwidth: a warp has all of its loads in flight (four at a time made a
+// training step of 131072 records 42.5 us long, twenty 39).  With the update
+// as a kernel of its own, and the records' weights summed anew for each step
+// of a call, a step took 43.4 us (18.6 instead of 12.4 with 1000 records).
 constexpr int kRedWarps = 8;
+constexpr int kRedLoads = 20;   // of a warp in flight: its share of 152 blocks' sums
+template <bool kAdam>
 __global__ void __launch_bounds__(32 * kRedWarps) k_guide_grad_reduce(const float* partial, int nblocks, float inv_n,
-                                                                        float* grad) {
+                                                                      float* grad, AdamStep A, float* loss) {
     __shared__ float s_sum[kRedWarps][32];
+    if (kAdam) tc::pdl_launch_dependents();
     tc::pdl_wait();   // k_guide_train has written every block's partials
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int t = blockIdx.x * 32 + lane;
+    const int p = t < kPSums ? guide_sum_param(t) : t < kPSums + kPPads ? guide_pad_param(t - kPSums) : -1;
+    float m = 0.f, v = 0.f, x = 0.f;   // Adam's state of the parameter, on its way meanwhile
+    if (kAdam && w == 0 && t < kPSums) {
+        m = A.m[p];
+        v = A.v[p];
+        x = A.w32[p];
+    }
     float acc = 0.f;
     if (t < kPSums) {
-#pragma unroll 4
-        for (int b = w; b < nblocks; b += kRedWarps) acc += partial[(size_t)b * kPSums + t];
+        for (int b0 = w; b0 < nblocks; b0 += kRedWarps * kRedLoads) {
+            float q[kRedLoads];
+#pragma unroll
+            for (int k = 0; k < kRedLoads; k++) {
+                const int b = b0 + k * kRedWarps;
+                q[k] = b < nblocks ? partial[(size_t)b * kPSums + t] : 0.f;
+            }
+#pragma unroll
+            for (int k = 0; k < kRedLoads; k++) acc += q[k];
+        }
     }
     s_sum[w][lane] = acc;
     __syncthreads();
-    if (w == 0 && t < kPSums) {
+    if (w != 0) return;
+    if (kAdam && loss && t == 0) *loss = 0.f;
+    if (t < kPSums) {
         float sum = 0.f;
 #pragma unroll
         for (int k = 0; k < kRedWarps; k++) sum += s_sum[k][lane];
-        grad[guide_sum_param(t)] = sum * inv_n;
-    }
-}
-
-// Adam on the fp32 master copy; refreshes the fp16 copy and clears the
-// gradient.  The padding rows of layer 3 stay zero.
-__global__ void k_guide_adam(float* w32, __half* w16, unsigned char* image, float* grad, float* m, float* v, float lr,
-                             float b1, float b2, float c1, float c2, float eps) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kGParams; i += gridDim.x * blockDim.x) {
-        const bool pad = (i >= kGW3 + kGOut * kGHid && i < kGB3) || i >= kGB3 + kGOut;
-        if (!pad) {
-            float g = grad[i];
-            float mi = b1 * m[i] + (1.f - b1) * g;
-            float vi = b2 * v[i] + (1.f - b2) * g * g;
-            m[i] = mi;
-            v[i] = vi;
-            w32[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+        const float g = sum * inv_n;
+        if (kAdam) {
+            // (the roundings are spelt out: Adam's quotient magnifies them)
+            m = fmaf(1.f - A.b1, g, __fmul_rn(A.b1, m));
+            v = fmaf(__fmul_rn(1.f - A.b2, g), g, __fmul_rn(A.b2, v));
+            x = __fsub_rn(x, __fmul_rn(A.lr, m / A.c1) / __fadd_rn(sqrtf(v / A.c2), A.eps));
+            A.m[p] = m;
+            A.v[p] = v;
         } else {
-            w32[i] = 0.f;
+            grad[p] = g;
         }
-        w16[i] = __float2half_rn(w32[i]);
-        write_image(image, i, w32[i]);
-        grad[i] = 0.f;
+    }
+    if (kAdam && p >= 0) {
+        A.w32[p] = x;   // (the padding: 0)
+        A.w16[p] = __float2half_rn(x);
+        write_image(A.image, p, x);
     }
 }
 
@@ -780,10 +827,14 @@ void guide_reserve(dl_guide* G, int64_t n) {
     G->wsum.ensure(kWsumMaxBlocks * sizeof(float));
 }
 
-// Gradient of the loss over `n` device records (every `stride`-th) written
-// to G->grad (entries outside the network's parameters untouched); the
-// loss sum lands in scratch[1].  guide_reserve(G, n) must have run.
-void guide_gradient(dl_guide* G, const void* d_recs, int64_t n, int stride, cudaStream_t st) {
+// The training kernels of one batch: `n` device records, every `stride`-th.
+// The loss sum lands in scratch[1].  `weigh`: sum the records' weights first
+// (a batch that repeats the last one on this stream skips it; its loss has
+// been cleared).  With `adam` the parameters are updated, else the gradient
+// goes to G->grad (entries outside the network's parameters untouched).
+// guide_reserve(G, n) must have run.
+static void launch_batch(dl_guide* G, const void* d_recs, int64_t n, int stride, cudaStream_t st, bool weigh,
+                         const AdamStep* adam, bool clear_loss) {
     static const bool setup = [] {
         DL_CUDA(cudaFuncSetAttribute(k_guide_train, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(GuideTrSmem)));
@@ -799,10 +850,10 @@ void guide_gradient(dl_guide* G, const void* d_recs, int64_t n, int stride, cuda
     const GuideRecord* R = static_cast<const GuideRecord*>(d_recs);
     const int nws = (int)std::min<int64_t>(kWsumMaxBlocks, (n + kWsumThreads - 1) / kWsumThreads);
     float* wsum = G->wsum.as<float>();
-    k_guide_weight_sum<<<nws, kWsumThreads, 0, st>>>(R, (int)n, stride, wsum, sc + 1);
-    // the next two kernels start their prologues while their predecessor
-    // runs (programmatic dependent launch); each waits for it before using
-    // what it wrote
+    if (weigh) k_guide_weight_sum<<<nws, kWsumThreads, 0, st>>>(R, (int)n, stride, wsum, sc + 1);
+    // each kernel starts its prologue while its predecessor runs
+    // (programmatic dependent launch) and waits for it before using what it
+    // wrote; the predecessors have waited for theirs
     float* part = G->partial.as<float>();
     float* grad = G->grad.as<float>();
     const void* img = G->image.ptr;
@@ -810,20 +861,41 @@ void guide_gradient(dl_guide* G, const void* d_recs, int64_t n, int stride, cuda
     const float inv_n = 1.f / (float)n;
     DL_CUDA(launch_dependent(k_guide_train, dim3(nb), dim3(kTrThreads), sizeof(GuideTrSmem), st, img, R, ni, stride,
                              (const float*)wsum, nws, part, sc + 1, err));
-    DL_CUDA(launch_dependent(k_guide_grad_reduce, dim3((kPSums + 31) / 32), dim3(32 * kRedWarps), 0, st,
-                             (const float*)part, nb, inv_n, grad));
+    if (adam)
+        DL_CUDA(launch_dependent(k_guide_grad_reduce<true>, dim3((kPSums + kPPads + 31) / 32), dim3(32 * kRedWarps), 0,
+                                 st, (const float*)part, nb, inv_n, (float*)nullptr, *adam,
+                                 clear_loss ? sc + 1 : (float*)nullptr));
+    else
+        DL_CUDA(launch_dependent(k_guide_grad_reduce<false>, dim3((kPSums + 31) / 32), dim3(32 * kRedWarps), 0, st,
+                                 (const float*)part, nb, inv_n, grad, AdamStep{}, (float*)nullptr));
     DL_CUDA(cudaGetLastError());
 }
 
-void guide_adam(dl_guide* G, cudaStream_t st) {
-    G->step += 1;
-    const float b1 = 0.9f, b2 = 0.999f;
-    const float c1 = 1.f - std::pow(b1, (float)G->step), c2 = 1.f - std::pow(b2, (float)G->step);
-    k_guide_adam<<<64, 256, 0, st>>>(G->w32.as<float>(), G->w16.as<__half>(), G->image.as<unsigned char>(),
-                                     G->grad.as<float>(),
-                                     G->m.as<float>(), G->v.as<float>(), G->cfg.learning_rate, b1, b2, c1, c2,
-                                     1e-8f);
-    DL_CUDA(cudaGetLastError());
+void guide_gradient(dl_guide* G, const void* d_recs, int64_t n, int stride, cudaStream_t st) {
+    launch_batch(G, d_recs, n, stride, st, true, nullptr, false);
+}
+
+static void guide_steps(dl_guide* G, const void* d_recs, int64_t n, int stride, int steps, cudaStream_t st) {
+    for (int k = 0; k < steps; k++) {
+        G->step += 1;
+        AdamStep A;
+        A.w32 = G->w32.as<float>();
+        A.w16 = G->w16.as<__half>();
+        A.image = G->image.as<unsigned char>();
+        A.m = G->m.as<float>();
+        A.v = G->v.as<float>();
+        A.lr = G->cfg.learning_rate;
+        A.b1 = 0.9f;
+        A.b2 = 0.999f;
+        A.c1 = 1.f - std::pow(A.b1, (float)G->step);
+        A.c2 = 1.f - std::pow(A.b2, (float)G->step);
+        A.eps = 1e-8f;
+        launch_batch(G, d_recs, n, stride, st, k == 0, &A, k + 1 < steps);
+    }
+}
+
+void guide_step(dl_guide* G, const void* d_recs, int64_t n, int stride, cudaStream_t st) {
+    guide_steps(G, d_recs, n, stride, 1, st);
 }
 
 // Train on `n` device records: `steps` Adam steps over the same batch.
@@ -831,10 +903,7 @@ float guide_train(dl_guide* G, const void* d_recs, int64_t n, int steps) {
     cudaStream_t st = G->ctx->stream;
     float loss = 0.f;
     guide_reserve(G, n);
-    for (int k = 0; k < steps; k++) {
-        guide_gradient(G, d_recs, n, 1, st);
-        guide_adam(G, st);
-    }
+    guide_steps(G, d_recs, n, 1, steps, st);
     if (steps > 0) {
         DL_CUDA(cudaMemcpyAsync(&loss, G->scratch.as<float>() + 1, 4, cudaMemcpyDeviceToHost, st));
         DL_CUDA(cudaStreamSynchronize(st));

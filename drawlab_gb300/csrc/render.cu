@@ -1403,9 +1403,7 @@ void render_guided(dl_scene* S, const dl_render_opts& o, dl_guide* G, float* d_f
             DL_CUDA(cudaEventRecord(G->t0, ts));
             for (int k = 0; k < steps; k++) {
                 const int64_t cnt = (nrec - k + steps - 1) / steps;
-                DL_CUDA(cudaMemsetAsync(G->grad.ptr, 0, kGuideParams * 4, ts));
-                guide_gradient(G, rec_half[half] + k, cnt, steps, ts);
-                guide_adam(G, ts);
+                guide_step(G, rec_half[half] + k, cnt, steps, ts);
             }
             DL_CUDA(cudaEventRecord(G->t1, ts));
             DL_CUDA(cudaEventRecord(G->train_done[half], ts));

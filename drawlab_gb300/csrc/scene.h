@@ -68,7 +68,7 @@ void guide_init_params(uint64_t seed, std::vector<float>& w);
 void guide_upload_params(dl_guide* G, const float* host);
 void guide_reserve(dl_guide* G, int64_t n);   // training buffers for batches of up to n records
 void guide_gradient(dl_guide* G, const void* d_recs, int64_t n, int stride, cudaStream_t st);
-void guide_adam(dl_guide* G, cudaStream_t st);
+void guide_step(dl_guide* G, const void* d_recs, int64_t n, int stride, cudaStream_t st);   // gradient and Adam
 float guide_train(dl_guide* G, const void* d_recs, int64_t n, int steps);
 void guide_forward(dl_guide* G, const float* d_in, float* d_out, int64_t n);
 // Guided progressive render into d_film (render.cu).

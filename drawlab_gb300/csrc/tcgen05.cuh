@@ -116,6 +116,11 @@ __device__ __forceinline__ void fence_smem_to_async() {
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
 }
 
+// What other kernels stored to global memory, before this thread's bulk copies read it.
+__device__ __forceinline__ void fence_global_to_async() {
+    asm volatile("fence.proxy.async.global;\n" ::: "memory");
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* mbar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" :: "r"(smem_addr(mbar)), "r"(count) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");

@@ -94,6 +94,24 @@ def test_adam_step_matches_oracle(ctx):
     assert np.all(got[go.W3 + 40 * 64:go.B3] == 0) and np.all(got[go.B3 + 40:] == 0)
 
 
+@pytest.mark.parametrize("n", [1, 200, 152 * 128 + 1, 50000])
+def test_steps_of_one_call_are_single_steps(ctx, n):
+    """Several steps in one call (the records' weights summed once, kernels
+    that begin while their predecessors run) and as many calls of one step
+    end with the same parameters, bit for bit, and the same last loss but
+    for the order of its sum over the warps (fp32)."""
+    rec = random_records(n, 21)
+    a, b = api.Guide(ctx, learning_rate=1e-3), api.Guide(ctx, learning_rate=1e-3)
+    p = random_params(22).astype(np.float32)
+    a.set_params(p)
+    b.set_params(p)
+    la = a.train(rec, steps=5)
+    for _ in range(5):
+        lb = b.train(rec, steps=1)
+    np.testing.assert_array_equal(a.params(), b.params())
+    assert abs(la - lb) <= 1e-4 * abs(lb), (la, lb)
+
+
 def target_records(n, rng):
     """Incident radiance proportional to a position-dependent vMF lobe:
     directions uniform on the sphere (pdf 1/4pi), L = the lobe's density."""
