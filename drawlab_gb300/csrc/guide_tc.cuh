@@ -217,17 +217,18 @@ __device__ __forceinline__ void encode_row_tc(const float* in6, __half* act, int
 }
 
 // One layer of warpgroup g: D (its tensor-memory columns) = act (128 x K)
-// W^T, W [N][K] in the image.
+// W^T, W [N][K] in the image.  The warpgroup's first warp, converged.
 template <int K, int N, class Sm>
 __device__ __forceinline__ void tc_issue_layer(Sm& S, int g, int w_off) {
     constexpr uint32_t idesc = tc::idesc_f16_f32(kTcRows, N);
-    const uint32_t a = tc::smem_addr(S.act[g]), b = tc::smem_addr(S.w + w_off);
+    const bool leader = tc::elect_one();
+    const uint64_t a = tc::smem_desc(tc::smem_addr(S.act[g]), 128, K * 16);
+    const uint64_t b = tc::smem_desc(tc::smem_addr(S.w + w_off), 128, K * 16);
     tc::fence_after_sync();
 #pragma unroll
     for (int ks = 0; ks < K / 16; ks++)
-        tc::mma_f16(S.tmem + 64u * g, tc::smem_desc(a + ks * 256, 128, K * 16), tc::smem_desc(b + ks * 256, 128, K * 16),
-                    idesc, ks > 0 ? 1u : 0u);
-    tc::commit(&S.bar_mma[g]);
+        tc::mma_f16_by(leader, S.tmem + 64u * g, a + ks * (256 / 16), b + ks * (256 / 16), idesc, ks > 0 ? 1u : 0u);
+    tc::commit_by(leader, &S.bar_mma[g]);
 }
 
 // The warp's 32 accumulator lanes in its warpgroup's columns.
@@ -250,8 +251,8 @@ __device__ __forceinline__ void tc_hidden_epilogue(Sm& S, int g, const float* bi
         uint32_t p[8];
 #pragma unroll
         for (int j = 0; j < 8; j++) {
-            __half2 h = __floats2half2_rn(fmaxf(v[2 * j] + bias[c0 + 2 * j], 0.f),
-                                          fmaxf(v[2 * j + 1] + bias[c0 + 2 * j + 1], 0.f));
+            __half2 h = __hmax2(__floats2half2_rn(v[2 * j] + bias[c0 + 2 * j], v[2 * j + 1] + bias[c0 + 2 * j + 1]),
+                                __float2half2_rn(0.f));
             p[j] = *reinterpret_cast<const uint32_t*>(&h);
         }
         *reinterpret_cast<uint4*>(act + canon_index(r, c0, kGHid)) = make_uint4(p[0], p[1], p[2], p[3]);
@@ -269,7 +270,7 @@ __device__ __forceinline__ void tc_hidden_epilogue(Sm& S, int g, const float* bi
 template <class Sm>
 __device__ __forceinline__ bool guide_tc_forward(Sm& S, int g, uint32_t& phase, unsigned* err) {
     bool failed = false;
-    const bool issuer = tc_row() == 0;
+    const bool issuer = tc_row() < 32;   // (a warp)
     auto wait = [&]() {
         if (!tc::mbar_wait(&S.bar_mma[g], phase, kTcWaitNs)) {
             failed = true;
