@@ -23,7 +23,17 @@
 //
 // Two shapes.  Few paths: 256 threads with up to 128 registers, no spills:
 // the shortest chain.  More: 448 threads at 72 registers, 28 warps an SM.
-// Measured (device ms, small | large shape | wavefront): Cornell 64x64 1 spp
+// Their slots are as many as leave the L1 cache 60 KB of the SM's 256 (two
+// blocks in 196 KB of shared memory) -- with 640 slots it had 28 KB, with 480
+// too few paths are in flight: Cornell 256x256 16 spp 1.24 | 1.29 (640) | 1.30
+// ms, textured box 333x251 16 spp 1.77 | 1.82 | 1.86, room 480x270 16 spp 4.03
+// | 4.08 | 4.21, 400k reference-sphere paths 2.46 | 2.73 | 2.40.  Up to 256
+// paths a block there is a small shape with 256 slots (L1 156 KB): 60k
+// reference-sphere paths 1.94 ms against 1.99, batch scene 256x256 1 spp 0.31
+// against 0.33; with more paths to take it is slower (Cornell 256x256 4 spp
+// 0.47 against 0.42).
+// Where the shapes cross, and the wavefront (device ms with 640 slots, small |
+// large shape | wavefront): Cornell 64x64 1 spp
 // 0.15 | 0.18 | 0.54; 256x256 1 spp 0.22 | 0.28 | 0.58; 4 spp 0.44 | 0.44 |
 // 0.71; 16 spp 1.41 | 1.28 | 1.39; sky 517x389 1 spp 0.41 | 0.45 | 0.94;
 // 16 spp 2.4 | 2.1 | 2.0; material spheres 1080p 1 spp 1.50 | 1.29 | 2.1;
@@ -35,7 +45,7 @@
 
 namespace dl {
 
-constexpr int kResStack = 6;                 // top traversal-stack entries of a thread in shared memory
+constexpr int kResStack = 4;                 // top traversal-stack entries of a thread in shared memory
 constexpr int kResMaxTurns = 1000000;        // queue chunks one warp takes
 constexpr int kResMaxSpins = 1 << 22;        // polls of one wait (each about 0.1 us)
 constexpr uint32_t kShadowTask = 0x8000u, kFreeEntry = 0x8000u, kNoEntry = 0xffffu;
@@ -553,13 +563,18 @@ static void launch_shape(int sms, const RenderParams& P, cudaStream_t st) {
 }
 
 void resident_launch(int sms, const RenderParams& P, bool multi, cudaStream_t st) {
-    // (the shapes cross between 0.2 and 0.4 M paths: see the top)
+    // (the shapes cross between 0.2 and 0.4 M paths, the slots at 256 a block: see the top)
     if (P.total <= kResidentFewPaths) {
-        if (multi) launch_shape<true, 256, 640, 2>(sms, P, st);
-        else launch_shape<false, 256, 640, 2>(sms, P, st);
+        if (P.total <= 2ull * sms * 256) {
+            if (multi) launch_shape<true, 256, 256, 2>(sms, P, st);
+            else launch_shape<false, 256, 256, 2>(sms, P, st);
+        } else {
+            if (multi) launch_shape<true, 256, 576, 2>(sms, P, st);
+            else launch_shape<false, 256, 576, 2>(sms, P, st);
+        }
     } else {
-        if (multi) launch_shape<true, 448, 640, 2>(sms, P, st);
-        else launch_shape<false, 448, 640, 2>(sms, P, st);
+        if (multi) launch_shape<true, 448, 608, 2>(sms, P, st);
+        else launch_shape<false, 448, 608, 2>(sms, P, st);
     }
 }
 
