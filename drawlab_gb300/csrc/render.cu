@@ -680,15 +680,30 @@ __global__ void __launch_bounds__(kGuided ? kTcThreads : kThreads, kGuided ? 2 :
 // Two tile sizes: 32 (four rows a thread) moves the fewest bytes and
 // instructions a pixel, 16 (one row a thread) has four times the blocks and a
 // shorter chain a sample, for frames whose tiles of 32 leave the chip idle.
+//
+// Bound by issue slots and the width of shared memory (57 % and 65 % of their
+// peaks at 1080p with tiles of 32).  A cell's geometry is the thread's, not
+// found again for every sample; weights are taken without bounds tests (those
+// of film pixels outside the tile are never read) and without integer
+// conversions; and what the sums read together is one vector.  That is 31 %
+// fewer instructions than a plane per value and a test per weight: film of 16
+// samples 1080p 0.73 -> 0.63 ms, 517x389 0.130 -> 0.085, 256x256 0.062 ->
+// 0.039 (launches alone).  Tiles of 32 at two blocks an SM: at three the 80
+// registers spill (1080p frame 3.93 ms against 3.87).
 constexpr int kFilmApron = 2, kFilmThreads = 256;
 constexpr int kFilmTaps = 2 * kFilmApron + 1;  // 5 film pixels per axis around a sample
 template <int kTile>
 struct FilmTile {
     static constexpr int kRegion = kTile + 2 * kFilmApron, kCells = kRegion * kRegion;
     static constexpr int kRows = kTile * kTile / kFilmThreads;                       // film pixels of a thread
-    static constexpr int kOwn = (kCells + kFilmThreads - 1) / kFilmThreads;          // staged cells of a thread
-    // staged per cell: r, g, b, 5 x weights, 5 y weights
-    static constexpr size_t kSmem = (size_t)(3 + 2 * kFilmTaps) * kCells * sizeof(float);
+    // staging: a thread's cells are in one region column, kStride rows apart
+    static constexpr int kStride = kFilmThreads / kRegion, kOwn = (kRegion + kStride - 1) / kStride;
+    // staged per cell: r, g, b, 5 y weights, 5 x weights
+    static constexpr size_t kSmem = (3 + 2 * kFilmTaps) * sizeof(float) * kCells;
+    // A cell's {r, g, b, y weight 4} is one vector; y weights 0..3 are two
+    // vectors where a thread with four rows takes several of them, else
+    // planes of words (a word of a vector costs the vector's bandwidth).
+    static constexpr bool kPairs = kRows > 1;
 };
 
 struct FilmParams {
@@ -705,16 +720,14 @@ struct FilmParams {
 };
 
 template <int kTile>
-__global__ void __launch_bounds__(kFilmThreads, kTile == 32 ? 3 : 4)
+__global__ void __launch_bounds__(kFilmThreads, kTile == 32 ? 2 : 4)
     k_film_gather(FilmParams F) {
     using Tile = FilmTile<kTile>;
     constexpr int kRows = Tile::kRows, kCells = Tile::kCells, kRegion = Tile::kRegion;
     extern __shared__ __align__(16) unsigned char dyn_smem[];
-    float* const s_r = reinterpret_cast<float*>(dyn_smem);
-    float* const s_g = s_r + kCells;
-    float* const s_b = s_g + kCells;
-    float* const s_wx = s_b + kCells;               // [kFilmTaps][kCells]
-    float* const s_wy = s_wx + kFilmTaps * kCells;  // [kFilmTaps][kCells]
+    float4* const s_v = reinterpret_cast<float4*>(dyn_smem);
+    float* const s_wy = reinterpret_cast<float*>(s_v + kCells);   // [4][kCells], or [2][kCells] pairs
+    float* const s_wx = s_wy + 4 * kCells;                        // [kFilmTaps][kCells]
     __shared__ float s_table[33];
     __shared__ unsigned int s_invalid;
     const int tx = threadIdx.x % kTile, ty = threadIdx.x / kTile;  // column, group of kRows rows
@@ -724,17 +737,29 @@ __global__ void __launch_bounds__(kFilmThreads, kTile == 32 ? 3 : 4)
     const size_t npix = (size_t)F.w * F.h;
     if (threadIdx.x < 33) s_table[threadIdx.x] = F.table[threadIdx.x];
     if (threadIdx.x == 0) s_invalid = 0;
-    // the thread's cells' samples of index k (w = 0 outside the image)
+    // the thread's cells: column rx of the region, rows ry0, ry0 + kStride, ...
+    const int rx = threadIdx.x % kRegion, ry0 = threadIdx.x / kRegion;
+    const int sx = IX0 + rx;
+    const bool stages = ry0 < Tile::kStride;
+    const bool inside = stages && sx >= 0 && sx < F.w;
+    const float fcol = (float)(X0 + rx);
+    // their samples of index k (w = 0 outside the image)
     float4 L[Tile::kOwn];
     auto load = [&](int k) {
 #pragma unroll
         for (int j = 0; j < Tile::kOwn; j++) {
-            const int e = threadIdx.x + j * kFilmThreads;
-            const int sx = IX0 + e % kRegion, sy = IY0 + e / kRegion;
+            const int ry = ry0 + j * Tile::kStride, sy = IY0 + ry;
             L[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (e < kCells && sx >= 0 && sx < F.w && sy >= 0 && sy < F.h)
+            if (inside && ry < kRegion && sy >= 0 && sy < F.h)
                 L[j] = F.samples[(size_t)k * npix + (size_t)sy * F.w + sx];
         }
+    };
+    // the filter's weight at distance |c - p|: entry min(int(distance x lookup),
+    // 32) of the table (the truncation by an addition that rounds towards
+    // zero: conversions run at a quarter of the rate); entry 32 is 0
+    auto weight = [&](float c, float p) {
+        const float v = fminf(__fmul_rn(fabsf(__fsub_rn(c, p)), F.lookup), 32.f);
+        return s_table[__float_as_int(__fadd_rz(v, 8388608.f)) - 0x4b000000];
     };
     load(0);
     __syncthreads();
@@ -744,17 +769,16 @@ __global__ void __launch_bounds__(kFilmThreads, kTile == 32 ? 3 : 4)
     for (int k = 0; k < F.nspp; k++) {
 #pragma unroll
         for (int j = 0; j < Tile::kOwn; j++) {
-            const int e = threadIdx.x + j * kFilmThreads;
-            if (e >= kCells) break;
-            const int rx = e % kRegion, ry = e / kRegion;
-            const int sx = IX0 + rx, sy = IY0 + ry;
+            const int ry = ry0 + j * Tile::kStride;
+            if (!stages || ry >= kRegion) break;
+            const int e = ry * kRegion + rx, sy = IY0 + ry;
             const bool ok = L[j].w != 0.f && L[j].x >= 0.f && L[j].y >= 0.f && L[j].z >= 0.f && isfinite(L[j].x) &&
                             isfinite(L[j].y) && isfinite(L[j].z);
             // each sample is counted by the tile that owns its pixel
             if (!ok && L[j].w != 0.f && rx >= kFilmApron && rx < kFilmApron + kTile && ry >= kFilmApron &&
                 ry < kFilmApron + kTile)
                 atomicAdd(&s_invalid, 1u);
-            float px = 0.f, py = 0.f;
+            float px = -1e6f, py = -1e6f;   // (weight 0 everywhere)
             if (ok) {
                 Pcg32 g;
                 seed_path(g, F.seed_mix, F.w, F.h, sx, sy, F.s_first + k);
@@ -763,20 +787,22 @@ __global__ void __launch_bounds__(kFilmThreads, kTile == 32 ? 3 : 4)
                 px = __fsub_rn(__fsub_rn(fx, 0.5f), (float)(-F.border));
                 py = __fsub_rn(__fsub_rn(fy, 0.5f), (float)(-F.border));
             }
-            s_r[e] = ok ? L[j].x : 0.f;
-            s_g[e] = ok ? L[j].y : 0.f;
-            s_b[e] = ok ? L[j].z : 0.f;
-            // weights of this sample for film columns X0 + rx - d and rows Y0 + ry - d
+            // weights of this sample for film columns X0 + rx - d and rows
+            // Y0 + ry - d (those outside the film or the tile are not used)
+            const float frow = (float)(Y0 + ry);
+            float wy[kFilmTaps];
 #pragma unroll
             for (int d = 0; d < kFilmTaps; d++) {
-                int cx = X0 + rx - d, cy = Y0 + ry - d;
-                float wx = 0.f, wy = 0.f;
-                if (ok && cx >= 0 && cx < F.cols)
-                    wx = s_table[min((int)__fmul_rn(fabsf(__fsub_rn((float)cx, px)), F.lookup), 32)];
-                if (ok && cy >= 0 && cy < F.rows)
-                    wy = s_table[min((int)__fmul_rn(fabsf(__fsub_rn((float)cy, py)), F.lookup), 32)];
-                s_wx[d * kCells + e] = wx;
-                s_wy[d * kCells + e] = wy;
+                s_wx[d * kCells + e] = weight(__fsub_rn(fcol, (float)d), px);
+                wy[d] = weight(__fsub_rn(frow, (float)d), py);
+            }
+            s_v[e] = make_float4(ok ? L[j].x : 0.f, ok ? L[j].y : 0.f, ok ? L[j].z : 0.f, wy[4]);
+            if (Tile::kPairs) {
+                reinterpret_cast<float2*>(s_wy)[e] = make_float2(wy[0], wy[1]);
+                reinterpret_cast<float2*>(s_wy)[kCells + e] = make_float2(wy[2], wy[3]);
+            } else {
+#pragma unroll
+                for (int d = 0; d < 4; d++) s_wy[d * kCells + e] = wy[d];
             }
         }
         __syncthreads();
@@ -785,20 +811,34 @@ __global__ void __launch_bounds__(kFilmThreads, kTile == 32 ? 3 : 4)
         // dy = r - j is a filter tap; per pixel the order is dy, then dx
 #pragma unroll
         for (int r = 0; r < kRows + kFilmTaps - 1; r++) {
+            const int lo = r < kRows ? 0 : r - kRows + 1, hi = r < kFilmTaps ? r : kFilmTaps - 1;  // taps in use
 #pragma unroll
             for (int dx = 0; dx < kFilmTaps; dx++) {
                 const int c = (kRows * ty + r) * kRegion + tx + dx;
                 const float wx = s_wx[dx * kCells + c];
-                const float R = __fmul_rn(s_r[c], wx), G = __fmul_rn(s_g[c], wx), B = __fmul_rn(s_b[c], wx);
+                const float4 v = s_v[c];
+                float wy[kFilmTaps];
+                wy[4] = v.w;
+                if (Tile::kPairs) {
+#pragma unroll
+                    for (int q = 0; q < 2; q++)
+                        if (lo <= 2 * q + 1 && hi >= 2 * q) {
+                            const float2 y = reinterpret_cast<const float2*>(s_wy)[q * kCells + c];
+                            wy[2 * q] = y.x;
+                            wy[2 * q + 1] = y.y;
+                        }
+                } else if (lo < 4) {
+                    wy[lo] = s_wy[lo * kCells + c];
+                }
+                const float R = __fmul_rn(v.x, wx), G = __fmul_rn(v.y, wx), B = __fmul_rn(v.z, wx);
 #pragma unroll
                 for (int j = 0; j < kRows; j++) {
                     const int dy = r - j;
                     if (dy < 0 || dy >= kFilmTaps) continue;
-                    const float wy = s_wy[dy * kCells + c];
-                    ar[j] = __fmaf_rn(R, wy, ar[j]);
-                    ag[j] = __fmaf_rn(G, wy, ag[j]);
-                    ab[j] = __fmaf_rn(B, wy, ab[j]);
-                    aw[j] = __fmaf_rn(wx, wy, aw[j]);
+                    ar[j] = __fmaf_rn(R, wy[dy], ar[j]);
+                    ag[j] = __fmaf_rn(G, wy[dy], ag[j]);
+                    ab[j] = __fmaf_rn(B, wy[dy], ab[j]);
+                    aw[j] = __fmaf_rn(wx, wy[dy], aw[j]);
                 }
             }
         }
@@ -828,14 +868,15 @@ static void launch_film(const FilmParams& F, cudaStream_t st) {
     DL_CUDA(cudaGetLastError());
 }
 
-// The gather of F's samples, on tiles of 32 when there is at least one per
-// SM.  Whole renders of an empty scene, device ms (tiles of 16 | of 32 | of
-// 32 before the prefetch): 64x64 64 spp 0.22 | 0.46 | 0.49; 256x256 16 spp
-// 0.14 | 0.19 | 0.27; 400x300 17 spp 0.22 | 0.22; 517x389 9 spp 0.19 | 0.17;
-// 1080p 64 spp 19.6 | 16.8 | 17.0.
+// The gather of F's samples, on tiles of 32 when there are three for every
+// four SMs: fewer leave the chip idle longer than the smaller tiles' wider
+// margins cost.  Whole renders of an empty scene, device ms (tiles of 16 | of
+// 32): 64x64 64 spp 0.134 | 0.255; 256x256 16 spp 0.097 | 0.119 (81 tiles of
+// 32 on 152 SMs); 360x270 16 spp 0.130 | 0.132 (108); 400x300 16 spp 0.156 |
+// 0.144 (130); 517x389 16 spp 0.53 | 0.51; 1280x720 16 spp 1.85 | 1.73.
 static void film_gather(const FilmParams& F, int sms, cudaStream_t st) {
     const int64_t tiles = (int64_t)((F.cols + 31) / 32) * ((F.rows + 31) / 32);
-    if (tiles >= sms) launch_film<32>(F, st);
+    if (4 * tiles >= 3 * (int64_t)sms) launch_film<32>(F, st);
     else launch_film<16>(F, st);
 }
 

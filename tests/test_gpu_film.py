@@ -41,9 +41,11 @@ def splat(L, pos, w, h, filt):
 
 
 # film sizes: one pixel; one tile of 16 and a column or row more; ragged small
-# frames; frames with at least one tile of 32 per SM, whole and ragged
+# frames; frames on both sides of three tiles of 32 for four of 152 SMs (112
+# and 114 tiles); frames with more of them, whole and ragged
 @pytest.mark.parametrize("filt", [abi.DL_FILTER_GAUSSIAN, abi.DL_FILTER_BOX])
-@pytest.mark.parametrize("w,h,spp", [(1, 1, 3), (12, 12, 2), (13, 12, 2), (16, 17, 2), (61, 35, 5), (508, 316, 1),
+@pytest.mark.parametrize("w,h,spp", [(1, 1, 3), (12, 12, 2), (13, 12, 2), (16, 17, 2), (61, 35, 5), (444, 252, 2), (604, 188, 2),
+                                     (508, 316, 1),
                                      (509, 320, 2), (640, 479, 1)])
 def test_film_equals_a_splat_of_its_samples(ctx, w, h, spp, filt):
     s = api.Scene.from_data(ctx, scenes.cornell(w, h))
