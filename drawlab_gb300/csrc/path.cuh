@@ -731,10 +731,10 @@ __device__ __forceinline__ bool scatter_vertex(const DevRequest& R, int type, in
 // Passes of at most kResidentMaxPaths paths run as one launch of the resident
 // kernel (resident.cu), the first kResidentFewPaths in its shape for few
 // paths.  At 2 M paths the wavefront catches up where paths are long and one
-// material prevails (device ms, resident | wavefront: Cornell 2.1 M 2.4 | 2.3,
-// textured Cornell 2.7 M 3.2 | 3.1, window-lit room 2.1 M 3.9 | 4.0), later
-// elsewhere (sky 3.2 M 2.1 | 2.0, MIS plates 3.7 M 2.6 | 2.7, material spheres
-// 33 M 16.5 | 15.3).
+// material prevails (device ms, resident | wavefront: Cornell 2.1 M 2.35 |
+// 2.3, textured Cornell 2.7 M 3.3 | 2.9, window-lit room 2.1 M 4.0 | 4.0, 4.2
+// M 7.8 | 6.1), later elsewhere (sky 3.2 M 2.2 | 2.0, MIS plates 3.7 M 2.7 |
+// 2.6, material spheres 4.1 M 2.4 | 2.9, 16.6 M 8.8 | 7.8).
 constexpr unsigned long long kResidentMaxPaths = 1ull << 21, kResidentFewPaths = 1ull << 18;
 constexpr unsigned kErrRounds = 8u;  // error-word bit: the resident kernel gave up (a wait or a warp's turns ran out)
 

@@ -23,11 +23,12 @@
 // and written whole: a full DRAM sector, no read-modify-write of partial
 // sectors.  Queues are compacted with warp ballots: one atomic per warp, or
 // per 32 entries where a warp stages them in shared memory; the hot counters
-// sit in separate 128-byte lines.  A
-// batch of iterations is captured once as a CUDA graph and replayed.  Every
-// path (x, y, s) owns a pcg32 stream and draws its numbers in the reference's
-// order (pixel 2D, aperture 2D, then per bounce NEE 2D, BSDF 2D, RR 1D), so
-// each path reproduces the oracle's path of the same (x, y, s).
+// sit in separate 128-byte lines.  A batch of iterations is captured as a CUDA
+// graph, replayed, and updated in place for other frames.  Passes of few paths
+// run in one launch instead (resident.cu).  Every path (x, y, s) owns a pcg32
+// stream and draws its numbers in the reference's order (pixel 2D, aperture
+// 2D, then per bounce NEE 2D, BSDF 2D, RR 1D), so each path reproduces the
+// oracle's path of the same (x, y, s).
 #include <cuda_runtime.h>
 
 #include <algorithm>
