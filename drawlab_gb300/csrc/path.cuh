@@ -735,7 +735,7 @@ __device__ __forceinline__ bool scatter_vertex(const DevRequest& R, int type, in
 // 2.3, textured Cornell 2.7 M 3.3 | 2.9, window-lit room 2.1 M 4.0 | 4.0, 4.2
 // M 7.8 | 6.1), later elsewhere (sky 3.2 M 2.2 | 2.0, MIS plates 3.7 M 2.7 |
 // 2.6, material spheres 4.1 M 2.4 | 2.9, 16.6 M 8.8 | 7.8).
-constexpr unsigned long long kResidentMaxPaths = 1ull << 21, kResidentFewPaths = 1ull << 18;
+constexpr unsigned long long kResidentMaxPaths = 1ull << 21, kResidentFewPaths = 7ull << 15;
 constexpr unsigned kErrRounds = 8u;  // error-word bit: the resident kernel gave up (a wait or a warp's turns ran out)
 
 // One pass of P.total paths as one launch on `st`; P.cnt reset before.

@@ -22,22 +22,25 @@
 // misses cost the sky scene 1.6x.
 //
 // Two shapes.  Few paths: 256 threads with up to 128 registers, no spills:
-// the shortest chain.  More: 448 threads at 72 registers, 28 warps an SM.
-// Their slots are as many as leave the L1 cache 60 KB of the SM's 256 (two
-// blocks in 196 KB of shared memory) -- with 640 slots it had 28 KB, with 480
-// too few paths are in flight: Cornell 256x256 16 spp 1.24 | 1.29 (640) | 1.30
-// ms, textured box 333x251 16 spp 1.77 | 1.82 | 1.86, room 480x270 16 spp 4.03
-// | 4.08 | 4.21, 400k reference-sphere paths 2.46 | 2.73 | 2.40.  Up to 256
+// the shortest chain.  More: 384 threads at 80 registers, 24 warps an SM (28
+// at 72 registers spilled twice as much: Cornell 256x256 16 spp 1.18 ms
+// against 1.22, sky 517x389 2 spp 0.53 | 0.55, 400k reference-sphere paths
+// 2.30 | 2.45; the batch scene 512x512 4 spp 1.25 | 1.23, the room 480x270 16
+// spp 4.00 | 3.98).  Their slots are as many as leave the L1 cache 60 KB of
+// the SM's 256 (two blocks in 196 KB of shared memory): with 640 slots it had
+// 28 KB, with 480 too few paths are in flight (Cornell 16 spp 1.24 | 1.29
+// (640) | 1.30 ms, textured box 333x251 16 spp 1.77 | 1.82 | 1.86).  Up to 256
 // paths a block there is a small shape with 256 slots (L1 156 KB): 60k
 // reference-sphere paths 1.94 ms against 1.99, batch scene 256x256 1 spp 0.31
 // against 0.33; with more paths to take it is slower (Cornell 256x256 4 spp
 // 0.47 against 0.42).
-// Where the shapes cross, and the wavefront (device ms with 640 slots, small |
-// large shape | wavefront): Cornell 64x64 1 spp
-// 0.15 | 0.18 | 0.54; 256x256 1 spp 0.22 | 0.28 | 0.58; 4 spp 0.44 | 0.44 |
-// 0.71; 16 spp 1.41 | 1.28 | 1.39; sky 517x389 1 spp 0.41 | 0.45 | 0.94;
-// 16 spp 2.4 | 2.1 | 2.0; material spheres 1080p 1 spp 1.50 | 1.29 | 2.1;
-// 64 spp (no shape) 66 | 58.
+// Where the shapes cross (device ms, small | large): Cornell 256x256 2 spp
+// 0.25 | 0.26, 3 spp 0.34 | 0.31, 4 spp 0.43 | 0.38; sky 517x389 1 spp 0.39 |
+// 0.41; textured box 2 spp 0.41 | 0.42, 3 spp 0.50 | 0.51; batch scene 3 spp
+// 0.48 | 0.47, 4 spp 0.55 | 0.53; room 2 spp 0.81 | 0.74.  Against the
+// wavefront: Cornell 64x64 1 spp 0.12 | 0.54 (wavefront), 256x256 1 spp 0.20 |
+// 0.58, 16 spp 1.18 | 1.39; sky 1 spp 0.39 | 0.94; material spheres 1080p 1
+// spp 1.31 | 2.1, 64 spp 66 | 58.
 #include <algorithm>
 
 #define DL_SHARED_FN __noinline__
@@ -575,7 +578,7 @@ static void launch_shape(int sms, const RenderParams& P, cudaStream_t st) {
 }
 
 void resident_launch(int sms, const RenderParams& P, bool multi, cudaStream_t st) {
-    // (the shapes cross between 0.2 and 0.4 M paths, the slots at 256 a block: see the top)
+    // (the shapes cross at about 0.2 M paths, the slots at 256 a block: see the top)
     if (P.total <= kResidentFewPaths) {
         if (P.total <= 2ull * sms * 256) {
             if (multi) launch_shape<true, 256, 256, 2>(sms, P, st);
@@ -585,8 +588,8 @@ void resident_launch(int sms, const RenderParams& P, bool multi, cudaStream_t st
             else launch_shape<false, 256, 576, 2>(sms, P, st);
         }
     } else {
-        if (multi) launch_shape<true, 448, 608, 2>(sms, P, st);
-        else launch_shape<false, 448, 608, 2>(sms, P, st);
+        if (multi) launch_shape<true, 384, 608, 2>(sms, P, st);
+        else launch_shape<false, 384, 608, 2>(sms, P, st);
     }
 }
 

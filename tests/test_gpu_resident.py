@@ -33,14 +33,16 @@ def make(name, w, h):
 
 
 # (paths: one; a warp and its neighbours; the edge between 256 and more slots
-# a block on 152 SMs, 77824; the edge between the kernel's two shapes, 2^18;
-# the largest pass, 2^21)
+# a block on 152 SMs, 77824; the edge between the kernel's two shapes, 229376;
+# larger passes; the largest, 2^21)
 @pytest.mark.parametrize("name,w,h,spp,depth,flags", [
     ("cornell", 1, 1, 1, 8, 0),
     ("cornell", 31, 1, 1, 0, 0),
     ("cornell", 33, 1, 1, 8, 0),
     ("textured", 304, 256, 1, 8, 0),
     ("textured", 305, 256, 1, 8, 0),
+    ("cornell", 448, 512, 1, 8, 0),
+    ("cornell", 449, 512, 1, 8, 0),
     ("cornell", 512, 512, 1, 8, 0),
     ("cornell", 513, 512, 1, 8, 0),
     ("cornell", 1024, 1024, 2, 4, 0),
