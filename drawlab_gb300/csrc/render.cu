@@ -195,7 +195,9 @@ __global__ void __launch_bounds__(128) k_traverse(RenderParams P, int p) {
                 }
             }
         }
-        if (__ballot_sync(0xffffffffu, has) == 0) break;
+        const unsigned with = __ballot_sync(0xffffffffu, has);
+        if (with == 0) break;
+        const int leave = __popc(with) > kDescendLanes ? kDescendLanes : 0;
         bool finished = false;
         int dest = 0;
         if (has) {
@@ -235,7 +237,7 @@ __global__ void __launch_bounds__(128) k_traverse(RenderParams P, int p) {
                 }
                 // the last lanes to descend would keep those that wait at a
                 // leaf idle: they go on next round
-                if (__popc(__activemask()) < kDescendLanes) break;
+                if (__popc(__activemask()) < leave) break;
             }
             finished = node == kDone;
             if (!finished && node < 0) {
