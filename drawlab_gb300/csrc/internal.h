@@ -113,6 +113,7 @@ struct RenderCounters {
     alignas(128) unsigned int work_sh;
     alignas(128) unsigned long long next_path;
     alignas(128) unsigned int guide_next;      // training records claimed (guided renders)
+    unsigned int tail_next;                    // paths the resident kernel has taken over from the wavefront
     // Values of the current pass, written by the host after the counters are
     // reset, so the captured graph stays valid across passes and frames.
     alignas(128) unsigned long long pass_total;  // paths of the pass

@@ -741,4 +741,18 @@ constexpr unsigned kErrRounds = 8u;  // error-word bit: the resident kernel gave
 // One pass of P.total paths as one launch on `st`; P.cnt reset before.
 void resident_launch(int sms, const RenderParams& P, bool multi, cudaStream_t st);
 
+// A wavefront pass whose paths have all been started is finished by the
+// resident kernel once at most kTailPaths are left (counted every graph
+// launch): long paths -- through glass, unbounded -- kept hundreds of almost
+// empty iterations of 50 us going.  Device ms with the wavefront to the end |
+// the rest at 2^14 | 2^17 | 2^20 paths: unbounded sky 1024x768 8 spp 18.4 |
+// 5.4 | 5.5 | 5.5, material spheres 800x600 8 spp 13.8 | 6.1 | 5.9 | 5.9,
+// reference spheres 640x480 16 spp 17.3 | 4.8 | 4.9 | 4.9, textured box
+// 1024x768 8 spp 5.7 | 5.6 | 5.1 | 5.1; depth 12, room 960x540 16 spp 10.9 |
+// 10.9 | 10.6 | 10.6.
+constexpr int kTailPaths = 1 << 17;
+// The `n` paths of extension queue 0 to their ends, as one launch on `st`;
+// their shadow rays have been traced.
+void resident_finish(int sms, const RenderParams& P, int n, bool multi, cudaStream_t st);
+
 }  // namespace dl

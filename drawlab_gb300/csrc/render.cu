@@ -1084,7 +1084,7 @@ static void check_render_error(unsigned int err) {
 // per-kernel times into kms.  `multi`: paths of a request table.
 static void run_wavefront(dl_context* ctx, RenderParams& P, int64_t cap, bool multi, bool count_traversal,
                           double* kms, int64_t& launches, int64_t& iters, RenderCounters& acc,
-                          unsigned long long total, int spp_offset, unsigned keep, void* recs = nullptr) {
+                          unsigned long long total, int spp_offset, unsigned keep, bool tail, void* recs = nullptr) {
     cudaStream_t st = ctx->stream;
     RenderBuffers& B = ctx->render;
     const TuneParams tp = ctx->tune;
@@ -1172,6 +1172,24 @@ static void run_wavefront(dl_context* ctx, RenderParams& P, int64_t cap, bool mu
         }
         check_render_error(hc->err);
         if (hc->ext[0] == 0 && hc->shadow[0] == 0 && hc->next_path >= total) break;
+        if (tail && hc->next_path >= total && hc->ext[0] <= kTailPaths) {
+            // few paths left: their shadow rays, then the rest in one launch
+            RenderParams R = P;
+            R.total = total;
+            const int blocks = sms * tp.trav_ctas_per_sm;
+            if (multi) k_traverse<false, true, true><<<blocks, 128, 0, st>>>(R, 0);
+            else k_traverse<false, true, false><<<blocks, 128, 0, st>>>(R, 0);
+            launches += 1;
+            if (hc->ext[0] > 0) {
+                resident_finish(sms, R, hc->ext[0], multi, st);
+                launches += 1;
+            }
+            DL_CUDA(cudaGetLastError());
+            DL_CUDA(cudaMemcpyAsync(hc, P.cnt, sizeof(RenderCounters), cudaMemcpyDeviceToHost, st));
+            DL_CUDA(cudaStreamSynchronize(st));
+            check_render_error(hc->err);
+            break;
+        }
         if (iters > 1000000) throw Error(DL_ERR_TIMEOUT, "render did not converge");
     }
     acc.stat_camera += std::min<unsigned long long>(hc->next_path, total);
@@ -1186,8 +1204,11 @@ static void run_wavefront(dl_context* ctx, RenderParams& P, int64_t cap, bool mu
 // A pass of `total` paths runs in the resident kernel: few paths, no pool
 // size asked for, and no need for the wavefront's separate kernels (their
 // times or traversal counts, or the tuning of their launch shape).
+static bool may_use_resident(const dl_context* ctx, int64_t pool, bool count_traversal) {
+    return pool == 0 && !count_traversal && !ctx->kernel_timing && !ctx->tuning;
+}
 static bool use_resident(const dl_context* ctx, int64_t pool, unsigned long long total, bool count_traversal) {
-    return total <= kResidentMaxPaths && pool == 0 && !count_traversal && !ctx->kernel_timing && !ctx->tuning;
+    return total <= kResidentMaxPaths && may_use_resident(ctx, pool, count_traversal);
 }
 
 // Budget of the per-path sample buffer; larger frames render in passes of
@@ -1308,13 +1329,14 @@ void render_run(dl_scene* S, const dl_render_opts& o, float* d_film, int64_t li_
     if (P.mode == 1) {
         if (!resident)
             run_wavefront(ctx, P, cap, false, count_traversal, kms, launches, iters, acc, (unsigned long long)li_n, 0,
-                          1u << 24);
+                          1u << 24, may_use_resident(ctx, o.max_paths_in_flight, count_traversal));
     } else {
         for (int s0 = 0; s0 < spp; s0 += chunk_spp) {
             int ns = std::min(chunk_spp, spp - s0);
             if (!resident)
                 run_wavefront(ctx, P, cap, false, count_traversal, kms, launches, iters, acc,
-                              npix * (unsigned long long)ns, o.spp_offset + s0, 1u << 24);
+                              npix * (unsigned long long)ns, o.spp_offset + s0, 1u << 24,
+                              may_use_resident(ctx, o.max_paths_in_flight, count_traversal));
             F.nspp = ns;
             F.s_first = o.spp_offset + s0;
             F.accumulate = s0 > 0;
@@ -1424,7 +1446,7 @@ void render_guided(dl_scene* S, const dl_render_opts& o, dl_guide* G, float* d_f
         // the half this pass writes must be free of the training that read it
         if (train && trained[half]) DL_CUDA(cudaStreamWaitEvent(st, G->train_done[half], 0));
         run_wavefront(ctx, P, cap, false, false, kms, launches, iters, acc, npix * (unsigned long long)ns,
-                      o.spp_offset + done, keep, rec_half[half]);
+                      o.spp_offset + done, keep, false, rec_half[half]);
         const int64_t claimed = train ? (int64_t)hc->guide_next : 0;
         const int64_t nrec = std::min<int64_t>(claimed, rec_cap);
         if (train && claimed > 0)
@@ -1541,7 +1563,8 @@ void render_batch(dl_context* ctx, const BatchItem* items, int n, bool count_tra
             resident_launch(ctx->num_sms > 0 ? ctx->num_sms : 152, P, true, st);
             launches = iters = 1;
         } else {
-            run_wavefront(ctx, P, cap, true, count_traversal, kms, launches, iters, acc, first, 0, 1u << 24);
+            run_wavefront(ctx, P, cap, true, count_traversal, kms, launches, iters, acc, first, 0, 1u << 24,
+                          may_use_resident(ctx, requested, count_traversal));
         }
         for (int a = 0; a < na; a++) {
             const int r = active[a];

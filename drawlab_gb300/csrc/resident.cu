@@ -432,10 +432,11 @@ __device__ __forceinline__ void resident_shade(const RenderParams& P, Sm& sm, in
 }
 
 // Misses (the envmap's radiance, the sample stored) and free slots: each
-// lane's slot starts the next path of the pass, 32 consecutive ones a warp.
-template <bool kMulti, class Sm>
+// lane's slot starts the next path of the pass, 32 consecutive ones a warp;
+// kTail: it takes the next of the `tail` paths that the wavefront left.
+template <bool kMulti, bool kTail, class Sm>
 __device__ __forceinline__ void resident_restart(const RenderParams& P, Sm& sm, uint32_t entry, bool active,
-                                                 uint32_t& err) {
+                                                 unsigned tail, uint32_t& err) {
     const int slot = (int)(entry & ~kFreeEntry);
     if (active && !(entry & kFreeEntry)) {
         PathState S;
@@ -449,9 +450,41 @@ __device__ __forceinline__ void resident_restart(const RenderParams& P, Sm& sm, 
         }
         resident_store<kMulti>(P, sm.pid[slot], S.L);
     }
-    const unsigned long long pid = warp_claim(&P.cnt->next_path, active);
-    const bool start = active && pid < P.total;
-    if (start) {
+    const unsigned long long pid = kTail ? warp_claim_u32(&P.cnt->tail_next, active) : warp_claim(&P.cnt->next_path, active);
+    bool start = active && pid < (kTail ? tail : P.total);
+    if (kTail && start) {
+        const int from = P.ext_q[0][pid];
+        if (slot_ok(P, from)) {
+            const RayRec r = P.rec[from].ray;
+            const MetaRec mr = P.rec[from].meta;
+            const PathRec pr = mr.m.y & PF_CAMERA ? camera_record() : P.rec[from].path;
+            sm.o[0][slot] = r.o.x;
+            sm.o[1][slot] = r.o.y;
+            sm.o[2][slot] = r.o.z;
+            sm.d[0][slot] = r.d.x;
+            sm.d[1][slot] = r.d.y;
+            sm.d[2][slot] = r.d.z;
+            sm.tmax[slot] = r.d.w;
+            sm.tp[0][slot] = pr.tp.x;
+            sm.tp[1][slot] = pr.tp.y;
+            sm.tp[2][slot] = pr.tp.z;
+            sm.eta[slot] = pr.tp.w;
+            sm.L[0][slot] = pr.L.x;
+            sm.L[1][slot] = pr.L.y;
+            sm.L[2][slot] = pr.L.z;
+            sm.pdf[slot] = pr.L.w;
+            sm.rng[0][slot] = mr.rng.x;
+            sm.rng[1][slot] = mr.rng.y;
+            sm.rng[2][slot] = mr.rng.z;
+            sm.rng[3][slot] = mr.rng.w;
+            sm.depth[slot] = mr.m.x;
+            sm.flags[slot] = mr.m.y;
+            sm.pid[slot] = (uint32_t)mr.m.z;
+            sm.pending[slot] = 1;
+        } else {
+            start = false;
+        }
+    } else if (start) {
         const int rid = kMulti ? find_request(P, pid) : 0;
         PathState S;
         float2 ps;
@@ -487,8 +520,8 @@ __device__ __forceinline__ void resident_restart(const RenderParams& P, Sm& sm, 
 }
 
 // `slots`: path slots each block uses (a multiple of 32, at most kSlots).
-template <bool kMulti, int kThreads, int kSlots, int kBlocks>
-__global__ void __launch_bounds__(kThreads, kBlocks) k_resident(RenderParams P, int slots) {
+template <bool kMulti, bool kTail, int kThreads, int kSlots, int kBlocks>
+__global__ void __launch_bounds__(kThreads, kBlocks) k_resident(RenderParams P, int slots, unsigned tail) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     auto& sm = *reinterpret_cast<ResidentSmem<kThreads, kSlots>*>(dyn_smem);
     const int lane = lane_id();
@@ -530,7 +563,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_resident(RenderParams P, 
             if (n > 0) {
                 const uint32_t e = lane < n ? ring_take(sm.queue[best], base + lane, &sm.abort, err) : kNoEntry;
                 const bool active = e != kNoEntry;
-                if (best == kEndedQueue) resident_restart<kMulti>(P, sm, e, active, err);
+                if (best == kEndedQueue) resident_restart<kMulti, kTail>(P, sm, e, active, tail, err);
                 else resident_shade<kMulti>(P, sm, best, active ? (int)e : 0, active, err);
                 idle = 0;
                 if (++turn == kResMaxTurns) st_shared(&sm.abort, 1);
@@ -556,10 +589,10 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_resident(RenderParams P, 
 }
 
 // One shape of the kernel, its blocks per SM found on first use.
-template <bool kMulti, int kThreads, int kSlots, int kBlocks>
-static void launch_shape(int sms, const RenderParams& P, cudaStream_t st) {
-    const unsigned long long total = P.total;
-    auto* fn = k_resident<kMulti, kThreads, kSlots, kBlocks>;
+// kTail: `total` paths that the wavefront left.
+template <bool kMulti, bool kTail, int kThreads, int kSlots, int kBlocks>
+static void launch_shape(int sms, const RenderParams& P, unsigned long long total, cudaStream_t st) {
+    auto* fn = k_resident<kMulti, kTail, kThreads, kSlots, kBlocks>;
     constexpr size_t smem = sizeof(ResidentSmem<kThreads, kSlots>);
     static_assert(kSlots % 32 == 0 && kSlots < (int)kFreeEntry && kBlocks * (smem + 1024) <= 228 * 1024, "shared memory");
     static const int per_sm = [=] {
@@ -573,7 +606,7 @@ static void launch_shape(int sms, const RenderParams& P, cudaStream_t st) {
     const int64_t share = (int64_t)((total + blocks - 1) / blocks);
     const int slots = (int)std::min<int64_t>(kSlots, (share + 31) / 32 * 32);
     const int grid = (int)std::min<int64_t>(blocks, (int64_t)((total + slots - 1) / slots));
-    fn<<<grid, kThreads, smem, st>>>(P, slots);
+    fn<<<grid, kThreads, smem, st>>>(P, slots, kTail ? (unsigned)total : 0u);
     DL_CUDA(cudaGetLastError());
 }
 
@@ -581,16 +614,21 @@ void resident_launch(int sms, const RenderParams& P, bool multi, cudaStream_t st
     // (the shapes cross at about 0.2 M paths, the slots at 256 a block: see the top)
     if (P.total <= kResidentFewPaths) {
         if (P.total <= 2ull * sms * 256) {
-            if (multi) launch_shape<true, 256, 256, 2>(sms, P, st);
-            else launch_shape<false, 256, 256, 2>(sms, P, st);
+            if (multi) launch_shape<true, false, 256, 256, 2>(sms, P, P.total, st);
+            else launch_shape<false, false, 256, 256, 2>(sms, P, P.total, st);
         } else {
-            if (multi) launch_shape<true, 256, 576, 2>(sms, P, st);
-            else launch_shape<false, 256, 576, 2>(sms, P, st);
+            if (multi) launch_shape<true, false, 256, 576, 2>(sms, P, P.total, st);
+            else launch_shape<false, false, 256, 576, 2>(sms, P, P.total, st);
         }
     } else {
-        if (multi) launch_shape<true, 384, 608, 2>(sms, P, st);
-        else launch_shape<false, 384, 608, 2>(sms, P, st);
+        if (multi) launch_shape<true, false, 384, 608, 2>(sms, P, P.total, st);
+        else launch_shape<false, false, 384, 608, 2>(sms, P, P.total, st);
     }
+}
+
+void resident_finish(int sms, const RenderParams& P, int n, bool multi, cudaStream_t st) {
+    if (multi) launch_shape<true, true, 256, 576, 2>(sms, P, (unsigned long long)n, st);
+    else launch_shape<false, true, 256, 576, 2>(sms, P, (unsigned long long)n, st);
 }
 
 }  // namespace dl

@@ -87,3 +87,39 @@ def test_resident_batch_equals_single_renders(ctx):
     for (s, o), img in zip(items, imgs):
         o.max_paths_in_flight = 8192
         assert np.array_equal(img, s.render(o))
+
+
+# more than 2^21 paths: the wavefront, whose last paths the resident kernel
+# takes over (unbounded and bounded depth, paths that all end in the first
+# graph launch); a pool size keeps the wavefront to the end
+@pytest.mark.parametrize("name,w,h,spp,depth", [
+    ("refspheres", 640, 480, 7, 0),
+    ("sky", 1024, 700, 3, 0),
+    ("textured", 801, 663, 5, 12),
+    ("spheres", 1201, 449, 4, 3),
+    ("empty", 1450, 1449, 1, 0),
+])
+def test_finished_wavefront_equals_wavefront(ctx, name, w, h, spp, depth):
+    s = api.Scene.from_data(ctx, make(name, w, h))
+    a = s.render_film(abi.make_opts(spp=spp, max_depth=depth, seed=6))
+    sa = ctx.stats()
+    b = s.render_film(abi.make_opts(spp=spp, max_depth=depth, seed=6, max_paths_in_flight=1 << 24))
+    sb = ctx.stats()
+    assert 1 < sa.iterations <= sb.iterations and (depth or name == "empty" or sa.iterations < sb.iterations)
+    assert np.array_equal(a, b)
+    assert (sa.camera_rays, sa.extension_rays, sa.shadow_rays) == (sb.camera_rays, sb.extension_rays, sb.shadow_rays)
+
+
+def test_finished_wavefront_paths_and_batch(ctx):
+    s = api.Scene.from_data(ctx, scenes.reference_spheres(96, 64))
+    n = (1 << 21) + 77
+    xys = np.random.default_rng(3).integers(0, (96, 64, 400), (n, 3)).astype(np.int32)
+    a = s.li(abi.make_opts(seed=9), xys)
+    b = s.li(abi.make_opts(seed=9, max_paths_in_flight=1 << 24), xys)
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+    made = [api.Scene.from_data(ctx, make(m, 700, 500)) for m in ("refspheres", "sky")]
+    items = [(m, abi.make_opts(spp=5, max_depth=0, seed=k)) for k, m in enumerate(made)]
+    imgs = ctx.render_batch(items)
+    for (m, o), img in zip(items, imgs):
+        o.max_paths_in_flight = 1 << 24
+        assert np.array_equal(img, m.render(o))
