@@ -742,8 +742,8 @@ constexpr unsigned kErrRounds = 8u;  // error-word bit: the resident kernel gave
 void resident_launch(int sms, const RenderParams& P, bool multi, cudaStream_t st);
 
 // A wavefront pass whose paths have all been started is finished by the
-// resident kernel once at most kTailPaths are left (counted every graph
-// launch): long paths -- through glass, unbounded -- kept hundreds of almost
+// resident kernel once at most kTailPaths are left (counted after every graph
+// launch, of 8 iterations in the figures): long paths -- through glass, unbounded -- kept hundreds of almost
 // empty iterations of 50 us going.  Device ms with the wavefront to the end |
 // the rest at 2^14 | 2^17 | 2^20 paths: unbounded sky 1024x768 8 spp 18.4 |
 // 5.4 | 5.5 | 5.5, material spheres 800x600 8 spp 13.8 | 6.1 | 5.9 | 5.9,

@@ -1088,7 +1088,13 @@ static void run_wavefront(dl_context* ctx, RenderParams& P, int64_t cap, bool mu
     cudaStream_t st = ctx->stream;
     RenderBuffers& B = ctx->render;
     const TuneParams tp = ctx->tune;
-    const int batch = tp.iters_per_graph;
+    // Where the resident kernel takes over the last paths, the host looks for
+    // them after every two iterations, unless the context's shape was set
+    // otherwise (device ms with 8 | 4 | 2: unbounded spheres 800x600 8 spp 6.0 |
+    // 5.0 | 5.0, sky 517x389 16 spp 1.78 | 1.56 | 1.57, textured box 640x500 16
+    // spp 4.38 | 4.38 | 4.28, spheres 1080p 4 spp 4.62 | 4.64 | 4.39, 64 spp
+    // 56.2 | 55.8 | 55.8; Cornell 512x512 16 spp 3.35 | 3.36 | 3.40).
+    const int batch = tail && tp.iters_per_graph == TuneParams().iters_per_graph ? 2 : tp.iters_per_graph;
     DL_CUDA(cudaMemsetAsync(P.cnt, 0, sizeof(RenderCounters), st));
     B.host_pass.ensure(sizeof(PassValues));
     PassValues* pv = B.host_pass.as<PassValues>();
@@ -1110,7 +1116,7 @@ static void run_wavefront(dl_context* ctx, RenderParams& P, int64_t cap, bool mu
         else launch_iteration<false>(P, k & 1, st, sms, tp, count, ev, ctx);
     };
     if (use_graph) {
-        std::vector<unsigned char> key(sizeof(P) + sizeof(int) + sizeof(cudaStream_t) + sizeof(TuneParams) + 1);
+        std::vector<unsigned char> key(sizeof(P) + sizeof(int) + sizeof(cudaStream_t) + sizeof(TuneParams) + 2);
         unsigned char* kp = key.data();
         std::memcpy(kp, &P, sizeof(P));
         kp += sizeof(P);
@@ -1120,7 +1126,8 @@ static void run_wavefront(dl_context* ctx, RenderParams& P, int64_t cap, bool mu
         kp += sizeof(cudaStream_t);
         std::memcpy(kp, &tp, sizeof(TuneParams));
         kp += sizeof(TuneParams);
-        *kp = multi ? 1 : 0;
+        *kp++ = multi ? 1 : 0;
+        *kp = (unsigned char)batch;
         if (!ctx->graph_exec || key != ctx->graph_key) {
             cudaGraph_t g = nullptr;
             DL_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
