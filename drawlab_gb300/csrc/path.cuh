@@ -730,12 +730,14 @@ __device__ __forceinline__ bool scatter_vertex(const DevRequest& R, int type, in
 
 // Passes of at most kResidentMaxPaths paths run as one launch of the resident
 // kernel (resident.cu), the first kResidentFewPaths in its shape for few
-// paths.  At 2 M paths the wavefront catches up where paths are long and one
-// material prevails (device ms, resident | wavefront: Cornell 2.1 M 2.35 |
-// 2.3, textured Cornell 2.7 M 3.3 | 2.9, window-lit room 2.1 M 4.0 | 4.0, 4.2
-// M 7.8 | 6.1), later elsewhere (sky 3.2 M 2.2 | 2.0, MIS plates 3.7 M 2.7 |
-// 2.6, material spheres 4.1 M 2.4 | 2.9, 16.6 M 8.8 | 7.8).
-constexpr unsigned long long kResidentMaxPaths = 1ull << 21, kResidentFewPaths = 7ull << 15;
+// paths.  Above, the wavefront's fuller kernels win on most scenes (device ms,
+// resident | wavefront, finished as below: Cornell 1.05 M 1.18 | 1.18, 1.57 M
+// 1.70 | 1.57, 2.0 M 2.15 | 1.89; sky 1.0 M 0.86 | 0.82, 1.6 M 1.20 | 1.07;
+// textured Cornell 1.0 M 1.37 | 1.42, 1.3 M 1.75 | 1.66, 2.0 M 2.50 | 2.14;
+// window-lit room 1.04 M 2.15 | 2.30, 1.56 M 3.10 | 2.86; MIS plates 0.9 M 0.75
+// | 0.90, 1.8 M 1.39 | 1.36), later on others (batch scene 1.6 M 1.77 | 1.99,
+// 2.0 M 2.20 | 2.32; material spheres 2.1 M 1.31 | 1.58).
+constexpr unsigned long long kResidentMaxPaths = 3ull << 19, kResidentFewPaths = 7ull << 15;
 constexpr unsigned kErrRounds = 8u;  // error-word bit: the resident kernel gave up (a wait or a warp's turns ran out)
 
 // One pass of P.total paths as one launch on `st`; P.cnt reset before.

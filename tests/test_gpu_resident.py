@@ -34,7 +34,7 @@ def make(name, w, h):
 
 # (paths: one; a warp and its neighbours; the edge between 256 and more slots
 # a block on 152 SMs, 77824; the edge between the kernel's two shapes, 229376;
-# larger passes; the largest, 2^21)
+# larger passes; the largest, 3 * 2^19)
 @pytest.mark.parametrize("name,w,h,spp,depth,flags", [
     ("cornell", 1, 1, 1, 8, 0),
     ("cornell", 31, 1, 1, 0, 0),
@@ -45,7 +45,7 @@ def make(name, w, h):
     ("cornell", 449, 512, 1, 8, 0),
     ("cornell", 512, 512, 1, 8, 0),
     ("cornell", 513, 512, 1, 8, 0),
-    ("cornell", 1024, 1024, 2, 4, 0),
+    ("cornell", 1024, 768, 2, 4, 0),
     ("sky", 97, 61, 7, 8, 0),
     ("sky", 300, 301, 5, 0, abi.DL_RENDER_POWER_LIGHT_PICK),
     ("textured", 83, 47, 9, 8, 0),
@@ -89,10 +89,11 @@ def test_resident_batch_equals_single_renders(ctx):
         assert np.array_equal(img, s.render(o))
 
 
-# more than 2^21 paths: the wavefront, whose last paths the resident kernel
+# more than 3 * 2^19 paths: the wavefront, whose last paths the resident kernel
 # takes over (unbounded and bounded depth, paths that all end in the first
 # graph launch); a pool size keeps the wavefront to the end
 @pytest.mark.parametrize("name,w,h,spp,depth", [
+    ("cornell", 1025, 768, 2, 4),
     ("refspheres", 640, 480, 7, 0),
     ("sky", 1024, 700, 3, 0),
     ("textured", 801, 663, 5, 12),
