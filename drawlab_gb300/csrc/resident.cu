@@ -572,7 +572,9 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_resident(RenderParams P, 
             // nothing to do: the pass has no more paths, or other warps hold
             // them.  A warp may leave: those that hold rays or paths go on by
             // themselves.
-            if (ld_shared(&sm.live) == 0 || ++idle > kResMaxSpins) break;
+            // The warp leaves as one: its lanes may read different counts, as
+            // other warps end paths meanwhile.
+            if (__any_sync(0xffffffffu, ld_shared(&sm.live) == 0 || ++idle > kResMaxSpins)) break;
             __nanosleep(100);
         }
         if (__any_sync(0xffffffffu, ld_shared(&sm.abort))) break;
