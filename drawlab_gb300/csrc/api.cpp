@@ -227,12 +227,13 @@ bool direct_out(const dl_context* ctx, const void* p, size_t align) {
 }
 // Before a kernel writes host array `p`: touches each of its pages.  A fresh
 // page costs 2.5 us here, 20 us when the device is the first to write it (and
-// a bad pointer fails on the host).
+// a bad pointer fails on the host).  The bytes stay as they are: the array may
+// overlap the rays, which are being read meanwhile.
 void touch_pages(void* p, size_t bytes) {
     static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-    volatile char* c = static_cast<char*>(p);
-    for (size_t i = 0; i < bytes; i += page) c[i] = 0;
-    c[bytes - 1] = 0;
+    unsigned char* c = static_cast<unsigned char*>(p);
+    for (size_t i = 0; i < bytes; i += page) (void)__atomic_fetch_or(&c[i], 0, __ATOMIC_RELAXED);
+    (void)__atomic_fetch_or(&c[bytes - 1], 0, __ATOMIC_RELAXED);
 }
 
 // `rays` where the traversal kernel reads them: in place, or copied.
@@ -286,10 +287,10 @@ int dl_trace_closest(dl_scene* S, const float* rays, int64_t n, int32_t* prim_id
         } else {
             float* s = B.split.as<float>();
             dl::split_hits_launch(ctx, B.hits.as<float>(), n, reinterpret_cast<int32_t*>(s), s + n, s + 2 * n, s + 3 * n);
-            DL_CUDA(cudaMemcpyAsync(prim_id, s, f, cudaMemcpyDeviceToHost, st));
             DL_CUDA(cudaMemcpyAsync(t, s + n, f, cudaMemcpyDeviceToHost, st));
             DL_CUDA(cudaMemcpyAsync(u, s + 2 * n, f, cudaMemcpyDeviceToHost, st));
             DL_CUDA(cudaMemcpyAsync(v, s + 3 * n, f, cudaMemcpyDeviceToHost, st));
+            DL_CUDA(cudaMemcpyAsync(prim_id, s, f, cudaMemcpyDeviceToHost, st));
         }
         finish_rays(ctx);
     });

@@ -168,14 +168,16 @@ __global__ void __launch_bounds__(kRayThreads) k_trace_rays(DevScene sc, const f
 
 // hits (n x float4) into the caller's four arrays: each warp writes 32
 // consecutive values of an array (split on the host, 200,003 hits took 420 us).
-__global__ void __launch_bounds__(256) k_split_hits(const float4* __restrict__ hits, int64_t n, int32_t* prim, float* t,
+// A caller that wants one of them may give one array for several: t, u, v and
+// prim (as bits, one type throughout) are stored in this order.
+__global__ void __launch_bounds__(256) k_split_hits(const float4* __restrict__ hits, int64_t n, float* prim, float* t,
                                                      float* u, float* v) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const float4 h = hits[i];
-        prim[i] = __float_as_int(h.w);
         t[i] = h.x;
         u[i] = h.y;
         v[i] = h.z;
+        prim[i] = h.w;
     }
 }
 
@@ -209,8 +211,8 @@ void trace_any_launch(dl_scene* S, const float* d_rays, int64_t n, uint8_t* d_oc
 
 void split_hits_launch(const dl_context* ctx, const float* d_hits, int64_t n, int32_t* prim, float* t, float* u,
                        float* v) {
-    k_split_hits<<<ray_grid(ctx, n, 256, 8), 256, 0, ctx->stream>>>(reinterpret_cast<const float4*>(d_hits), n, prim, t,
-                                                                   u, v);
+    k_split_hits<<<ray_grid(ctx, n, 256, 8), 256, 0, ctx->stream>>>(reinterpret_cast<const float4*>(d_hits), n,
+                                                                   reinterpret_cast<float*>(prim), t, u, v);
     DL_CUDA(cudaGetLastError());
 }
 void copy_bytes_launch(const dl_context* ctx, const uint8_t* from, int64_t n, uint8_t* to) {
