@@ -213,17 +213,22 @@ namespace {
 
 // Whether the kernels take host array `p` of `bytes` bytes as it is: the
 // device shares the host's page tables and the array has the alignment of the
-// kernels' accesses.  An input's ends are read here, so that a bad pointer
-// fails on the host as it does in a copy.
+// kernels' accesses.  Device memory is left to the copies: the host cannot
+// touch it.
+bool direct_out(const dl_context* ctx, const void* p, size_t align) {
+    if (!ctx->host_direct || reinterpret_cast<uintptr_t>(p) % align != 0) return false;
+    cudaPointerAttributes a;
+    DL_CUDA(cudaPointerGetAttributes(&a, p));
+    return a.type != cudaMemoryTypeDevice;
+}
+// An input's ends are read here, so that a bad pointer fails on the host as it
+// does in a copy.
 bool direct_in(const dl_context* ctx, const void* p, size_t bytes, size_t align) {
-    if (!ctx->host_direct || bytes == 0 || reinterpret_cast<uintptr_t>(p) % align != 0) return false;
+    if (bytes == 0 || !direct_out(ctx, p, align)) return false;
     const volatile char* c = static_cast<const char*>(p);
     (void)c[0];
     (void)c[bytes - 1];
     return true;
-}
-bool direct_out(const dl_context* ctx, const void* p, size_t align) {
-    return ctx->host_direct && reinterpret_cast<uintptr_t>(p) % align == 0;
 }
 // Before a kernel writes host array `p`: touches each of its pages.  A fresh
 // page costs 2.5 us here, 20 us when the device is the first to write it (and
@@ -241,7 +246,7 @@ const float* rays_on_device(dl_context* ctx, const float* rays, int64_t n) {
     const size_t bytes = (size_t)n * 32;
     if (direct_in(ctx, rays, bytes, 16)) return rays;
     ctx->trace.rays.ensure(bytes);
-    DL_CUDA(cudaMemcpyAsync(ctx->trace.rays.ptr, rays, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    DL_CUDA(cudaMemcpyAsync(ctx->trace.rays.ptr, rays, bytes, cudaMemcpyDefault, ctx->stream));
     return ctx->trace.rays.as<float>();
 }
 
@@ -287,10 +292,10 @@ int dl_trace_closest(dl_scene* S, const float* rays, int64_t n, int32_t* prim_id
         } else {
             float* s = B.split.as<float>();
             dl::split_hits_launch(ctx, B.hits.as<float>(), n, reinterpret_cast<int32_t*>(s), s + n, s + 2 * n, s + 3 * n);
-            DL_CUDA(cudaMemcpyAsync(t, s + n, f, cudaMemcpyDeviceToHost, st));
-            DL_CUDA(cudaMemcpyAsync(u, s + 2 * n, f, cudaMemcpyDeviceToHost, st));
-            DL_CUDA(cudaMemcpyAsync(v, s + 3 * n, f, cudaMemcpyDeviceToHost, st));
-            DL_CUDA(cudaMemcpyAsync(prim_id, s, f, cudaMemcpyDeviceToHost, st));
+            DL_CUDA(cudaMemcpyAsync(t, s + n, f, cudaMemcpyDefault, st));
+            DL_CUDA(cudaMemcpyAsync(u, s + 2 * n, f, cudaMemcpyDefault, st));
+            DL_CUDA(cudaMemcpyAsync(v, s + 3 * n, f, cudaMemcpyDefault, st));
+            DL_CUDA(cudaMemcpyAsync(prim_id, s, f, cudaMemcpyDefault, st));
         }
         finish_rays(ctx);
     });
@@ -312,7 +317,7 @@ int dl_trace_any(dl_scene* S, const float* rays, int64_t n, uint8_t* occluded) {
             touch_pages(occluded, (size_t)n);
             dl::copy_bytes_launch(ctx, B.hits.as<uint8_t>(), n, occluded);
         } else {
-            DL_CUDA(cudaMemcpyAsync(occluded, B.hits.ptr, (size_t)n, cudaMemcpyDeviceToHost, st));
+            DL_CUDA(cudaMemcpyAsync(occluded, B.hits.ptr, (size_t)n, cudaMemcpyDefault, st));
         }
         finish_rays(ctx);
     });
@@ -794,13 +799,13 @@ int dl_guide_forward(dl_guide* G, int64_t n, const float* inputs, float* outputs
         const bool in_place = direct_in(ctx, inputs, in_bytes, 4);
         if (!in_place) {
             G->io_in.ensure(in_bytes);
-            DL_CUDA(cudaMemcpyAsync(G->io_in.ptr, inputs, in_bytes, cudaMemcpyHostToDevice, ctx->stream));
+            DL_CUDA(cudaMemcpyAsync(G->io_in.ptr, inputs, in_bytes, cudaMemcpyDefault, ctx->stream));
         }
         G->io_out.ensure((size_t)n * 160);
         DL_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
         dl::guide_forward(G, in_place ? inputs : G->io_in.as<float>(), G->io_out.as<float>(), n);
         DL_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
-        DL_CUDA(cudaMemcpyAsync(outputs, G->io_out.ptr, (size_t)n * 160, cudaMemcpyDeviceToHost, ctx->stream));
+        DL_CUDA(cudaMemcpyAsync(outputs, G->io_out.ptr, (size_t)n * 160, cudaMemcpyDefault, ctx->stream));
         unsigned* err = ctx->words.as<unsigned>();
         DL_CUDA(cudaMemcpyAsync(err, G->scratch.as<char>() + dl::kGuideErrOffset, 4, cudaMemcpyDeviceToHost,
                                 ctx->stream));
