@@ -835,13 +835,12 @@ void guide_reserve(dl_guide* G, int64_t n) {
 // guide_reserve(G, n) must have run.
 static void launch_batch(dl_guide* G, const void* d_recs, int64_t n, int stride, cudaStream_t st, bool weigh,
                          const AdamStep* adam, bool clear_loss) {
-    static const bool setup = [] {
+    if (!G->ctx->train_ready) {
         DL_CUDA(cudaFuncSetAttribute(k_guide_train, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(GuideTrSmem)));
         DL_CUDA(cudaFuncSetAttribute(k_guide_train, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-        return true;
-    }();
-    (void)setup;
+        G->ctx->train_ready = true;
+    }
     const int nb = (int)train_blocks(G, n);
     if (n < 1 || G->partial.bytes < (size_t)nb * kPSums * 4 || G->wsum.bytes < kWsumMaxBlocks * sizeof(float))
         throw Error(DL_ERR_INVALID_ARG, "guide training buffers not reserved for this batch");
@@ -912,7 +911,7 @@ float guide_train(dl_guide* G, const void* d_recs, int64_t n, int steps) {
 }
 
 // Blocks of k_guide_infer resident at once on one SM, from its registers and
-// shared memory; the first call raises the kernel's shared-memory limit.
+// shared memory; a context's first call raises the kernel's shared-memory limit.
 static int infer_blocks_per_sm() {
     DL_CUDA(cudaFuncSetAttribute(k_guide_infer, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)sizeof(InferSmem)));
@@ -930,7 +929,8 @@ static int infer_blocks_per_sm() {
 }
 
 void guide_forward(dl_guide* G, const float* d_in, float* d_out, int64_t n) {
-    static const int per_sm = infer_blocks_per_sm();
+    int& per_sm = G->ctx->infer_per_sm;
+    if (per_sm == 0) per_sm = infer_blocks_per_sm();
     cudaStream_t st = G->ctx->stream;
     unsigned* err = reinterpret_cast<unsigned*>(G->scratch.as<char>() + kGuideErrOffset);
     DL_CUDA(cudaMemsetAsync(err, 0, sizeof(unsigned), st));

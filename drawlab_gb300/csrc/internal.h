@@ -170,6 +170,12 @@ struct dl_context {
     dl::RenderBuffers render;
     dl::TraceBuffers trace;
     int num_sms = 0;
+    // Blocks per SM of kernels that need more shared memory than 48 KB, found
+    // when the context first launches them: the raised limit belongs to a
+    // device, so nothing of this is kept for the process.
+    int resident_per_sm[8] = {0};   // the resident kernel's variants (resident.cu)
+    int guided_per_sm = 0, infer_per_sm = 0;
+    bool train_ready = false;
     // The device reads and writes pageable host memory through the host's page
     // tables (Grace): kernels take the caller's arrays as they are, without
     // copies (200,003 rays: 6.4 MB in 49 us by copy, 19 us read by the kernel).

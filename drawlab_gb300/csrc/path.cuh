@@ -741,7 +741,7 @@ constexpr unsigned long long kResidentMaxPaths = 3ull << 19, kResidentFewPaths =
 constexpr unsigned kErrRounds = 8u;  // error-word bit: the resident kernel gave up (a wait or a warp's turns ran out)
 
 // One pass of P.total paths as one launch on `st`; P.cnt reset before.
-void resident_launch(int sms, const RenderParams& P, bool multi, cudaStream_t st);
+void resident_launch(dl_context* ctx, const RenderParams& P, bool multi, cudaStream_t st);
 
 // A wavefront pass whose paths have all been started is finished by the
 // resident kernel once at most kTailPaths are left (counted after every graph
@@ -755,6 +755,6 @@ void resident_launch(int sms, const RenderParams& P, bool multi, cudaStream_t st
 constexpr int kTailPaths = 1 << 17;
 // The `n` paths of extension queue 0 to their ends, as one launch on `st`;
 // their shadow rays have been traced.
-void resident_finish(int sms, const RenderParams& P, int n, bool multi, cudaStream_t st);
+void resident_finish(dl_context* ctx, const RenderParams& P, int n, bool multi, cudaStream_t st);
 
 }  // namespace dl

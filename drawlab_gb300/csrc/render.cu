@@ -1188,7 +1188,7 @@ static void run_wavefront(dl_context* ctx, RenderParams& P, int64_t cap, bool mu
             else k_traverse<false, true, false><<<blocks, 128, 0, st>>>(R, 0);
             launches += 1;
             if (hc->ext[0] > 0) {
-                resident_finish(sms, R, hc->ext[0], multi, st);
+                resident_finish(ctx, R, hc->ext[0], multi, st);
                 launches += 1;
             }
             DL_CUDA(cudaGetLastError());
@@ -1330,7 +1330,7 @@ void render_run(dl_scene* S, const dl_render_opts& o, float* d_film, int64_t li_
     if (resident) {   // (a whole render: its samples fit the buffer)
         P.total = chunk_total;
         DL_CUDA(cudaMemsetAsync(P.cnt, 0, sizeof(RenderCounters), st));
-        resident_launch(ctx->num_sms > 0 ? ctx->num_sms : 152, P, false, st);
+        resident_launch(ctx, P, false, st);
         launches = iters = 1;
     }
     if (P.mode == 1) {
@@ -1364,8 +1364,8 @@ void render_run(dl_scene* S, const dl_render_opts& o, float* d_film, int64_t li_
 // estimate whichever network drew it.
 // Blocks of a guided material launch: as many as are resident at once (each
 // loads the weights once and walks tiles), from the SM's registers and
-// shared memory.  The first call raises the kernels' dynamic shared-memory
-// limit (before any graph capture).
+// shared memory.  A context's first call raises the kernels' dynamic
+// shared-memory limit (before any graph capture).
 template <int T>
 static int guided_resident_blocks() {
     auto* fn = k_material<T, false, true, kTcThreads>;
@@ -1383,11 +1383,12 @@ static int guided_resident_blocks() {
     const int by_smem = (int)(prop.sharedMemPerMultiprocessor / smem);
     return std::max(1, std::min(by_regs, by_smem));
 }
-static int guided_blocks(int sms) {
-    static const int per_sm = std::min(std::min(guided_resident_blocks<MAT_DIFFUSE>(),
-                                                guided_resident_blocks<MAT_MICROFACET>()),
-                                       guided_resident_blocks<MAT_ANISO_GGX>());
-    return sms * per_sm;
+static int guided_blocks(dl_context* ctx) {
+    if (ctx->guided_per_sm == 0)
+        ctx->guided_per_sm = std::min(std::min(guided_resident_blocks<MAT_DIFFUSE>(),
+                                               guided_resident_blocks<MAT_MICROFACET>()),
+                                      guided_resident_blocks<MAT_ANISO_GGX>());
+    return ctx->num_sms * ctx->guided_per_sm;
 }
 
 void render_guided(dl_scene* S, const dl_render_opts& o, dl_guide* G, float* d_film, bool train) {
@@ -1410,7 +1411,7 @@ void render_guided(dl_scene* S, const dl_render_opts& o, dl_guide* G, float* d_f
     P.samples = B.samples.as<float4>();
     P.guided = 1;
     P.gnet.image = G->image.ptr;
-    P.gnet.blocks = guided_blocks(ctx->num_sms);
+    P.gnet.blocks = guided_blocks(ctx);
     P.gnet.fraction = G->cfg.guide_fraction;
     P.gnet.max_depth = G->cfg.max_guided_depth;
     P.grec = B.grec.as<GuideRec>();
@@ -1567,7 +1568,7 @@ void render_batch(dl_context* ctx, const BatchItem* items, int n, bool count_tra
         if (resident) {   // (one pass: every request's samples fit the buffer)
             P.total = first;
             DL_CUDA(cudaMemsetAsync(P.cnt, 0, sizeof(RenderCounters), st));
-            resident_launch(ctx->num_sms > 0 ? ctx->num_sms : 152, P, true, st);
+            resident_launch(ctx, P, true, st);
             launches = iters = 1;
         } else {
             run_wavefront(ctx, P, cap, true, count_traversal, kms, launches, iters, acc, first, 0, 1u << 24,

@@ -590,20 +590,24 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_resident(RenderParams P, 
     if (err) atomicOr(&P.cnt->err, err);
 }
 
-// One shape of the kernel, its blocks per SM found on first use.
-// kTail: `total` paths that the wavefront left.
+static int resident_sms(const dl_context* ctx) { return ctx->num_sms > 0 ? ctx->num_sms : 152; }
+
+// One shape of the kernel (`index`: 0 .. 3), its blocks per SM found when the
+// context first launches it.  kTail: `total` paths that the wavefront left.
 template <bool kMulti, bool kTail, int kThreads, int kSlots, int kBlocks>
-static void launch_shape(int sms, const RenderParams& P, unsigned long long total, cudaStream_t st) {
+static void launch_shape(dl_context* ctx, int index, const RenderParams& P, unsigned long long total,
+                         cudaStream_t st) {
     auto* fn = k_resident<kMulti, kTail, kThreads, kSlots, kBlocks>;
     constexpr size_t smem = sizeof(ResidentSmem<kThreads, kSlots>);
     static_assert(kSlots % 32 == 0 && kSlots < (int)kFreeEntry && kBlocks * (smem + 1024) <= 228 * 1024, "shared memory");
-    static const int per_sm = [=] {
+    int& per_sm = ctx->resident_per_sm[2 * index + (kMulti ? 1 : 0)];
+    if (per_sm == 0) {
         DL_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int n = 0;
         DL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kThreads, smem));
-        return std::max(1, n);
-    }();
-    const int64_t blocks = (int64_t)sms * per_sm;
+        per_sm = std::max(1, n);
+    }
+    const int64_t blocks = (int64_t)resident_sms(ctx) * per_sm;
     // few paths: spread over all blocks, whole warps of them
     const int64_t share = (int64_t)((total + blocks - 1) / blocks);
     const int slots = (int)std::min<int64_t>(kSlots, (share + 31) / 32 * 32);
@@ -612,25 +616,25 @@ static void launch_shape(int sms, const RenderParams& P, unsigned long long tota
     DL_CUDA(cudaGetLastError());
 }
 
-void resident_launch(int sms, const RenderParams& P, bool multi, cudaStream_t st) {
+void resident_launch(dl_context* ctx, const RenderParams& P, bool multi, cudaStream_t st) {
     // (the shapes cross at about 0.2 M paths, the slots at 256 a block: see the top)
     if (P.total <= kResidentFewPaths) {
-        if (P.total <= 2ull * sms * 256) {
-            if (multi) launch_shape<true, false, 256, 256, 2>(sms, P, P.total, st);
-            else launch_shape<false, false, 256, 256, 2>(sms, P, P.total, st);
+        if (P.total <= 2ull * resident_sms(ctx) * 256) {
+            if (multi) launch_shape<true, false, 256, 256, 2>(ctx, 0, P, P.total, st);
+            else launch_shape<false, false, 256, 256, 2>(ctx, 0, P, P.total, st);
         } else {
-            if (multi) launch_shape<true, false, 256, 576, 2>(sms, P, P.total, st);
-            else launch_shape<false, false, 256, 576, 2>(sms, P, P.total, st);
+            if (multi) launch_shape<true, false, 256, 576, 2>(ctx, 1, P, P.total, st);
+            else launch_shape<false, false, 256, 576, 2>(ctx, 1, P, P.total, st);
         }
     } else {
-        if (multi) launch_shape<true, false, 384, 608, 2>(sms, P, P.total, st);
-        else launch_shape<false, false, 384, 608, 2>(sms, P, P.total, st);
+        if (multi) launch_shape<true, false, 384, 608, 2>(ctx, 2, P, P.total, st);
+        else launch_shape<false, false, 384, 608, 2>(ctx, 2, P, P.total, st);
     }
 }
 
-void resident_finish(int sms, const RenderParams& P, int n, bool multi, cudaStream_t st) {
-    if (multi) launch_shape<true, true, 256, 576, 2>(sms, P, (unsigned long long)n, st);
-    else launch_shape<false, true, 256, 576, 2>(sms, P, (unsigned long long)n, st);
+void resident_finish(dl_context* ctx, const RenderParams& P, int n, bool multi, cudaStream_t st) {
+    if (multi) launch_shape<true, true, 256, 576, 2>(ctx, 3, P, (unsigned long long)n, st);
+    else launch_shape<false, true, 256, 576, 2>(ctx, 3, P, (unsigned long long)n, st);
 }
 
 }  // namespace dl
