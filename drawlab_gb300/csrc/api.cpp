@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <new>
 #include <string>
 
@@ -45,6 +46,15 @@ void need(bool ok, const char* what) {
 void need(bool ok, const std::string& what) {
     if (!ok) throw dl::Error(DL_ERR_INVALID_ARG, what);
 }
+
+// Around kernels and copies on the caller's arrays, several to a call: a call
+// that fails half way waits for them, as the caller may free the arrays then.
+struct WaitOnError {
+    dl_context* ctx;
+    ~WaitOnError() {
+        if (std::uncaught_exceptions() > 0) cudaStreamSynchronize(ctx->stream);
+    }
+};
 
 void check_opts(const dl_render_opts* o) {
     need(o != nullptr, "opts is NULL");
@@ -284,6 +294,7 @@ int dl_trace_closest(dl_scene* S, const float* rays, int64_t n, int32_t* prim_id
         const bool direct = direct_out(ctx, prim_id, 4) && direct_out(ctx, t, 4) && direct_out(ctx, u, 4) &&
                             direct_out(ctx, v, 4);
         if (!direct) B.split.ensure(4 * f);
+        WaitOnError wait{ctx};
         DL_CUDA(cudaEventRecord(ctx->ev0, st));
         dl::trace_closest_launch(S, rays_on_device(ctx, rays, n), n, B.hits.as<float>(), B.occ.ptr);
         if (direct) {
@@ -311,6 +322,7 @@ int dl_trace_any(dl_scene* S, const float* rays, int64_t n, uint8_t* occluded) {
         dl::TraceBuffers& B = ctx->trace;
         B.hits.ensure((size_t)n);
         B.occ.ensure(64);
+        WaitOnError wait{ctx};
         DL_CUDA(cudaEventRecord(ctx->ev0, st));
         dl::trace_any_launch(S, rays_on_device(ctx, rays, n), n, B.hits.as<uint8_t>(), B.occ.ptr);
         if (direct_out(ctx, occluded, 1)) {
@@ -580,6 +592,7 @@ int dl_render_batch(dl_context* ctx, const dl_request* reqs, int32_t n) {
         for (int32_t r = 0; r < n; r++)
             if (reqs[r].rgb) maxrgb = std::max(maxrgb, (size_t)items[r].cam.w * items[r].cam.h * 3);
         ctx->render.rgb.ensure(std::max<size_t>(maxrgb, 1) * 4);
+        WaitOnError wait{ctx};
         dl::render_batch(ctx, items.data(), n, false, [&] {
             for (int32_t r = 0; r < n; r++) {  // (one after another on the stream)
                 if (!reqs[r].rgb) continue;
@@ -802,6 +815,7 @@ int dl_guide_forward(dl_guide* G, int64_t n, const float* inputs, float* outputs
             DL_CUDA(cudaMemcpyAsync(G->io_in.ptr, inputs, in_bytes, cudaMemcpyDefault, ctx->stream));
         }
         G->io_out.ensure((size_t)n * 160);
+        WaitOnError wait{ctx};
         DL_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
         dl::guide_forward(G, in_place ? inputs : G->io_in.as<float>(), G->io_out.as<float>(), n);
         DL_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));

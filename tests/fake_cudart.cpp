@@ -22,6 +22,7 @@ cudaError_t last = cudaSuccess;
 std::map<const void*, std::string> names;
 std::map<const void*, int> limit[kDevices];
 std::string log_text, fail_name;
+int fail_skip = 0;   // launches of that name that still go through
 dl::RenderCounters* counters = nullptr;   // of the pass in progress
 unsigned long long total = 0;
 struct Config {
@@ -38,7 +39,7 @@ cudaError_t launch(const void* fn, size_t smem) {
     std::lock_guard<std::recursive_mutex> lk(mu);
     const std::string name = names.count(fn) ? names[fn] : "?";
     const int max = limit[device].count(fn) ? limit[device][fn] : 48 * 1024;
-    const bool wanted = !fail_name.empty() && name.find(fail_name) != std::string::npos;
+    const bool wanted = !fail_name.empty() && name.find(fail_name) != std::string::npos && fail_skip-- <= 0;
     const bool ok = (int)smem <= max && !wanted;
     note((ok ? "launch " : "refused ") + std::to_string(device) + " " + name);
     if (!ok) return fail(wanted ? cudaErrorLaunchOutOfResources : cudaErrorInvalidValue);
@@ -55,7 +56,10 @@ extern "C" {
 // ---- the test's side
 const char* fake_log() { return log_text.c_str(); }
 void fake_clear_log() { log_text.clear(); }
-void fake_fail_kernel(const char* part_of_name) { fail_name = part_of_name; }
+void fake_fail_kernel(const char* part_of_name, int skip) {
+    fail_name = part_of_name;
+    fail_skip = skip;
+}
 
 // ---- what compiled CUDA code calls by itself
 void** __cudaRegisterFatBinary(void*) {
@@ -139,6 +143,7 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
 cudaError_t cudaGetSymbolAddress(void** p, const void* s) { return *p = const_cast<void*>(s), cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void* to, const void* from, size_t n, cudaMemcpyKind, cudaStream_t) {
     std::memcpy(to, from, n);
+    note("copy");
     if (n == 24) {   // a wavefront pass's values, among its counters
         counters = reinterpret_cast<dl::RenderCounters*>(static_cast<char*>(to) - offsetof(dl::RenderCounters, pass_total));
         std::memcpy(&total, from, sizeof(total));

@@ -15,7 +15,7 @@ from drawlab_gb300 import abi, api, scenes
 api.lib()
 fake = C.CDLL("libcudart.so.13")
 fake.fake_log.restype = C.c_char_p
-fake.fake_fail_kernel.argtypes = [C.c_char_p]
+fake.fake_fail_kernel.argtypes = [C.c_char_p, C.c_int]
 log = lambda: fake.fake_log().decode().split("\\n")[:-1]
 """ % REPO
 
