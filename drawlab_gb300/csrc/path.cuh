@@ -738,7 +738,7 @@ __device__ __forceinline__ bool scatter_vertex(const DevRequest& R, int type, in
 // | 0.90, 1.8 M 1.39 | 1.36), later on others (batch scene 1.6 M 1.77 | 1.99,
 // 2.0 M 2.20 | 2.32; material spheres 2.1 M 1.31 | 1.58).
 constexpr unsigned long long kResidentMaxPaths = 3ull << 19, kResidentFewPaths = 7ull << 15;
-constexpr unsigned kErrRounds = 8u;  // error-word bit: the resident kernel gave up (a wait or a warp's turns ran out)
+constexpr unsigned kErrRounds = 8u;  // error-word bit: the resident kernel gave up (a wait or a path's vertices ran out)
 
 // One pass of P.total paths as one launch on `st`; P.cnt reset before.
 void resident_launch(dl_context* ctx, const RenderParams& P, bool multi, cudaStream_t st);

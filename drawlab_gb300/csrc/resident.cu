@@ -49,7 +49,12 @@
 namespace dl {
 
 constexpr int kResStack = 4;                 // top traversal-stack entries of a thread in shared memory
-constexpr int kResMaxTurns = 1000000;        // queue chunks one warp takes
+// Vertices of one path, as many as the wavefront's host loop allows
+// iterations: what bounds the kernel's work, whatever the number of paths.
+#ifndef DL_MAX_VERTICES   // (tests set a small one)
+#define DL_MAX_VERTICES 1000000
+#endif
+constexpr int kResMaxVertices = DL_MAX_VERTICES;
 constexpr int kResMaxSpins = 1 << 22;        // polls of one wait (each about 0.1 us)
 constexpr uint32_t kShadowTask = 0x8000u, kFreeEntry = 0x8000u, kNoEntry = 0xffffu;
 constexpr int kEndedQueue = kNumMaterialTypes;  // misses, and kFreeEntry | slot for empty slots
@@ -375,6 +380,10 @@ __device__ __forceinline__ void resident_shade(const RenderParams& P, Sm& sm, in
         S.depth = sm.depth[slot];
         S.flags = sm.flags[slot];
         S.pid = sm.pid[slot];
+        if (S.depth >= kResMaxVertices) {   // give up, all warps of the block
+            err |= kErrRounds;
+            st_shared(&sm.abort, 1);
+        }
         const int rid = S.flags >> kReqShift;
         const DevRequest& R = request<kMulti>(P, rid);
         const float3 dir = f3(sm.d[0][slot], sm.d[1][slot], sm.d[2][slot]);
@@ -543,7 +552,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_resident(RenderParams P, 
     uint32_t err = 0;
     unsigned n_ext = 0, n_shadow = 0;
     int idle = 0;
-    for (int turn = 0;;) {
+    for (;;) {
         // the fullest queue, and the rays
         int most = 0, rays = 0;
         if (lane <= kNumMaterialTypes)
@@ -566,7 +575,6 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_resident(RenderParams P, 
                 if (best == kEndedQueue) resident_restart<kMulti, kTail>(P, sm, e, active, tail, err);
                 else resident_shade<kMulti>(P, sm, best, active ? (int)e : 0, active, err);
                 idle = 0;
-                if (++turn == kResMaxTurns) st_shared(&sm.abort, 1);
             }
         } else {
             // nothing to do: the pass has no more paths, or other warps hold
