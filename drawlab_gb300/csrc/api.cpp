@@ -611,7 +611,7 @@ int dl_context_get_tune(const dl_context* ctx, dl_tune_params* out) {
     out->paths_in_flight = ctx->tune.paths_in_flight;
     out->traverse_ctas_per_sm = ctx->tune.trav_ctas_per_sm;
     out->shade_ctas_per_sm = ctx->tune.shade_ctas_per_sm;
-    out->iterations_per_graph = ctx->tune.iters_per_graph;
+    out->iterations_per_graph = dl::graph_iterations(ctx->tune, false);
     out->shade_threads = ctx->tune.shade_threads;
     return DL_OK;
 }
@@ -688,6 +688,7 @@ int dl_autotune(dl_context* ctx, const dl_request* reqs, int32_t n, int32_t tria
             ctx->tuning = false;
             throw;
         }
+        best.iters_per_graph = dl::graph_iterations(best, false);   // (as timed)
         ctx->tune = best;
         ctx->kernel_timing = timing;
         ctx->tuning = false;

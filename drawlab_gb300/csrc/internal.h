@@ -86,7 +86,8 @@ constexpr int kNumMaterialTypes = 5;
 
 // Launch shape of the wavefront, chosen by dl_autotune (these defaults
 // otherwise): path slots in flight, resident CTAs per SM of the traversal
-// kernels and of the shading kernels, iterations per captured graph (even).
+// kernels and of the shading kernels, iterations per captured graph (even; 0:
+// not set by the caller, see graph_iterations).
 struct TuneParams {
     // 32M slots (6.9 GB of path state; a render uses at most one slot per
     // path): fewer, fuller wavefront iterations per frame
@@ -94,8 +95,20 @@ struct TuneParams {
     int trav_ctas_per_sm = 8;
     int shade_ctas_per_sm = 16;
     int shade_threads = 128;   // threads per CTA of the miss and material kernels
-    int iters_per_graph = 8;
+    int iters_per_graph = 0;
 };
+
+// Iterations per captured graph launch, after which the host looks at the
+// counters.  Where the resident kernel takes over the last paths (`tail`) they
+// are looked for more often, unless the caller set a number (device ms with
+// 8 | 4 | 2: unbounded spheres 800x600 8 spp 6.0 | 5.0 | 5.0, sky 517x389 16 spp
+// 1.78 | 1.56 | 1.57, textured box 640x500 16 spp 4.38 | 4.38 | 4.28, spheres
+// 1080p 4 spp 4.62 | 4.64 | 4.39, 64 spp 56.2 | 55.8 | 55.8; Cornell 512x512 16
+// spp 3.35 | 3.36 | 3.40).
+constexpr int kGraphIterations = 8, kTailGraphIterations = 2;
+inline int graph_iterations(const TuneParams& tp, bool tail) {
+    return tp.iters_per_graph > 0 ? tp.iters_per_graph : tail ? kTailGraphIterations : kGraphIterations;
+}
 
 // A queue length that kernels bump with atomics, alone in its 128-byte line:
 // atomics on one line serialise in one L2 slice, so the hot counters are

@@ -1088,13 +1088,7 @@ static void run_wavefront(dl_context* ctx, RenderParams& P, int64_t cap, bool mu
     cudaStream_t st = ctx->stream;
     RenderBuffers& B = ctx->render;
     const TuneParams tp = ctx->tune;
-    // Where the resident kernel takes over the last paths, the host looks for
-    // them after every two iterations, unless the context's shape was set
-    // otherwise (device ms with 8 | 4 | 2: unbounded spheres 800x600 8 spp 6.0 |
-    // 5.0 | 5.0, sky 517x389 16 spp 1.78 | 1.56 | 1.57, textured box 640x500 16
-    // spp 4.38 | 4.38 | 4.28, spheres 1080p 4 spp 4.62 | 4.64 | 4.39, 64 spp
-    // 56.2 | 55.8 | 55.8; Cornell 512x512 16 spp 3.35 | 3.36 | 3.40).
-    const int batch = tail && tp.iters_per_graph == TuneParams().iters_per_graph ? 2 : tp.iters_per_graph;
+    const int batch = graph_iterations(tp, tail);
     DL_CUDA(cudaMemsetAsync(P.cnt, 0, sizeof(RenderCounters), st));
     B.host_pass.ensure(sizeof(PassValues));
     PassValues* pv = B.host_pass.as<PassValues>();
@@ -1646,9 +1640,9 @@ void render_li_fixed(dl_scene* S, const dl_render_opts& o, void* pool, int64_t s
     int64_t iters = 0;
     const TuneParams tp;  // default launch shape
     for (;;) {
-        for (int k = 0; k < tp.iters_per_graph; k++)
+        for (int k = 0; k < kGraphIterations; k++)
             launch_iteration<false>(P, k & 1, st, sms, tp, false, nullptr, nullptr);
-        iters += tp.iters_per_graph;
+        iters += kGraphIterations;
         DL_CUDA(cudaGetLastError());
         DL_CUDA(cudaMemcpyAsync(&hc, P.cnt, sizeof(RenderCounters), cudaMemcpyDeviceToHost, st));
         DL_CUDA(cudaStreamSynchronize(st));

@@ -428,7 +428,9 @@ typedef struct dl_tune_params {
     int64_t paths_in_flight;        /* 32 .. 2^28; opts.max_paths_in_flight overrides */
     int32_t traverse_ctas_per_sm;   /* 1 .. 16 */
     int32_t shade_ctas_per_sm;      /* 1 .. 64 */
-    int32_t iterations_per_graph;   /* 2, 4, 6 or 8 */
+    int32_t iterations_per_graph;   /* 2, 4, 6 or 8.  Where none was set it reads 8, and
+                                       renders whose last paths one launch may finish
+                                       use 2 */
     int32_t shade_threads;          /* 64, 128 or 256; 0 = 128 */
 } dl_tune_params;
 int dl_context_get_tune(const dl_context* ctx, dl_tune_params* out);

@@ -1,0 +1,25 @@
+"""Launch shapes set by the caller are the ones renders use."""
+import pytest
+
+from drawlab_gb300 import abi, api, scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def test_iterations_per_graph_set_by_the_caller_are_kept():
+    # more paths than the resident kernel takes alone, few vertices each: the
+    # render ends with the first graph launch after its last vertex
+    ctx = api.Context(0)
+    s = api.Scene.from_data(ctx, scenes.cornell(1300, 1250))
+    opts = abi.make_opts(spp=1, max_depth=2, seed=1)
+    s.render(opts)
+    assert ctx.stats().iterations in (2, 4)   # none set: looked at after every two
+    t = ctx.get_tune()
+    assert t.iterations_per_graph == 8
+    for k in (8, 6, 4, 2, 8):
+        t.iterations_per_graph = k
+        ctx.set_tune(t)
+        assert ctx.get_tune().iterations_per_graph == k
+        s.render(opts)
+        it = ctx.stats().iterations
+        assert it == k or (k == 2 and it == 4)
