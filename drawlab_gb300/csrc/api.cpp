@@ -688,7 +688,7 @@ int dl_autotune(dl_context* ctx, const dl_request* reqs, int32_t n, int32_t tria
             ctx->tuning = false;
             throw;
         }
-        best.iters_per_graph = dl::graph_iterations(best, false);   // (as timed)
+        best.iters_per_graph = dl::graph_iterations(best, true);   // (as timed)
         ctx->tune = best;
         ctx->kernel_timing = timing;
         ctx->tuning = false;

@@ -196,7 +196,7 @@ struct dl_context {
     dl::HostBuf words;   // pinned: error words on their way to the host
     dl::TuneParams tune;
     bool kernel_timing = false;
-    bool tuning = false;   // dl_autotune is timing the wavefront's launch shapes
+    bool tuning = false;   // dl_autotune is timing the wavefront's launch shapes: no pass runs without it
     std::vector<cudaEvent_t> timing_events;  // created on first timed render
     // CUDA graph of one batch of wavefront iterations, reused while the
     // kernel parameters stay byte-identical.

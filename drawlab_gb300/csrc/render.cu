@@ -1202,14 +1202,16 @@ static void run_wavefront(dl_context* ctx, RenderParams& P, int64_t cap, bool mu
     acc.stat_tris_sh += hc->stat_tris_sh;
 }
 
-// A pass of `total` paths runs in the resident kernel: few paths, no pool
-// size asked for, and no need for the wavefront's separate kernels (their
-// times or traversal counts, or the tuning of their launch shape).
-static bool may_use_resident(const dl_context* ctx, int64_t pool, bool count_traversal) {
-    return pool == 0 && !count_traversal && !ctx->kernel_timing && !ctx->tuning;
+// Whether the resident kernel may take over a wavefront pass's last paths: no
+// pool size asked for, and no need for the wavefront's separate kernels (their
+// times or traversal counts).
+static bool may_finish(const dl_context* ctx, int64_t pool, bool count_traversal) {
+    return pool == 0 && !count_traversal && !ctx->kernel_timing;
 }
+// Whether it runs a whole pass of `total` paths: few, and not to tune the
+// wavefront's launch shape, which it has no use for.
 static bool use_resident(const dl_context* ctx, int64_t pool, unsigned long long total, bool count_traversal) {
-    return total <= kResidentMaxPaths && may_use_resident(ctx, pool, count_traversal);
+    return total <= kResidentMaxPaths && may_finish(ctx, pool, count_traversal) && !ctx->tuning;
 }
 
 // Budget of the per-path sample buffer; larger frames render in passes of
@@ -1330,14 +1332,14 @@ void render_run(dl_scene* S, const dl_render_opts& o, float* d_film, int64_t li_
     if (P.mode == 1) {
         if (!resident)
             run_wavefront(ctx, P, cap, false, count_traversal, kms, launches, iters, acc, (unsigned long long)li_n, 0,
-                          1u << 24, may_use_resident(ctx, o.max_paths_in_flight, count_traversal));
+                          1u << 24, may_finish(ctx, o.max_paths_in_flight, count_traversal));
     } else {
         for (int s0 = 0; s0 < spp; s0 += chunk_spp) {
             int ns = std::min(chunk_spp, spp - s0);
             if (!resident)
                 run_wavefront(ctx, P, cap, false, count_traversal, kms, launches, iters, acc,
                               npix * (unsigned long long)ns, o.spp_offset + s0, 1u << 24,
-                              may_use_resident(ctx, o.max_paths_in_flight, count_traversal));
+                              may_finish(ctx, o.max_paths_in_flight, count_traversal));
             F.nspp = ns;
             F.s_first = o.spp_offset + s0;
             F.accumulate = s0 > 0;
@@ -1566,7 +1568,7 @@ void render_batch(dl_context* ctx, const BatchItem* items, int n, bool count_tra
             launches = iters = 1;
         } else {
             run_wavefront(ctx, P, cap, true, count_traversal, kms, launches, iters, acc, first, 0, 1u << 24,
-                          may_use_resident(ctx, requested, count_traversal));
+                          may_finish(ctx, requested, count_traversal));
         }
         for (int a = 0; a < na; a++) {
             const int r = active[a];

@@ -423,7 +423,10 @@ int dl_render_batch(dl_context* ctx, const dl_request* reqs, int32_t n);
 /* Launch shape of the wavefront renderer: path slots in flight (the pool),
  * CTAs per SM of the traversal kernels and of the shading kernels, threads
  * per CTA of the shading kernels (the miss and the material kernels),
- * wavefront iterations per captured graph launch (between queue checks). */
+ * wavefront iterations per captured graph launch (between queue checks).
+ * Passes of up to 1,572,864 paths (pixels x samples, or paths of dl_li) of
+ * renders that give no pool size and are not guided run as one launch that
+ * has no such shape; images do not depend on it. */
 typedef struct dl_tune_params {
     int64_t paths_in_flight;        /* 32 .. 2^28; opts.max_paths_in_flight overrides */
     int32_t traverse_ctas_per_sm;   /* 1 .. 16 */
@@ -440,8 +443,9 @@ int dl_context_set_tune(dl_context* ctx, const dl_tune_params* tune);
  * an eighth of each request's spp, at least 1) under candidate launch shapes
  * -- a coordinate search over the pool size, then the traversal and shading
  * grid sizes, the shading block size, then the graph length -- times each
- * on the GPU, and keeps the
- * fastest on the context.  `out` (may be NULL) receives it; `trials` (may be
+ * on the GPU, and keeps the fastest on the context.  The trials run on the
+ * wavefront whatever their size (a pass of full spp may be one that does),
+ * and end as its renders do.  `out` (may be NULL) receives it; `trials` (may be
  * NULL) the number of shapes timed.  Outputs of the requests are not written. */
 int dl_autotune(dl_context* ctx, const dl_request* reqs, int32_t n, int32_t trial_spp, dl_tune_params* out,
                 int32_t* trials);

@@ -23,3 +23,16 @@ def test_iterations_per_graph_set_by_the_caller_are_kept():
         s.render(opts)
         it = ctx.stats().iterations
         assert it == k or (k == 2 and it == 4)
+
+
+def test_autotune_times_what_renders_run():
+    # unbounded paths through glass: a render looks for its last paths and
+    # finishes them in one launch, and so does a trial (here the last one, of
+    # eight iterations a graph)
+    ctx = api.Context(0)
+    s = api.Scene.from_data(ctx, scenes.reference_spheres(640, 480))
+    opts = abi.make_opts(spp=16, max_depth=0, seed=2)
+    t, _ = ctx.autotune([(s, opts)], trial_spp=2)
+    assert ctx.stats().iterations == 8
+    s.render(opts)
+    assert ctx.stats().iterations < 150   # (232 to the end, at an eighth of the samples)
