@@ -160,13 +160,18 @@ __device__ __forceinline__ int ring_claim(Ring<N>& r, int want, uint32_t& base) 
     base = __shfl_sync(0xffffffffu, h, 0);
     return __shfl_sync(0xffffffffu, n, 0);
 }
-// Entry `at` of a claimed range.
-template <int N>
-__device__ __forceinline__ uint32_t ring_take(Ring<N>& r, uint32_t at, int* abort, uint32_t& err) {
+// Entry `at` of a claimed range.  (In the bounds-checked build one that names
+// no slot of the block ends the block's work.)
+template <class Sm, int N>
+__device__ __forceinline__ uint32_t ring_take(const RenderParams& P, Sm& sm, Ring<N>& r, uint32_t at, uint32_t& err) {
     volatile uint16_t* e = &r.entry[at % N];
-    const uint32_t v = ring_wait(e, false, abort, err);
+    const uint32_t v = ring_wait(e, false, &sm.abort, err);
     *e = (uint16_t)kNoEntry;
     __threadfence_block();
+    if (!DL_IN_BOUNDS(v == kNoEntry || (int)(v & ~kFreeEntry) < Sm::kBlockSlots, &P.cnt->err)) {
+        st_shared(&sm.abort, 1);
+        return kNoEntry;
+    }
     return v;
 }
 
@@ -203,7 +208,11 @@ __device__ __forceinline__ void ray_done(const RenderParams& P, Sm& sm, int slot
         resident_store<kMulti>(P, sm.pid[slot], f3(sm.L[0][slot], sm.L[1][slot], sm.L[2][slot]));
         ring_push_lane(sm.queue[kEndedQueue], kFreeEntry | (uint32_t)slot, &sm.abort, err);
     } else {
-        ring_push_lane(sm.queue[sm.hit[slot] >> 27], (uint32_t)slot, &sm.abort, err);
+        const int q = sm.hit[slot] >> 27;
+        if (DL_IN_BOUNDS(q >= 0 && q <= kEndedQueue, &P.cnt->err))
+            ring_push_lane(sm.queue[q], (uint32_t)slot, &sm.abort, err);
+        else
+            st_shared(&sm.abort, 1);
     }
 }
 
@@ -251,7 +260,7 @@ __device__ __forceinline__ void resident_trace(const RenderParams& P, Sm& sm, ui
             const int n = ring_claim(sm.rays, __popc(m), base);
             const int i = __popc(m & ((1u << lane) - 1u));
             if (!has && i < n) {
-                const uint32_t task = ring_take(sm.rays, base + i, &sm.abort, err);
+                const uint32_t task = ring_take(P, sm, sm.rays, base + i, err);
                 if (task != kNoEntry) {
                     any = (task & kShadowTask) != 0;
                     slot = (int)(task & ~kShadowTask);
@@ -462,8 +471,8 @@ __device__ __forceinline__ void resident_restart(const RenderParams& P, Sm& sm, 
     const unsigned long long pid = kTail ? warp_claim_u32(&P.cnt->tail_next, active) : warp_claim(&P.cnt->next_path, active);
     bool start = active && pid < (kTail ? tail : P.total);
     if (kTail && start) {
-        const int from = P.ext_q[0][pid];
-        if (slot_ok(P, from)) {
+        const int from = DL_IN_BOUNDS(pid < (unsigned)P.capacity, &P.cnt->err) ? P.ext_q[0][pid] : -1;
+        if (from >= 0 && slot_ok(P, from)) {
             const RayRec r = P.rec[from].ray;
             const MetaRec mr = P.rec[from].meta;
             const PathRec pr = mr.m.y & PF_CAMERA ? camera_record() : P.rec[from].path;
@@ -570,7 +579,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_resident(RenderParams P, 
             uint32_t base;
             const int n = ring_claim(sm.queue[best], 32, base);
             if (n > 0) {
-                const uint32_t e = lane < n ? ring_take(sm.queue[best], base + lane, &sm.abort, err) : kNoEntry;
+                const uint32_t e = lane < n ? ring_take(P, sm, sm.queue[best], base + lane, err) : kNoEntry;
                 const bool active = e != kNoEntry;
                 if (best == kEndedQueue) resident_restart<kMulti, kTail>(P, sm, e, active, tail, err);
                 else resident_shade<kMulti>(P, sm, best, active ? (int)e : 0, active, err);
