@@ -1,4 +1,6 @@
-"""Launch shapes set by the caller are the ones renders use."""
+"""Launch shapes set by the caller are the ones renders use, and images do not
+depend on them."""
+import numpy as np
 import pytest
 
 from drawlab_gb300 import abi, api, scenes
@@ -36,3 +38,18 @@ def test_autotune_times_what_renders_run():
     assert ctx.stats().iterations == 8
     s.render(opts)
     assert ctx.stats().iterations < 150   # (232 to the end, at an eighth of the samples)
+
+
+@pytest.mark.parametrize("threads", [64, 128, 256])
+def test_launch_shapes_render_the_same_images(threads):
+    # a pool size keeps small frames on the wavefront, which has a launch shape
+    ctx = api.Context(0)
+    made = [api.Scene.from_data(ctx, f(48, 40)) for f in (scenes.cornell, scenes.env_spheres, scenes.reference_spheres)]
+    items = [(s, abi.make_opts(spp=4 + k, max_depth=6, seed=k, max_paths_in_flight=8192)) for k, s in enumerate(made)]
+    ref = ctx.render_batch([(s, abi.make_opts(spp=4 + k, max_depth=6, seed=k)) for k, s in enumerate(made)])
+    for iterations, trav, shade in ((2, 1, 1), (4, 4, 8), (6, 16, 64), (8, 8, 16)):
+        ctx.set_tune(abi.dl_tune_params(paths_in_flight=1 << 20, traverse_ctas_per_sm=trav, shade_ctas_per_sm=shade,
+                                        iterations_per_graph=iterations, shade_threads=threads))
+        for (s, o), img, want in zip(items, ctx.render_batch(items), ref):
+            assert np.array_equal(img, want) and np.array_equal(s.render(o), want)
+            assert ctx.stats().iterations > 1
