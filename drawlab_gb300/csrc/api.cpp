@@ -746,7 +746,6 @@ int dl_guide_create(dl_context* ctx, const dl_guide_config* cfg, dl_guide** out)
         G->cfg = *cfg;
         const size_t pb = dl::kGuideParams * 4;
         for (dl::DevBuf* b : {&G->w32, &G->grad, &G->m, &G->v}) b->ensure(pb);
-        G->w16.ensure(dl::kGuideParams * 2);
         G->image.ensure(dl::kGuideImageBytes);
         G->scratch.ensure(256);
         // training overlaps the next render pass; at the highest priority its

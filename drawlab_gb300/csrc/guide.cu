@@ -14,8 +14,7 @@
 //                        tensor memory; one partial gradient per block
 //   k_guide_grad_reduce  the blocks' partial gradients summed; in a training
 //                        step also Adam on the fp32 master weights, which
-//                        refreshes the fp16 copy and the tensor cores' weight
-//                        image
+//                        refreshes the tensor cores' fp16 weight image
 // Inference (k_guide_infer, and the guided material kernels in render.cu)
 // runs on tcgen05 too (guide_tc.cuh).
 #include <cuda_fp16.h>
@@ -230,7 +229,7 @@ __device__ __forceinline__ float record_grad_half(const float* o, float3 w, floa
 //
 // What bounds it: a tile is a chain of six dependent steps -- products, their
 // completion, an epilogue over 128 rows, a barrier -- of 10600 cycles when a
-// block works on one tile, the tensor cores busy for 2600 of them (55
+// block works on one tile, the tensor cores busy for 2600 of them (48
 // products of 128 rows, 48 to 82 cycles each: at these widths the operands'
 // way from shared memory sets the time).  The second tile in the first one's
 // waits makes it 13400 cycles for two.  The issuing warp keeps its control
@@ -663,7 +662,6 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_guide_train(const void* image
 // Adam's state and this step's constants.
 struct AdamStep {
     float* w32;              // fp32 master weights
-    __half* w16;
     unsigned char* image;    // the tensor cores' weight image
     float *m, *v;
     float lr, b1, b2, c1, c2, eps;
@@ -681,7 +679,7 @@ static_assert(guide_pad_param(0) == kGW3 + kGOut * kGHid && guide_pad_param(kPPa
 // the training blocks of their sums' slot t.  A block takes 32 consecutive
 // slots; its 8 warps split the blocks' sums and add theirs in shared memory.
 // kAdam: the warp that has the gradients updates their parameters (fp32
-// master, fp16 copy, weight image) and clears the batch's loss if `loss` is
+// master, weight image) and clears the batch's loss if `loss` is
 // given (for the next batch of a call).  Otherwise grad[p] is written.  The
 // padding parameters have no slots: Adam clears them.
 //
@@ -742,16 +740,13 @@ __global__ void __launch_bounds__(32 * kRedWarps) k_guide_grad_reduce(const floa
     }
     if (kAdam && p >= 0) {
         A.w32[p] = x;   // (the padding: 0)
-        A.w16[p] = __float2half_rn(x);
         write_image(A.image, p, x);
     }
 }
 
-__global__ void k_guide_to_half(const float* w32, __half* w16, unsigned char* image) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kGParams; i += gridDim.x * blockDim.x) {
-        w16[i] = __float2half_rn(w32[i]);
+__global__ void k_guide_image(const float* w32, unsigned char* image) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kGParams; i += gridDim.x * blockDim.x)
         write_image(image, i, w32[i]);
-    }
 }
 
 // ------------------------------------------------------------------ host
@@ -790,7 +785,7 @@ void guide_init_params(uint64_t seed, std::vector<float>& w) { init_params(seed,
 void guide_upload_params(dl_guide* G, const float* host) {
     cudaStream_t st = G->ctx->stream;
     DL_CUDA(cudaMemcpyAsync(G->w32.ptr, host, kGParams * 4, cudaMemcpyHostToDevice, st));
-    k_guide_to_half<<<64, 256, 0, st>>>(G->w32.as<float>(), G->w16.as<__half>(), G->image.as<unsigned char>());
+    k_guide_image<<<64, 256, 0, st>>>(G->w32.as<float>(), G->image.as<unsigned char>());
     DL_CUDA(cudaGetLastError());
 }
 
@@ -879,7 +874,6 @@ static void guide_steps(dl_guide* G, const void* d_recs, int64_t n, int stride, 
         G->step += 1;
         AdamStep A;
         A.w32 = G->w32.as<float>();
-        A.w16 = G->w16.as<__half>();
         A.image = G->image.as<unsigned char>();
         A.m = G->m.as<float>();
         A.v = G->v.as<float>();

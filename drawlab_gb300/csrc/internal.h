@@ -219,12 +219,12 @@ struct dl_context {
     }
 };
 
-// Learned guiding proposal: parameters (fp32 master, fp16 copy), Adam state
+// Learned guiding proposal: parameters (fp32 master, fp16 image), Adam state
 // and training buffers (guide.cu).
 struct dl_guide {
     dl_context* ctx = nullptr;
     dl_guide_config cfg{};
-    dl::DevBuf w32, w16, grad, m, v, scratch, recs, io_in, io_out;
+    dl::DevBuf w32, grad, m, v, scratch, recs, io_in, io_out;
     dl::DevBuf image;       // the weights as the tensor-core kernels load them (guide_tc.cuh)
     dl::DevBuf pass_recs;   // training records of guided render passes (two halves, alternating)
     dl::DevBuf partial;                    // a training batch's per-block gradient sums

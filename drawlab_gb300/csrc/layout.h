@@ -7,7 +7,6 @@
 namespace dl {
 
 // ------------------------------------------------------------------ layout
-constexpr int32_t kEmptyChild = 0x7fffffff;
 constexpr int kStackSize = 64;
 constexpr float kRayEps = 1e-4f;   // M_EPSILON, include/core/math/math.h:14
 constexpr float kPiF = 3.14159265358979323846f;

@@ -1578,7 +1578,7 @@ void render_batch(dl_context* ctx, const BatchItem* items, int n, bool count_tra
             F.nspp = ns[a];
             F.s_first = hreq[a].spp_offset;
             F.accumulate = done[r] > 0;
-                film_gather(F, ctx->num_sms, st);
+            film_gather(F, ctx->num_sms, st);
             launches += 1;
             done[r] += ns[a];
         }

@@ -59,18 +59,9 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" :: "r"(taddr), "r"(ncols) : "memory");
 }
 
-// D[taddr] (+)= A x B^T, one instruction; `accumulate` 0 overwrites D.
-__device__ __forceinline__ void mma_f16(uint32_t taddr, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                        uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-        :: "r"(taddr), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-
-// The same by the lane of a converged warp whose `leader` is set: control
-// flow, descriptors and addresses stay the warp's, in uniform registers.
+// D[taddr] (+)= A x B^T, one instruction, by the lane of a converged warp
+// whose `leader` is set: control flow, descriptors and addresses stay the
+// warp's, in uniform registers.  `accumulate` 0 overwrites D.
 __device__ __forceinline__ void mma_f16_by(bool leader, uint32_t taddr, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                            uint32_t accumulate) {
     asm volatile(
@@ -81,13 +72,8 @@ __device__ __forceinline__ void mma_f16_by(bool leader, uint32_t taddr, uint64_t
         :: "r"(taddr), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"((uint32_t)leader) : "memory");
 }
 
-// The mbarrier arrives once all tcgen05 operations this thread issued
-// before have completed.
-__device__ __forceinline__ void commit(uint64_t* mbar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
-                 :: "r"(smem_addr(mbar)) : "memory");
-}
-
+// The mbarrier arrives once all tcgen05 operations the leader issued before
+// have completed.
 __device__ __forceinline__ void commit_by(bool leader, uint64_t* mbar) {
     asm volatile(
         "{\n\t.reg .pred q;\n\t"
