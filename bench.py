@@ -93,10 +93,13 @@ NET_MAC_TRAIN = NET_MAC_FWD + (48 * 64 + 64 * 64) + NET_MAC_FWD
 
 
 def network_roofline(ctx, api, train_rows=(131072, 32768)):
-    """Device time of the network kernels alone (dl_guide_forward on 4M rows;
-    dl_guide_gradient on training batches of train_rows records, the first
-    the renderer's default batch, 131072), as FLOP/s against the measured
-    tensor peak and as bytes/s against HBM."""
+    """Device time of the network kernels alone (dl_guide_forward on 16M rows
+    in device memory, 403 MB, more than L2; dl_guide_gradient on training batches of train_rows
+    records, the first the renderer's default batch, 131072), as FLOP/s
+    against the measured tensor peak and as bytes/s against HBM; beside it the
+    same forward kernel on 4M rows in host memory, which it reads over the
+    host link."""
+    import torch
     tpk, tkind = tensor_peak()
     hbm, hkind = peaks()
     rng = np.random.default_rng(3)
@@ -107,6 +110,15 @@ def network_roofline(ctx, api, train_rows=(131072, 32768)):
     times = []
     for _ in range(4):
         g.forward(inp)
+        times.append(ctx.stats().guide_ms)
+    t_host = float(np.median(times[1:]))
+    nd = 4 * n
+    d_in = torch.from_numpy(inp).to("cuda").repeat(4, 1)   # (the context's device is current)
+    d_out = torch.empty((nd, 40), dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    times = []
+    for _ in range(4):
+        ctx.check(ctx.lib.dl_guide_forward(g.h, nd, d_in.data_ptr(), d_out.data_ptr()))
         times.append(ctx.stats().guide_ms)
     t_inf = float(np.median(times[1:]))
     train = []
@@ -125,11 +137,12 @@ def network_roofline(ctx, api, train_rows=(131072, 32768)):
         tr_tf = 2.0 * NET_MAC_TRAIN * nb / (t_tr * 1e-3) / 1e12
         train.append({"kernels": "k_guide_weight_sum + k_guide_train + k_guide_grad_reduce (tcgen05)", "rows": nb, "ms": t_tr, "tflops": tr_tf, "frac_tensor": tr_tf / tpk,
                       "flop_per_row": 2 * NET_MAC_TRAIN})
-    inf_tf = 2.0 * NET_MAC_FWD * n / (t_inf * 1e-3) / 1e12
-    inf_gbs = (24 + 160) * n / (t_inf * 1e-3) / 1e9
-    return {"inference": {"kernel": "k_guide_infer (tcgen05)", "rows": n, "ms": t_inf, "tflops": inf_tf,
+    del d_in, d_out
+    inf_tf = 2.0 * NET_MAC_FWD * nd / (t_inf * 1e-3) / 1e12
+    inf_gbs = (24 + 160) * nd / (t_inf * 1e-3) / 1e9
+    return {"inference": {"kernel": "k_guide_infer (tcgen05)", "rows": nd, "ms": t_inf, "tflops": inf_tf,
                           "frac_tensor": inf_tf / tpk, "gbs": inf_gbs, "frac_hbm": inf_gbs / hbm,
-                          "bytes_per_row": 184, "flop_per_row": 2 * NET_MAC_FWD},
+                          "host_rows": n, "host_rows_ms": t_host, "bytes_per_row": 184, "flop_per_row": 2 * NET_MAC_FWD},
             "training_batch": train[0], "training_batches": train,
             "peak_tflops": tpk, "peak_kind": tkind, "hbm_peak": hbm, "hbm_kind": hkind}
 

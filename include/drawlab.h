@@ -212,7 +212,8 @@ int dl_scene_get_info(const dl_scene* scene, dl_scene_info* info);
  * with the Moller-Trumbore test of Mesh::rayIntersect
  * (src/tracer/mesh/mesh.cpp:180-220).  prim_id is the global triangle index
  * (meshes concatenated in order), -1 on a miss; t, u, v as the reference
- * computes them.  Host buffers. */
+ * computes them.  Host buffers; the results may overlap the rays, and one
+ * another (stored in the order t, u, v, prim_id). */
 int dl_trace_closest(dl_scene* scene, const float* rays, int64_t n,
                      int32_t* prim_id, float* t, float* u, float* v);
 
@@ -480,7 +481,8 @@ int dl_guide_create(dl_context* ctx, const dl_guide_config* cfg, dl_guide** out)
 int dl_guide_destroy(dl_guide* guide);
 int dl_guide_get_params(const dl_guide* guide, float* params);
 int dl_guide_set_params(dl_guide* guide, const float* params);
-/* Network outputs (n x 40) for inputs (n x 6: position in [0,1]^3, normal). */
+/* Network outputs (n x 40) for inputs (n x 6: position in [0,1]^3, normal).
+ * Host buffers, or device memory. */
 int dl_guide_forward(dl_guide* guide, int64_t n, const float* inputs, float* outputs);
 /* Training records, 12 floats each: position in [0,1]^3 (3), normal (3),
  * sampled direction (3), its sampling pdf, radiance estimate along it, 0.
@@ -508,7 +510,7 @@ typedef struct dl_stats {
     int64_t extension_rays;    /* closest-hit rays traced (camera rays included) */
     int64_t shadow_rays;       /* any-hit rays traced */
     int64_t invalid_samples;   /* samples dropped by the film (NaN/Inf/negative) */
-    int64_t iterations;        /* wavefront iterations of the last render */
+    int64_t iterations;        /* wavefront iterations of the last render (1: it ran as one launch) */
     double render_ms;          /* device time of the last render */
     double trace_ms;           /* device time of the last dl_trace_* call */
     /* Per-kernel device time of the last render, summed over its launches
@@ -523,10 +525,17 @@ typedef struct dl_stats {
     double guide_train_ms;     /* device time of the last training round of the last guided
                                   render (rounds overlap the next pass's rendering) */
     double guide_ms;           /* device time of the network kernels of the last
-                                  dl_guide_forward / dl_guide_gradient call */
+                                  dl_guide_forward / dl_guide_gradient call; on a device
+                                  that walks the host's page tables the forward kernel
+                                  reads its rows over the host link meanwhile (rows given
+                                  in device memory: the kernel alone) */
 } dl_stats;
 
-/* Enable (1) or disable (0) per-kernel event timing on a context. */
+/* Enable (1) or disable (0) per-kernel event timing on a context.  Renders
+ * then run on the wavefront from the first path to the last, one kernel after
+ * another: render_ms is the time of that.  Without it independent kernels run
+ * side by side, a render of few paths is one launch, and the last paths of a
+ * large one are; the image is the same. */
 int dl_context_set_kernel_timing(dl_context* ctx, int enabled);
 
 /* Counters of the last dl_render* / dl_li / dl_trace_* call on ctx. */
