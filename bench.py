@@ -61,10 +61,10 @@ NODE_BYTES, TRI_BYTES, RAY_IN, HIT_OUT = 64, 48, 32, 16
 # bytes (dram__bytes_read.sum + dram__bytes_write.sum) summed over the
 # frame's launches of each kernel, divided by the frame's extension / shadow
 # rays.  Profile measurements, scaled here by the rays of the timed frames.
-EXT_L2_BYTES_PER_RAY = 158925079 * 32 / 14984872            # 339.4 B
-EXT_DRAM_BYTES_PER_RAY = (2181426688 + 471964416) / 14984872  # 177.1 B
-SH_L2_BYTES_PER_RAY = 63489526 * 32 / 5484823                 # 370.4 B
-SH_DRAM_BYTES_PER_RAY = (954967296 + 120330240) / 5484823     # 196.1 B
+EXT_L2_BYTES_PER_RAY = 158406602 * 32 / 14984872            # 338.3 B
+EXT_DRAM_BYTES_PER_RAY = (2170802944 + 471431936) / 14984872  # 176.3 B
+SH_L2_BYTES_PER_RAY = 64186735 * 32 / 5484823                 # 374.5 B
+SH_DRAM_BYTES_PER_RAY = (953086976 + 119751424) / 5484823     # 195.6 B
 
 
 def peaks():
@@ -493,7 +493,7 @@ def traversal_roofline(hbm, peak_kind, l2_peak, ext_ms, sh_ms, ext_rays, sh_rays
          "bytes_per_ray": bytes_per_ray, "node_visits_per_ray": n_node, "tri_tests_per_ray": n_tri,
          "algorithmic_bytes_per_launch": bytes_per_ray * ext_rays / max(1, ext_launches),
          "traffic": EXT_DRAM_BYTES_PER_RAY * ext_rays / max(1, ext_launches),
-         "traffic_note": "DRAM bytes per launch: the profile's DRAM bytes per ray (177 B) x this frame's rays per "
+         "traffic_note": "DRAM bytes per launch: the profile's DRAM bytes per ray (176 B) x this frame's rays per "
                          "launch",
          "l2_traffic": {"bytes_per_ray": EXT_L2_BYTES_PER_RAY, "achieved": l2_gbs, "frac": l2_gbs / l2_peak,
                         "l1_served_fraction": 1.0 - EXT_L2_BYTES_PER_RAY / bytes_per_ray,

@@ -1,8 +1,9 @@
 // A pass of few paths in one launch: the wavefront's path slots and queues
 // held in shared memory, block by block.
 //
-// A wavefront iteration (render.cu) costs about 30 us however few paths it
-// advances -- eight kernels and two joins -- and keeps its paths in DRAM.
+// A wavefront iteration (render.cu) costs 24 us with no path in it and 35-55 us
+// with a few -- eight kernels, two joins, the longest search -- and keeps its
+// paths in DRAM.
 // Here each block owns some hundred slots and takes paths of the pass until
 // none are left.  Its warps work through queues in shared memory without
 // block-wide barriers: a warp takes 32 hits on one material (or 32 ended
@@ -13,10 +14,11 @@
 // adds its terms in the same order, so images are bit-equal.
 //
 // What bounds it: the chain of dependent searches and vertices while there
-// are fewer paths than threads (about 10 us a vertex), then issue slots
-// (50 %: instruction fetch, 2-4 stalls per issue, since a warp runs a vertex
-// alone where the wavefront's kernels run it in step) and the traversal's L1
-// wavefronts.  Hence one copy of the vertex code for all materials (`type`
+// are fewer paths than threads (about 10 us a vertex; Cornell 256x256 1 spp:
+// issue slots 37 % used, 15 of 64 warps), then issue slots (16 spp: 52 %;
+// instruction fetch is the largest stall, 3.3-4.0 cycles per issue, since a
+// warp runs a vertex alone where the wavefront's kernels run it in step) and
+// half-idle warps (14-17 of 32 lanes).  Hence one copy of the vertex code for all materials (`type`
 // is the same for all lanes of a warp) and helpers as functions: with five
 // inlined copies the code was 285 KB, now 100 KB, and the instruction cache
 // misses cost the sky scene 1.6x.

@@ -31,10 +31,12 @@ struct RayScratch {
 // each lane descends to a leaf, then tests the leaf's triangles.  Bounded by
 // the latency of dependent node fetches while the rays are no more than the
 // resident threads (one thread a ray), then by the L1's wavefronts, as the
-// renderer's traversal.  Material-sphere scene, 200,003 host rays, half from
-// the camera: whole calls of dl_trace_closest 590 -> 166 us (rays read in
-// place, hits split by a kernel), of dl_trace_any 147 -> 107 us; 2 M rays 5.1
-// -> 0.78 ms (device part 1.07 -> 0.73).
+// renderer's traversal.  Material-sphere scene, whole calls on host arrays used
+// before | on new ones, against one thread a ray, copies and hits split on the
+// host: dl_trace_closest of 1000 rays 73 -> 62 us | 118 -> 93, 20,000 136 -> 76
+// | 195 -> 110, 200,003 568 -> 131 | 742 -> 211, 2 M 4.97 -> 0.57 ms | 6.20 ->
+// 1.43; dl_trace_any of 200,003 139 -> 102 us | 255 -> 141, 2 M 669 -> 399 |
+// 758 -> 475.
 template <bool kAny>
 __global__ void __launch_bounds__(kRayThreads) k_trace_rays(DevScene sc, const float4* __restrict__ rays, int64_t n,
                                                              void* __restrict__ out, RayScratch* scratch) {
