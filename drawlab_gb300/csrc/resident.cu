@@ -18,10 +18,10 @@
 // issue slots 37 % used, 15 of 64 warps), then issue slots (16 spp: 52 %;
 // instruction fetch is the largest stall, 3.3-4.0 cycles per issue, since a
 // warp runs a vertex alone where the wavefront's kernels run it in step) and
-// half-idle warps (14-17 of 32 lanes).  Hence one copy of the vertex code for all materials (`type`
-// is the same for all lanes of a warp) and helpers as functions: with five
-// inlined copies the code was 285 KB, now 100 KB, and the instruction cache
-// misses cost the sky scene 1.6x.
+// half-idle warps (14-17 of 32 lanes).  Hence one copy of the vertex code for
+// all materials (`type` is the same for all lanes of a warp) and helpers as
+// functions: with five inlined copies the code was 285 KB, now 100 KB, and the
+// instruction cache misses cost the sky scene 1.6x.
 //
 // Two shapes.  Few paths: 256 threads with up to 128 registers, no spills:
 // the shortest chain.  More: 384 threads at 80 registers, 24 warps an SM (28

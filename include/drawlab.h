@@ -4,7 +4,9 @@
  * Plain C types only (pointers, sizes, PODs): any FFI (ctypes, cgo, JNI,
  * N-API) can bind it.  Every entry point returns an int status (DL_OK on
  * success); dl_last_error() gives the message of the last failure on a
- * context.  No C++ exception crosses this boundary.
+ * context.  No C++ exception crosses this boundary.  A call that fails leaves
+ * its outputs unspecified: a render in one launch learns of its failure (a
+ * bounded wait that ran out) together with its results.
  *
  * The reference (xuxmin/DrawLab) exposes the same path as C++ virtual
  * interfaces.  Each entry point below names the reference interface it
